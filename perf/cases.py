@@ -109,7 +109,8 @@ def draw(rng):
                      box=0.0, steps=min(steps, 40), replicas=rng.randint(8, 24), cluster=1)
         return c
     if kind == "grad":
-        return {"kind": "grad", "rows": 128 * _logint(rng, 1, 63)}
+        # batches up to 1024 rows in steps of 128, larger ones in steps of 1024
+        return {"kind": "grad", "rows": rng.choice([128 * rng.randint(1, 8), 1024 * rng.randint(1, 7)])}
     if kind == "predict":
         return {"kind": "predict", "rows": _logint(rng, 100, 50000)}
     return {"kind": "train", "rows": _logint(rng, 16000, 131000)}
