@@ -1,11 +1,9 @@
 // surrogate_host.cu -- the pair-energy surrogate object: parameters, dataset, training.
 //
 // Training is plain mini-batch Adam on the mean squared error against targets clipped
-// to +-clip kcal/mol (clashes only need to read as "large").  Every step runs the
-// project's own kernels (mlp_kernels.cu): FP32 layer 1, three tcgen05 BF16 GEMMs with
-// fused bias/SiLU epilogues, FP32 output, then the backward pass as split-K tcgen05
-// GEMMs for the weight gradients (reduced in a fixed order) and GEMMs with fused SiLU'
-// epilogues for the activation gradients.
+// to +-clip kcal/mol (clashes only need to read as "large").  A step is three launches of
+// the project's own kernels (mlp_kernels.cu), enqueued without waiting; an epoch's
+// losses and the error flag are read once, at its end.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -41,21 +39,32 @@ float uniform_pm(uint64_t &s, float a)
     return (float)((2.0 * u - 1.0) * a);
 }
 
+// Rows of features staged on the device by one inference launch (2 MB of features).
+constexpr int kStageRows = 65536;
+
 }  // namespace
 
 struct cgppd_surrogate {
     int batch = 0;
     int k_split = 0;
+    int max_ctas = 1;
     uint64_t seed = 0;
     int adam_t = 0;
     cudaStream_t stream = nullptr;
+    // page-locked words the end of a call is read through: error flag, loss sum
+    struct Ends {
+        unsigned err;
+        float loss_sum;
+    } *ends = nullptr;
 
     DevBuf<float> P, G, am, av;
-    DevBuf<__nv_bfloat16> Wf, Wt;
-    // activations of one batch
-    DevBuf<float> X, y, Z, o, dO, r2, Cpart, scalars;
-    DevBuf<__nv_bfloat16> H, HT, dZ, dZT;
+    DevBuf<__nv_bfloat16> Wf, wtiles;
+    // one batch: inputs, tile images and partial gradient sums (k_net_rows, k_net_wgrad)
+    DevBuf<float> X, y, xb, dO, r2, wpart, losses;
+    DevBuf<__nv_bfloat16> act;
     DevBuf<unsigned> err;
+    // inference: staged features and predictions of up to kStageRows rows
+    DevBuf<float> stageX, stageO;
     // dataset
     DevBuf<float> dsX, dsY;
     DevBuf<int> perm;
@@ -66,6 +75,8 @@ struct cgppd_surrogate {
     {
         if (stream)
             cudaStreamDestroy(stream);
+        if (ends)
+            cudaFreeHost(ends);
     }
 
     int init(int b, uint64_t sd)
@@ -73,14 +84,18 @@ struct cgppd_surrogate {
         batch = b;
         seed = sd;
         k_split = std::min(batch, 1024);
-        if (cgppd_check(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "surrogate stream") != 0)
+        int dev = 0;
+        if (cgppd_check(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "surrogate stream") != 0 ||
+            cgppd_check(cudaMallocHost(&ends, sizeof(Ends)), "surrogate result words") != 0 ||
+            cgppd_check(cudaGetDevice(&dev), "surrogate device") != 0 ||
+            cgppd_check(cudaDeviceGetAttribute(&max_ctas, cudaDevAttrMultiProcessorCount, dev), "surrogate device") != 0 ||
+            cgppd_check(net_set_limits(), "surrogate shared-memory limits") != 0)
             return -1;
-        const size_t BH = (size_t)batch * kSurH;
+        const size_t tiles = (size_t)batch / kNetRows;
         if (P.zero(kSurParamsPad) || G.zero(kSurParamsPad) || am.zero(kSurParamsPad) || av.zero(kSurParamsPad) ||
-            Wf.alloc(3 * kSurH * kSurH) || Wt.alloc(3 * kSurH * kSurH) || X.zero((size_t)batch * kSurIn) ||
-            y.zero(batch) || Z.alloc(4 * BH) || o.alloc(batch) || dO.alloc(batch) || r2.alloc(batch) ||
-            Cpart.alloc((size_t)(batch / k_split) * kSurH * kSurH) || scalars.zero(4) || H.alloc(4 * BH) ||
-            HT.alloc(4 * BH) || dZ.alloc(2 * BH) || dZT.alloc(2 * BH) || err.zero(1))
+            Wf.alloc(3 * kSurH * kSurH) || wtiles.alloc(6 * kSurH * kSurH) || X.zero((size_t)batch * kSurIn) ||
+            y.zero(batch) || act.alloc(kActKinds * tiles * kNetTileElems) || xb.alloc((size_t)batch * kSurIn) ||
+            dO.alloc(batch) || r2.alloc(batch) || wpart.alloc((size_t)3 * (batch / k_split) * kSurH * kSurH) || losses.zero(1) || err.zero(1))
             return -1;
         // PyTorch-Linear-style initialisation: U(-1/sqrt(fan_in), 1/sqrt(fan_in))
         std::vector<float> p(kSurParamsPad, 0.f);
@@ -103,113 +118,90 @@ struct cgppd_surrogate {
 
     int set_params(const float *host)
     {
-        if (cgppd_check(cudaMemcpy(P.ptr, host, kSurParams * sizeof(float), cudaMemcpyHostToDevice), "surrogate params"))
+        if (cgppd_check(cudaMemcpyAsync(P.ptr, host, kSurParams * sizeof(float), cudaMemcpyHostToDevice, stream),
+                        "surrogate params") ||
+            cgppd_check(launch_net_copies(P.ptr, Wf.ptr, wtiles.ptr, stream), "surrogate bf16 copies"))
             return -1;
-        launch_bf16_copies(P.ptr, Wf.ptr, Wt.ptr, stream);
         return cgppd_check(cudaStreamSynchronize(stream), "surrogate bf16 copies");
     }
 
-    // forward (and backward when `grad`) over the batch in X/y (n rows, n % 128 == 0,
-    // n <= batch).  Returns 0 or -1.
-    int step(int n, bool with_targets, bool grad, float *loss_out)
+    // Enqueue predictions of n rows of device features.
+    int enqueue_forward(const float *dX, int n, float *dO)
     {
-        const size_t BH = (size_t)n * kSurH;
-        cudaStream_t st = stream;
-        float *Zl[4];
-        __nv_bfloat16 *Hl[4], *HTl[4];
-        for (int l = 0; l < 4; ++l) {
-            Zl[l] = Z.ptr + l * BH;
-            Hl[l] = H.ptr + l * BH;
-            HTl[l] = HT.ptr + l * BH;
-        }
-        launch_layer1_fwd(X.ptr, P.ptr, Zl[0], Hl[0], HTl[0], n, st);
-        for (int l = 2; l <= 4; ++l) {
-            GemmArgs g{};
-            g.A = Hl[l - 2];
-            g.B = Wf.ptr + (size_t)(l - 2) * kSurH * kSurH;
-            g.M = n;
-            g.K = kSurH;
-            g.k_split = kSurH;
-            g.bias = P.ptr + sur_b_off(l);
-            g.Z = Zl[l - 1];
-            g.H = Hl[l - 1];
-            g.HT = HTl[l - 1];
-            g.err = err.ptr;
-            if (cgppd_check(launch_gemm(kGemmFwd, g, st), "surrogate forward GEMM"))
-                return -1;
-        }
-        launch_out_fwd(Hl[3], P.ptr, with_targets ? y.ptr : nullptr, o.ptr, dO.ptr, r2.ptr, n, st);
-        if (with_targets)
-            launch_vec_sum(r2.ptr, n, scalars.ptr, st);
-        if (grad) {
-            const int ks = std::min(n, k_split);
-            if (n % ks != 0 || ks % 64 != 0)
-                return cgppd_fail("surrogate: batch must be a multiple of 64 (and of the split size)");
-            // output layer
-            launch_row_reduce(HTl[3], kSurH, n, nullptr, 0, dO.ptr, nullptr, G.ptr + kOffW5, st);
-            launch_vec_sum(dO.ptr, n, G.ptr + kOffB5, st);
-            __nv_bfloat16 *dZl[2] = {dZ.ptr, dZ.ptr + BH}, *dZTl[2] = {dZT.ptr, dZT.ptr + BH};
-            launch_out_bwd(dO.ptr, P.ptr, Zl[3], dZl[0], dZTl[0], n, st);
-            int cur = 0;
-            for (int l = 4; l >= 2; --l) {
-                GemmArgs gw{};
-                gw.A = dZTl[cur];
-                gw.B = HTl[l - 2];
-                gw.M = kSurH;
-                gw.K = n;
-                gw.k_split = ks;
-                gw.C = Cpart.ptr;
-                gw.err = err.ptr;
-                if (cgppd_check(launch_gemm(kGemmStore, gw, st), "surrogate weight-gradient GEMM"))
-                    return -1;
-                launch_splitk_reduce(Cpart.ptr, n / ks, kSurH * kSurH, G.ptr + sur_w_off(l), st);
-                launch_row_reduce(dZTl[cur], kSurH, n, nullptr, 0, nullptr, G.ptr + sur_b_off(l), nullptr, st);
-                GemmArgs gb{};
-                gb.A = dZl[cur];
-                gb.B = Wt.ptr + (size_t)(l - 2) * kSurH * kSurH;
-                gb.M = n;
-                gb.K = kSurH;
-                gb.k_split = kSurH;
-                gb.Zp = Zl[l - 2];
-                gb.H = dZl[cur ^ 1];
-                gb.HT = dZTl[cur ^ 1];
-                gb.err = err.ptr;
-                if (cgppd_check(launch_gemm(kGemmBwd, gb, st), "surrogate activation-gradient GEMM"))
-                    return -1;
-                cur ^= 1;
-            }
-            launch_row_reduce(dZTl[cur], kSurH, n, X.ptr, kSurIn, nullptr, G.ptr + kOffB1, G.ptr + kOffW1, st);
-        }
-        if (cgppd_check(cudaGetLastError(), "surrogate kernels"))
-            return -1;
-        if (loss_out && with_targets) {
-            float v = 0.f;
-            if (cgppd_check(cudaMemcpyAsync(&v, scalars.ptr, sizeof(float), cudaMemcpyDeviceToHost, st), "loss") ||
-                cgppd_check(cudaStreamSynchronize(st), "surrogate step"))
-                return -1;
-            *loss_out = v / (float)n;
-        }
-        return check_err();
+        NetRowsArgs r{};
+        r.X = dX;
+        r.rows = n;
+        r.P = P.ptr;
+        r.wtiles = wtiles.ptr;
+        r.o = dO;
+        r.err = err.ptr;
+        return cgppd_check(launch_net_rows(r, false, max_ctas, stream), "surrogate forward pass");
     }
 
-    int check_err()
+    // Enqueue the loss sum over n rows (n % 128 == 0, n <= batch) into *loss and, with
+    // `grad`, their gradient: into G, or straight into an Adam step of rate `lr` (lr > 0).
+    // `rows_of`: the batch's rows of dX / dY (targets clipped), or null for rows 0 .. n - 1.
+    int enqueue_step(const float *dX, const float *dY, const int *rows_of, float clip, int n, bool grad, float lr,
+                     float *loss)
     {
-        unsigned e = 0;
-        if (cgppd_check(cudaMemcpyAsync(&e, err.ptr, sizeof(unsigned), cudaMemcpyDeviceToHost, stream), "err") ||
+        const int ks = std::min(n, k_split);
+        if (grad && (n % ks != 0 || ks % 64 != 0))
+            return cgppd_fail("surrogate: batch must be a multiple of 64 (and of the split size)");
+        const int tiles = (n + kNetRows - 1) / kNetRows;
+        NetRowsArgs r{};
+        r.X = dX;
+        r.y = dY;
+        r.perm = rows_of;
+        r.clip = clip;
+        r.rows = n;
+        r.P = P.ptr;
+        r.wtiles = wtiles.ptr;
+        r.act = act.ptr;
+        r.xb = xb.ptr, r.dO = dO.ptr, r.r2 = r2.ptr;
+        r.err = err.ptr;
+        if (cgppd_check(launch_net_rows(r, true, max_ctas, stream), "surrogate forward and backward pass"))
+            return -1;
+        NetUpdateArgs u{};
+        u.wpart = wpart.ptr;
+        u.splits = n / ks;
+        u.act = act.ptr;
+        u.xb = xb.ptr, u.dO = dO.ptr, u.r2 = r2.ptr;
+        u.rows = n;
+        u.G = G.ptr;
+        u.loss_sum = loss;
+        if (!grad)
+            return cgppd_check(launch_net_update(u, kNetLossOnly, stream), "surrogate loss");
+        NetWgradArgs w{};
+        w.act = act.ptr;
+        w.tiles = tiles;
+        w.splits = u.splits;
+        w.split_tiles = ks / kNetRows;
+        w.part = wpart.ptr;
+        w.err = err.ptr;
+        if (cgppd_check(launch_net_wgrad(w, stream), "surrogate weight gradients"))
+            return -1;
+        if (lr > 0.f) {
+            ++adam_t;
+            u.P = P.ptr, u.m = am.ptr, u.v = av.ptr;
+            u.lr = lr, u.b1 = 0.9f, u.b2 = 0.999f, u.eps = 1e-8f;
+            u.c1 = 1.f - std::pow(u.b1, (float)adam_t), u.c2 = 1.f - std::pow(u.b2, (float)adam_t);
+            u.Wf = Wf.ptr, u.wtiles = wtiles.ptr;
+        }
+        return cgppd_check(launch_net_update(u, lr > 0.f ? kNetAdam : kNetGradient, stream), "surrogate update");
+    }
+
+    // Wait for the stream and report a GEMM that gave up; the loss sum at `loss` (if any)
+    // is in ends->loss_sum afterwards.
+    int finish(const float *loss = nullptr)
+    {
+        if (cgppd_check(cudaMemcpyAsync(&ends->err, err.ptr, sizeof(unsigned), cudaMemcpyDeviceToHost, stream), "err") ||
+            (loss && cgppd_check(cudaMemcpyAsync(&ends->loss_sum, loss, sizeof(float), cudaMemcpyDeviceToHost, stream),
+                                 "loss")) ||
             cgppd_check(cudaStreamSynchronize(stream), "surrogate sync"))
             return -1;
-        if (e)
+        if (ends->err)
             return cgppd_fail("surrogate: a tensor-core GEMM timed out waiting for its MMAs");
         return 0;
-    }
-
-    void adam(float lr)
-    {
-        ++adam_t;
-        const float b1 = 0.9f, b2 = 0.999f;
-        const float c1 = 1.f - std::pow(b1, (float)adam_t), c2 = 1.f - std::pow(b2, (float)adam_t);
-        launch_adam(P.ptr, G.ptr, am.ptr, av.ptr, kSurParams, lr, b1, b2, 1e-8f, c1, c2, stream);
-        launch_bf16_copies(P.ptr, Wf.ptr, Wt.ptr, stream);
     }
 
     int upload_dataset()
@@ -222,22 +214,22 @@ struct cgppd_surrogate {
         return 0;
     }
 
-    // predictions for rows [0, n) of host or device features (host if `host`)
+    // predictions for n rows of features (host or device memory), kStageRows at a time
     int predict(const float *Xsrc, int n, float *out_host)
     {
-        for (int s0 = 0; s0 < n; s0 += batch) {
-            const int cnt = std::min(batch, n - s0);
-            const int padded = (cnt + 127) / 128 * 128;
-            if (cgppd_check(cudaMemsetAsync(X.ptr, 0, (size_t)padded * kSurIn * sizeof(float), stream), "memset") ||
-                cgppd_check(cudaMemcpyAsync(X.ptr, Xsrc + (size_t)s0 * kSurIn, (size_t)cnt * kSurIn * sizeof(float),
-                                            cudaMemcpyDefault, stream),
-                            "features"))
-                return -1;
-            if (step(padded, false, false, nullptr))
-                return -1;
-            if (cgppd_check(cudaMemcpyAsync(out_host + s0, o.ptr, cnt * sizeof(float), cudaMemcpyDeviceToHost, stream),
+        const int chunk = std::min(n, kStageRows);
+        if (stageO.n < (size_t)chunk && (stageX.alloc((size_t)chunk * kSurIn) || stageO.alloc(chunk)))
+            return -1;
+        for (int s0 = 0; s0 < n; s0 += chunk) {
+            const int cnt = std::min(chunk, n - s0);
+            if (cgppd_check(cudaMemcpyAsync(stageX.ptr, Xsrc + (size_t)s0 * kSurIn,
+                                            (size_t)cnt * kSurIn * sizeof(float), cudaMemcpyDefault, stream),
+                            "features") ||
+                enqueue_forward(stageX.ptr, cnt, stageO.ptr) ||
+                cgppd_check(cudaMemcpyAsync(out_host + s0, stageO.ptr, cnt * sizeof(float), cudaMemcpyDeviceToHost,
+                                            stream),
                             "predictions") ||
-                cgppd_check(cudaStreamSynchronize(stream), "predict"))
+                finish())
                 return -1;
         }
         return 0;
@@ -286,13 +278,19 @@ int cgppd_surrogate_loss_grad(cgppd_surrogate *s, const float *X, const float *y
         return cgppd_fail("cgppd_surrogate_loss_grad: null argument");
     if (n <= 0 || n > s->batch || n % 128 != 0)
         return cgppd_fail("cgppd_surrogate_loss_grad: n must be a multiple of 128 no larger than the batch");
-    if (cgppd_check(cudaMemcpy(s->X.ptr, X, (size_t)n * kSurIn * sizeof(float), cudaMemcpyHostToDevice), "X") ||
-        cgppd_check(cudaMemcpy(s->y.ptr, y, (size_t)n * sizeof(float), cudaMemcpyHostToDevice), "y"))
+    if (cgppd_check(cudaMemcpyAsync(s->X.ptr, X, (size_t)n * kSurIn * sizeof(float), cudaMemcpyHostToDevice, s->stream),
+                    "X") ||
+        cgppd_check(cudaMemcpyAsync(s->y.ptr, y, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, s->stream), "y") ||
+        s->enqueue_step(s->X.ptr, s->y.ptr, nullptr, 0.f, n, grad != nullptr, 0.f, s->losses.ptr))
         return -1;
-    if (s->step(n, true, grad != nullptr, loss))
+    if (grad && cgppd_check(cudaMemcpyAsync(grad, s->G.ptr, kSurParams * sizeof(float), cudaMemcpyDeviceToHost,
+                                            s->stream),
+                            "grad"))
         return -1;
-    if (grad)
-        return cgppd_check(cudaMemcpy(grad, s->G.ptr, kSurParams * sizeof(float), cudaMemcpyDeviceToHost), "grad");
+    if (s->finish(s->losses.ptr))
+        return -1;
+    if (loss)
+        *loss = s->ends->loss_sum / (float)n;
     return 0;
 }
 
@@ -355,6 +353,8 @@ int cgppd_surrogate_train(cgppd_surrogate *s, int epochs, float lr, float clip, 
     std::vector<int> perm(ntrain);
     uint64_t rs = s->seed ^ 0x7A11ull;
     const long long nb = ntrain / B;
+    if (s->losses.n < (size_t)nb && s->losses.alloc(nb))
+        return -1;
     for (int e = 0; e < epochs; ++e) {
         std::iota(perm.begin(), perm.end(), 0);
         for (long long i = ntrain - 1; i > 0; --i) {
@@ -365,22 +365,22 @@ int cgppd_surrogate_train(cgppd_surrogate *s, int epochs, float lr, float clip, 
                                         s->stream),
                         "permutation"))
             return -1;
-        double sse = 0.0;
-        long long nlog = 0;
-        for (long long b = 0; b < nb; ++b) {
-            launch_gather_rows(s->dsX.ptr, s->dsY.ptr, s->perm.ptr + b * B, B, s->X.ptr, s->y.ptr, clip, s->stream);
-            float loss = 0.f;
-            const bool want_loss = (b == nb - 1) || (b % 16 == 0);
-            if (s->step(B, true, true, want_loss ? &loss : nullptr))
+        for (long long b = 0; b < nb; ++b)
+            if (s->enqueue_step(s->dsX.ptr, s->dsY.ptr, s->perm.ptr + b * B, clip, B, true, lr, s->losses.ptr + b))
                 return -1;
-            s->adam(lr);
-            if (want_loss) {
-                sse += (double)loss;
+        std::vector<float> sums(nb);
+        if (cgppd_check(cudaMemcpyAsync(sums.data(), s->losses.ptr, nb * sizeof(float), cudaMemcpyDeviceToHost,
+                                        s->stream),
+                        "training losses") ||
+            s->finish())
+            return -1;
+        double sse = 0.0;  // every 16th batch and the last
+        long long nlog = 0;
+        for (long long b = 0; b < nb; ++b)
+            if (b == nb - 1 || b % 16 == 0) {
+                sse += (double)(sums[b] / (float)B);
                 ++nlog;
             }
-        }
-        if (cgppd_check(cudaStreamSynchronize(s->stream), "training epoch"))
-            return -1;
         if (history) {
             history[2 * e] = (float)std::sqrt(sse / (double)std::max(1ll, nlog));
             history[2 * e + 1] = -1.f;

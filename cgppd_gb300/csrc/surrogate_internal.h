@@ -4,41 +4,63 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include "surrogate.cuh"
+
 struct cgppd_surrogate;
 
 namespace cgppd {
 
-enum GemmMode { kGemmStore = 0, kGemmFwd = 1, kGemmBwd = 2 };
+constexpr int kNetRows = 64;                       // batch rows of one tile
+constexpr int kNetTileElems = kSurH * kNetRows;    // a 256 x 64 bf16 tile image (tc05.cuh)
 
-// C = A * B^T on the tcgen05 tensor cores, A [M][K], B [256][K] (bf16, K-major).
-struct GemmArgs {
-    const __nv_bfloat16 *A;   // [M][K]
-    const __nv_bfloat16 *B;   // [256][K]
-    int M, K, k_split;        // M % 128 == 0, K % k_split == 0, k_split % 64 == 0
-    float *C;                 // store: [K / k_split][M][256]
-    const float *bias;        // fwd
-    float *Z;                 // fwd: [M][256]
-    __nv_bfloat16 *H, *HT;    // fwd: [M][256], [256][M]; bwd: dZ, dZ^T
-    const float *Zp;          // bwd: pre-activation of the layer below, [M][256]
+// Tile images of a batch, [kind][tile][256 x 64]: activations of layers 1..4 and
+// pre-activation gradients of layers 1..4.
+enum NetAct { kActH1 = 0, kActZ1 = 4, kActKinds = 8 };
+
+struct NetRowsArgs {
+    const float *X;                // [..][8] features
+    const float *y;                // targets (backward)
+    const int *perm;               // row -> row of X and y (targets then clipped to +-clip), or null
+    float clip;
+    int rows;
+    const float *P;                // FP32 master parameters
+    const __nv_bfloat16 *wtiles;   // [6][4][256 x 64]: W2 W3 W4, then their transposes W4 W3 W2
+    float *o;                      // [rows] predictions, or null
+    __nv_bfloat16 *act;            // [kActKinds][tiles][256 x 64] (backward)
+    float *xb, *dO, *r2;           // (backward) the batch's features, [8][rows]; 2 (o - y) / rows; (o - y)^2
     unsigned *err;
 };
 
-cudaError_t launch_gemm(int mode, const GemmArgs &g, cudaStream_t st);
-void launch_layer1_fwd(const float *X, const float *P, float *Z, __nv_bfloat16 *H, __nv_bfloat16 *HT, int B,
-                       cudaStream_t st);
-void launch_out_fwd(const __nv_bfloat16 *H4, const float *P, const float *y, float *o, float *dO, float *r2, int B,
-                    cudaStream_t st);
-void launch_out_bwd(const float *dO, const float *P, const float *Z4, __nv_bfloat16 *dZ, __nv_bfloat16 *dZT, int B,
-                    cudaStream_t st);
-void launch_row_reduce(const __nv_bfloat16 *MT, int rows, int B, const float *X, int nx, const float *u,
-                       float *sum_out, float *dot_out, cudaStream_t st);
-void launch_vec_sum(const float *v, int n, float *out, cudaStream_t st);
-void launch_splitk_reduce(const float *part, int splits, int n, float *out, cudaStream_t st);
-void launch_adam(float *P, const float *G, float *m, float *v, int n, float lr, float b1, float b2, float eps,
-                 float c1, float c2, cudaStream_t st);
-void launch_bf16_copies(const float *P, __nv_bfloat16 *Wf, __nv_bfloat16 *Wt, cudaStream_t st);
-void launch_gather_rows(const float *X, const float *y, const int *perm, int n, float *Xb, float *yb, float clip,
-                        cudaStream_t st);
+struct NetWgradArgs {
+    const __nv_bfloat16 *act;
+    int tiles, splits, split_tiles;  // tiles = splits * split_tiles
+    float *part;                     // [3][splits][256][256]
+    unsigned *err;
+};
+
+struct NetUpdateArgs {
+    const float *wpart;   // of k_net_wgrad
+    int splits;
+    const __nv_bfloat16 *act;  // of k_net_rows, and its xb, dO, r2
+    const float *xb, *dO, *r2;
+    int rows;
+    int first;            // first block of the work (set by the launcher)
+    float *G;             // gradient (no Adam step)
+    float *loss_sum;      // sum of squared residuals
+    float *P, *m, *v;     // Adam
+    float lr, b1, b2, eps, c1, c2;
+    __nv_bfloat16 *Wf, *wtiles;
+};
+
+// What k_net_update does with the sums: end the loss alone, store the gradient, or take
+// an Adam step.
+enum NetUpdateMode { kNetLossOnly = 0, kNetGradient, kNetAdam };
+
+cudaError_t net_set_limits();
+cudaError_t launch_net_rows(const NetRowsArgs &a, bool backward, int max_ctas, cudaStream_t st);
+cudaError_t launch_net_wgrad(const NetWgradArgs &a, cudaStream_t st);
+cudaError_t launch_net_update(const NetUpdateArgs &a, NetUpdateMode mode, cudaStream_t st);
+cudaError_t launch_net_copies(const float *P, __nv_bfloat16 *Wf, __nv_bfloat16 *wtiles, cudaStream_t st);
 
 // The engine reads a trained surrogate's FP32 parameters and BF16 forward weights.
 const float *surrogate_device_params(const cgppd_surrogate *s);

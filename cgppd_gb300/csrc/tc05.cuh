@@ -2,13 +2,17 @@
 // tensor-memory allocation, shared-memory matrix descriptors, the single-thread MMA
 // issue, commit to an mbarrier with a bounded wait, and tensor-memory loads.
 //
-// Operand layout used throughout: K-major, no swizzle.  A tile of R rows x 64 bf16 is
-// stored as core matrices of 8 rows x 16 bytes (128 contiguous bytes, rows 16 bytes
-// apart); core matrix (row group g, 16-byte column c) sits at (g * 8 + c) * 128.
-// Neighbouring core matrices along K are therefore 128 bytes apart (the descriptor's
-// leading-dimension offset) and neighbouring 8-row groups 1024 bytes apart (its
-// stride-dimension offset).  One kind::f16 MMA consumes K = 16, i.e. two core matrices
-// along K: the k-th MMA of a 64-wide chunk starts 256 * k bytes into the tile.
+// Operand layout used throughout: no swizzle.  A tile of R rows x 64 bf16 is stored as
+// core matrices of 8 rows x 16 bytes (128 contiguous bytes, rows 16 bytes apart); core
+// matrix (row group g, 16-byte column c) sits at (g * 8 + c) * 128.  The same image
+// serves two operands:
+//   rows x K (K-major): neighbouring core matrices along K are 128 bytes apart (the
+//     descriptor's leading-dimension offset) and neighbouring 8-row groups 1024 bytes
+//     apart (its stride-dimension offset).  One kind::f16 MMA consumes K = 16, i.e. two
+//     core matrices along K: the k-th MMA of a 64-wide chunk starts 256 * k bytes in.
+//   K x columns (MN-major, the row index is K and the 64 columns are M or N): 8-row
+//     groups along K are 1024 bytes apart (leading-dimension offset), 8-column groups
+//     128 bytes (stride-dimension offset); the k-th MMA starts 2048 * k bytes in.
 #pragma once
 
 #include <cstdint>
@@ -16,35 +20,41 @@
 namespace cgppd {
 namespace tc05 {
 
-constexpr int kChunkK = 64;          // bf16 elements per staged K chunk (128 bytes per row)
-constexpr uint32_t kLBO = 128;       // bytes between core matrices adjacent in K
-constexpr uint32_t kSBO = 1024;      // bytes between 8-row groups
+constexpr int kChunkK = 64;          // bf16 elements per tile row (128 bytes)
+constexpr uint32_t kColStep = 128;   // bytes between core matrices adjacent along a row
+constexpr uint32_t kRowStep = 1024;  // bytes between 8-row groups
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p)
 {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// Byte offset of the 16-byte piece (row r, piece c) of a staged K-major tile.
-__device__ __forceinline__ uint32_t tile_offset(int r, int c) { return (uint32_t)(((r >> 3) * 8 + c) * 128 + (r & 7) * 16); }
+// Byte offset of the 16-byte piece (row r, piece c) of a tile.
+__host__ __device__ __forceinline__ uint32_t tile_offset(int r, int c) { return (uint32_t)(((r >> 3) * 8 + c) * 128 + (r & 7) * 16); }
 
 // Shared-memory matrix descriptor: start address, LBO, SBO (all >> 4), descriptor
 // version 1 at bits 46-47, base offset 0, absolute LBO mode, no swizzle (bits 61-63 = 0).
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr)
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo)
 {
     uint64_t d = 0;
     d |= (uint64_t)((addr & 0x3FFFFu) >> 4);
-    d |= (uint64_t)((kLBO >> 4) & 0x3FFFu) << 16;
-    d |= (uint64_t)((kSBO >> 4) & 0x3FFFu) << 32;
+    d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
+    d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
     d |= (uint64_t)1 << 46;
     return d;
 }
 
+// Descriptors of a tile as a rows x K operand and as a K x columns operand.
+__device__ __forceinline__ uint64_t desc_k_major(uint32_t addr) { return smem_desc(addr, kColStep, kRowStep); }
+__device__ __forceinline__ uint64_t desc_mn_major(uint32_t addr) { return smem_desc(addr, kRowStep, kColStep); }
+
 // Instruction descriptor of kind::f16: D f32 (bits 4-5 = 1), A and B bf16 (bits 7-9 and
-// 10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3 at bits 17-22, M >> 4 at bits 24-28.
-__host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N)
+// 10-12 = 1), A K-major (bit 15 = 0), B K-major or MN-major (bit 16), N >> 3 at bits
+// 17-22, M >> 4 at bits 24-28.
+__host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N, bool b_mn_major)
 {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(N >> 3) << 17) |
+           ((uint32_t)(M >> 4) << 24);
 }
 
 __device__ __forceinline__ void tmem_alloc(uint32_t *dst_smem, uint32_t ncols)
@@ -96,7 +106,36 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, long l
     return false;
 }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread.
+// Announce `bytes` of bulk copies on `bar` (one arrival).
+__device__ __forceinline__ void mbar_expect(uint64_t *bar, uint32_t bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes)
+                 : "memory");
+}
+
+// Bulk copy of `bytes` (a multiple of 16, both addresses 16-byte aligned) from global to
+// shared memory; completes on `bar`.
+__device__ __forceinline__ void bulk_load(uint32_t dst_smem, const void *src, uint32_t bytes, uint64_t *bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+                     dst_smem),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+
+// Bulk copy from shared to global memory in this thread's current bulk group.
+__device__ __forceinline__ void bulk_store(void *dst, uint32_t src_smem, uint32_t bytes)
+{
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(dst), "r"(src_smem), "r"(bytes)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+}
+
+// Every bulk store of this thread has read its shared memory (and, `done`, is written).
+__device__ __forceinline__ void bulk_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory"); }
+__device__ __forceinline__ void bulk_store_wait_done() { asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory"); }
+
+// D[tmem] (+)= A[smem] * B[smem], issued by one thread.
 __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, bool accumulate)
 {
     asm volatile(
