@@ -35,7 +35,7 @@ cudaError_t launch_pose_samples(const EngineArgs &a, const int4 *items, int n, u
 cudaError_t launch_mc_block(const EngineArgs &a, int total_replicas, int nsteps, int threads, size_t smem,
                             cudaStream_t stream);
 cudaError_t set_mc_smem_limit(size_t smem);
-cudaError_t launch_init_energy(const EngineArgs &a, int total_replicas, size_t smem, double *potential_out,
+cudaError_t launch_init_energy(const EngineArgs &a, int total_replicas, int n_work, double *potential_out,
                                cudaStream_t stream);
 cudaError_t launch_exchange(const EngineArgs &a, int nsims, int total_replicas, int steps_per_block,
                             cudaStream_t stream);
@@ -113,6 +113,60 @@ void frame_residues(const HostMolecule &hm, int &f0, int &f1, int &f2)
     }
 }
 
+// The work list of k_init_pairs: whole consecutive molecules are grouped up to kInitI
+// (kInitJ) residues for the first (second) side of a pair block, every two groups that
+// hold a pair a < b are a task, and each flexible molecule is one; (replica, task) items
+// by decreasing pairs.
+void plan_init(const std::vector<DevSim> &sims, const std::vector<DevMol> &mols, std::vector<InitTask> &tasks,
+               std::vector<int2> &work)
+{
+    std::vector<std::pair<double, int>> cost;  // (pairs, simulation) of each task
+    for (size_t s = 0; s < sims.size(); ++s) {
+        const DevSim &S = sims[s];
+        const DevMol *m = mols.data() + S.mol_off;
+        auto groups = [&](int residues, int molecules) {
+            std::vector<std::pair<int, int>> g;
+            int n = 0;
+            for (int k = 0; k < S.M; ++k) {
+                if (g.empty() || n + m[k].count > residues || g.back().second >= molecules) {
+                    g.push_back({k, 0});
+                    n = 0;
+                }
+                ++g.back().second;
+                n += m[k].count;
+            }
+            return g;
+        };
+        auto residues = [&](std::pair<int, int> g) {
+            double n = 0.0;
+            for (int k = g.first; k < g.first + g.second; ++k)
+                n += m[k].count;
+            return n;
+        };
+        const auto first = groups(kInitI, kInitSegs), second = groups(kInitJ, kInitMols);
+        for (const auto &x : first)
+            for (const auto &y : second)
+                if (y.first + y.second - 1 > x.first) {
+                    tasks.push_back(InitTask{x.first, x.second, y.first, y.second});
+                    cost.push_back({residues(x) * residues(y), (int)s});
+                }
+        for (int k = 0; k < S.M; ++k)
+            if (m[k].flags & kMolFlexible) {
+                tasks.push_back(InitTask{k, 1, 0, 0});
+                cost.push_back({2.0 * m[k].count * m[k].count, (int)s});
+            }
+    }
+    std::vector<int> order(tasks.size());
+    for (size_t k = 0; k < order.size(); ++k)
+        order[k] = (int)k;
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x].first > cost[y].first; });
+    for (int k : order) {
+        const DevSim &S = sims[cost[k].second];
+        for (int r = 0; r < S.R; ++r)
+            work.push_back(make_int2(S.rep_off + r, k));
+    }
+}
+
 }  // namespace
 
 struct cgppd_engine {
@@ -158,6 +212,9 @@ struct cgppd_engine {
     DevBuf<float4> d_torsV, d_torsS;
     DevBuf<int> d_branch, d_localres, d_crankres;
     DevBuf<int2> d_tiles;
+    DevBuf<InitTask> d_init_tasks;
+    DevBuf<int2> d_init_work;
+    int init_work = 0;
     DevBuf<float> d_table;
     DevBuf<float4> d_pos, d_rel, d_center;
     DevBuf<double> d_emat, d_intra, d_potential, d_scratch_pot, d_scratch_emat, d_scratch_intra;
@@ -214,6 +271,8 @@ struct cgppd_engine {
         a.localres = d_localres.ptr;
         a.crankres = d_crankres.ptr;
         a.tiles = d_tiles.ptr;
+        a.init_tasks = d_init_tasks.ptr;
+        a.init_work = d_init_work.ptr;
         a.table = d_table.ptr;
         a.pos = d_pos.ptr;
         a.rel = d_rel.ptr;
@@ -576,7 +635,14 @@ int cgppd_engine::build()
     std::stable_sort(rep_order.begin(), rep_order.end(),
                      [&](int x, int y) { return sim_work[rep_sim[x]] > sim_work[rep_sim[y]]; });
 
+    std::vector<InitTask> init_tasks;
+    std::vector<int2> work;
+    plan_init(h_sims, h_mols, init_tasks, work);
+    init_work = (int)work.size();
+
     int rc = 0;
+    rc |= d_init_tasks.upload(init_tasks);
+    rc |= d_init_work.upload(work);
     rc |= d_sims.upload(h_sims);
     rc |= d_rep_sim.upload(rep_sim);
     rc |= d_rep_order.upload(rep_order);
@@ -964,7 +1030,7 @@ int cgppd_engine_finalize(cgppd_engine *e, int cluster, int threads)
     if (cgppd_check(cudaStreamCreateWithFlags(&e->own_stream, cudaStreamNonBlocking), "engine stream") != 0)
         return -1;
     EngineArgs a = e->args();
-    if (cgppd_check(launch_init_energy(a, e->total_replicas, s_init, e->d_potential.ptr, e->own_stream),
+    if (cgppd_check(launch_init_energy(a, e->total_replicas, e->init_work, e->d_potential.ptr, e->own_stream),
                     "initial energy") != 0)
         return -1;
     if (cgppd_check(cudaStreamSynchronize(e->own_stream), "initial energy") != 0)
@@ -1109,7 +1175,6 @@ int cgppd_engine_recompute(cgppd_engine *e, double *out, int write_state)
     if (cgppd_check(cudaStreamSynchronize(e->own_stream), "recompute") != 0)
         return -1;
     EngineArgs a = e->args();
-    const size_t s_init = engine_smem_bytes(e->max_mol, e->max_n, e->max_m, 1, 0, e->any_flexible, 0, nullptr);
     double *dst = write_state ? e->d_potential.ptr : e->d_scratch_pot.ptr;
     if (!write_state) {
         // evaluate into scratch copies so the running state is untouched
@@ -1120,7 +1185,7 @@ int cgppd_engine_recompute(cgppd_engine *e, double *out, int write_state)
         a.emat = e->d_scratch_emat.ptr;
         a.intra = e->d_scratch_intra.ptr;
     }
-    if (cgppd_check(launch_init_energy(a, e->total_replicas, s_init, dst, e->own_stream), "recompute") != 0)
+    if (cgppd_check(launch_init_energy(a, e->total_replicas, e->init_work, dst, e->own_stream), "recompute") != 0)
         return -1;
     if (cgppd_check(cudaStreamSynchronize(e->own_stream), "recompute") != 0)
         return -1;
@@ -1239,8 +1304,7 @@ int cgppd_engine_upload(cgppd_engine *e, int sim, const float *pos4, const float
         rc |= cgppd_check(cudaMemcpyAsync(e->d_center.ptr + S.molst_off, centers4, sizeof(float4) * S.M * S.R,
                                           cudaMemcpyHostToDevice, st), "upload centres");
     if (rc == 0 && recompute) {
-        const size_t s_init = engine_smem_bytes(e->max_mol, e->max_n, e->max_m, 1, 0, e->any_flexible, 0, nullptr);
-        rc |= cgppd_check(launch_init_energy(e->args(), e->total_replicas, s_init, e->d_potential.ptr, st),
+        rc |= cgppd_check(launch_init_energy(e->args(), e->total_replicas, e->init_work, e->d_potential.ptr, st),
                           "upload recompute");
     }
     return rc ? -1 : 0;

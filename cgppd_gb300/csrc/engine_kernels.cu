@@ -1916,115 +1916,402 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
 
 // ------------------------------------------------------------------ initial energies
 
-// CTA (g, a): row a of replica g's matrix for b > a, and the internal energy of a.
-__global__ void __launch_bounds__(256) k_init_rows(EngineArgs a)
+constexpr int kInitThreads = kInitJ / 2;  // two residues j a thread
+
+// Lennard-Jones terms of one residue i with a thread's two residues j (pair_term's
+// arithmetic on packed halves; the repulsive branch is left to repulsive2), and what the
+// Debye-Hueckel term needs.
+struct Pair2 {
+    f2 u, r2, inv, m4, s6;
+};
+
+// The two residues j: negated positions, the image shift -L k, half radii, charges and
+// their columns of the contact table (bytes).
+struct Other2 {
+    f2 nx, ny, nz, sx, sy, sz, w, q;
+    const char *c0, *c1;
+};
+
+// MI 0: every pair takes j as it is; 1: j's image is the same for all i (nearest the
+// segment's middle), the shift added to each difference; 2: the minimum image per pair.
+// The difference is min_image's in all three, bit for bit.
+template <int MI>
+__device__ __forceinline__ f2 image2(f2 xi, f2 nxj, f2 shift, f2 L, f2 invL)
 {
-    extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ FF s_red[kMaxWarps];
-    const int t = threadIdx.x, T = blockDim.x;
-    const int g = blockIdx.x / a.max_m, am = blockIdx.x % a.max_m;
-    const int s = a.rep_sim[g];
-    const DevSim S = a.sims[s];
-    if (am >= S.M)
-        return;
-    const int r = g - S.rep_off, N = S.N, M = S.M;
-    const SmemLayout Ly = smem_layout(a.max_mol, a.max_n, a.max_m, a.max_n, 0, a.any_flexible);
-    float *s_table = reinterpret_cast<float *>(smem + Ly.table);
-    float4 *s_ipos = reinterpret_cast<float4 *>(smem + Ly.ipos);
-    float2 *s_iq = reinterpret_cast<float2 *>(smem + Ly.iq);
-    int4 *s_iexcl = reinterpret_cast<int4 *>(smem + Ly.iexcl);
-    load_table(s_table, a.table, t, T);
-    const DevMol mol = a.mols[S.mol_off + am];
-    const long long st0 = S.state_off + (long long)r * N;
-    const float4 *stat = a.rstat + S.res_off;
-    const int4 *excl = a.rexcl + S.res_off;
-    const int n = mol.count, start = mol.start;
-    for (int i = t; i < n; i += T) {
-        const float4 p = a.pos[st0 + start + i];
-        const float4 sr = stat[start + i];
-        s_ipos[i] = make_float4(p.x, p.y, p.z, sr.x);
-        s_iq[i] = make_float2(sr.y, sr.z);
-        s_iexcl[i] = excl[start + i];
+    f2 d = f2_add(xi, nxj);
+    if (MI == 1)
+        d = f2_add(d, shift);
+    if (MI == 2) {
+        const f2 magic = f2_dup(12582912.0f), back = f2_dup(-12582912.0f);
+        d = f2_fma(L, f2_add(f2_fma(d, invL, magic), back), d);  // (L holds -L)
     }
-    __syncthreads();
+    return d;
+}
+
+template <int MI>
+__device__ __forceinline__ Pair2 pair2(ulonglong2 xy, ulonglong2 zw, int trow, const Other2 &o, f2 L, f2 invL)
+{
+    Pair2 p;
+    const f2 dx = image2<MI>(xy.x, o.nx, o.sx, L, invL);
+    const f2 dy = image2<MI>(xy.y, o.ny, o.sy, L, invL);
+    const f2 dz = image2<MI>(zw.x, o.nz, o.sz, L, invL);
+    p.r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
+    float ra, rb;
+    f2_unpack(p.r2, ra, rb);
+    p.inv = f2_pack(rsqrt_sfu(ra), rsqrt_sfu(rb));
+    p.m4 = f2_pack(*reinterpret_cast<const float *>(o.c0 + trow), *reinterpret_cast<const float *>(o.c1 + trow));
+    const f2 so = f2_mul(f2_add(zw.y, o.w), p.inv), s2 = f2_mul(so, so);
+    p.s6 = f2_mul(f2_mul(s2, s2), s2);
+    float sa, sb;
+    f2_unpack(p.s6, sa, sb);
+    p.u = f2_mul(p.m4, f2_fma(p.s6, p.s6, f2_pack(-sa, -sb)));
+    return p;
+}
+
+// Whether a pair of p lies in the repulsive branch's range (s6 > 1/2: closer than
+// 2^(1/6) sigma; rare, so the branch is taken out of the straight path).
+__device__ __forceinline__ bool close2(const Pair2 &p)
+{
+    float a, b;
+    f2_unpack(p.s6, a, b);
+    return fmaxf(a, b) > 0.5f;
+}
+
+__device__ __forceinline__ void repulsive2(Pair2 &p)
+{
+    float a, b, ma, mb, ua, ub;
+    f2_unpack(p.s6, a, b);
+    f2_unpack(p.m4, ma, mb);
+    f2_unpack(p.u, ua, ub);
+    if (ma < 0.0f && a > 0.5f)
+        ua = fmaf(-0.5f, ma, -ua);
+    if (mb < 0.0f && b > 0.5f)
+        ub = fmaf(-0.5f, mb, -ub);
+    p.u = f2_pack(ua, ub);
+}
+
+__device__ __forceinline__ f2 with_dh2(const Pair2 &p, float qi, f2 qj)
+{
+    const f2 arg = f2_mul(f2_mul(p.r2, p.inv), f2_dup(-kLog2e / kXi));
+    float ea, eb;
+    f2_unpack(arg, ea, eb);
+    const f2 e = f2_mul(f2_mul(f2_dup(qi), qj), f2_pack(ex2_sfu(ea), ex2_sfu(eb)));
+    return f2_fma(e, p.inv, p.u);
+}
+
+// The residues [i, end) of one segment with a thread's two residues j, summed in order of
+// i and folded into the float-float accumulators after every 32nd residue of the molecule
+// (`phase`: the first residue's place in it).
+template <int MI>
+__device__ __forceinline__ void init_span(const float4 *s_xy, const float4 *s_zw, const float2 *s_qt, int i, int end,
+                                          int phase, const Other2 &o, float L, float invL, f2 &part, FF &e0, FF &e1)
+{
+    const ulonglong2 *xy = reinterpret_cast<const ulonglong2 *>(s_xy), *zw = reinterpret_cast<const ulonglong2 *>(s_zw);
+    const f2 L2 = f2_dup(-L), invL2 = f2_dup(invL);
+    auto add = [&](const Pair2 &p, int k) {
+        const float qi = s_qt[k].x;
+        part = f2_add(part, qi != 0.0f ? with_dh2(p, qi, o.q) : p.u);
+    };
+    while (i < end) {
+        const int stop = min(end, i + 32 - (phase & 31));
+        phase += stop - i;
+        for (; i + 1 < stop; i += 2) {
+            Pair2 p = pair2<MI>(xy[i], zw[i], __float_as_int(s_qt[i].y), o, L2, invL2);
+            Pair2 q = pair2<MI>(xy[i + 1], zw[i + 1], __float_as_int(s_qt[i + 1].y), o, L2, invL2);
+            if (close2(p) || close2(q)) {
+                repulsive2(p);
+                repulsive2(q);
+            }
+            add(p, i);
+            add(q, i + 1);
+        }
+        if (i < stop) {
+            Pair2 p = pair2<MI>(xy[i], zw[i], __float_as_int(s_qt[i].y), o, L2, invL2);
+            repulsive2(p);
+            add(p, i);
+            ++i;
+        }
+        if ((phase & 31) == 0) {
+            float a, b;
+            f2_unpack(part, a, b);
+            ff_add(e0, a);
+            ff_add(e1, b);
+            part = 0ull;
+        }
+    }
+}
+
+// Energies from scratch, one InitTask of one replica a CTA: the pair matrix's entries of
+// two groups of whole molecules, or a flexible molecule's internal energy.  Each thread
+// keeps two residues j of the second group in registers and reads the first group's
+// residues from shared memory, where each value stands twice (the packed operand); a
+// molecule's pairs then sum per j and, at the end of the task, per molecule by one warp.
+// Grouping whole molecules keeps the lanes of a warp busy whatever the molecules' sizes
+// and lets one CTA finish every entry it starts (no partial sums in memory).  Pairs skip
+// the minimum image where the first molecule's bounding box and j leave only one image
+// possible.  Crowded configuration (24 proteins, 40 crowders of 20 residues, 32
+// replicas, 151 M pairs): one CTA per molecule and replica with a loop and a CTA
+// reduction per other molecule took 1243 us.
+__global__ void __launch_bounds__(kInitThreads) k_init_pairs(EngineArgs a)
+{
+    __shared__ __align__(16) float s_table[kTableStride * kTableStride];
+    __shared__ float4 s_xy[kInitI], s_zw[kInitI];  // (x, x, y, y), (z, z, sigma/2, sigma/2)
+    __shared__ float2 s_qt[kInitI];                // charge, table row (bytes)
+    __shared__ float2 s_e[kInitSegs][kInitJ];      // per molecule of the first group and residue j
+    __shared__ FF s_sum[kInitSegs][kInitMols];     // running sums per pair of molecules
+    __shared__ float4 s_mid[kInitSegs], s_half[kInitSegs];
+    __shared__ int2 s_mol[kInitSegs];              // first and end residue of the first group's molecules
+    __shared__ FF s_red[kMaxWarps];
+    const int t = threadIdx.x, T = kInitThreads, warp = t >> 5, lane = t & 31, NW = T >> 5;
+    const int2 work = a.init_work[blockIdx.x];
+    const InitTask task = a.init_tasks[work.y];
+    const int g = work.x, s = a.rep_sim[g];
+    const DevSim &S = a.sims[s];
+    const int r = g - S.rep_off, N = S.N, M = S.M, crowd_start = S.crowd_start, non_crowders = S.non_crowders;
+    const DevMol *mols = a.mols + S.mol_off;
+    const float4 *pos = a.pos + S.state_off + (long long)r * N;
+    const float4 *stat = a.rstat + S.res_off;
     const float L = S.box, invL = (S.box != 0.0f) ? 1.0f / S.box : 0.0f;
-    double *E = a.emat + S.emat_off + (long long)r * M * M;
-    for (int b = am + 1; b < M; ++b) {
-        const DevMol mb = a.mols[S.mol_off + b];
-        const bool crowd = S.crowd_start >= 0 && (am >= S.non_crowders || b >= S.non_crowders);
+    load_table(s_table, a.table, t, T);
+
+    if (task.nb == 0) {
+        // internal energy of a flexible molecule: unexcluded pairs (i < j, threads over j),
+        // indirect neighbours, bonded terms
+        const DevMol &mol = mols[task.a0];
+        const int n = mol.count;
+        const float4 *p = pos + mol.start;
+        const int4 *excl = a.rexcl + S.res_off + mol.start;
+        __shared__ int4 s_ex[kInitI];
         FF acc{0.f, 0.f};
-        for (int jj = t; jj < mb.count; jj += T) {
-            const int j = mb.start + jj;
-            const float4 pj = a.pos[st0 + j];
-            const float4 sj = stat[j];
-            const float4 rj = make_float4(pj.x, pj.y, pj.z, sj.x);
-            const float2 qj = make_float2(sj.y, sj.z);
+        for (int jc = 0; jc < n; jc += T) {
+            const int j = jc + t;
+            float4 rj = make_float4(0.f, 0.f, 0.f, 0.f);
+            float2 qj = make_float2(0.f, 0.f);
+            int4 ej = make_int4(0, 0, 0, 0);
+            if (j < n) {
+                const float4 pj = p[j], sj = stat[mol.start + j];
+                rj = make_float4(pj.x, pj.y, pj.z, sj.x);
+                qj = make_float2(sj.y, sj.z);
+                ej = excl[j];
+            }
             float part = 0.f;
-            for (int i = 0; i < n; ++i) {
-                part += crowd ? crowder_kcal(s_ipos[i], rj, L, invL)
-                              : pair_kcal(s_ipos[i], s_iq[i], rj, qj, s_table, L, invL);
-                if ((i & 31) == 31) {
-                    ff_add(acc, part);
-                    part = 0.f;
+            const int last = min(n, jc + T);
+            for (int ib = 0; ib < last; ib += kInitI) {
+                __syncthreads();
+                if (ib + t < last) {
+                    const float4 pi = p[ib + t], si = stat[mol.start + ib + t];
+                    s_xy[t] = make_float4(pi.x, pi.y, pi.z, si.x);
+                    s_qt[t] = make_float2(si.y, si.z);
+                    s_ex[t] = excl[ib + t];
+                }
+                __syncthreads();
+                const int end = (j < n) ? min(kInitI, j - ib) : 0;
+                for (int i = 0; i < end; ++i) {
+                    if (!intra_excluded(s_ex[i], ej))
+                        part += pair_kcal(s_xy[i], s_qt[i], rj, qj, s_table, L, invL);
+                    if ((i & 31) == 31) {
+                        ff_add(acc, part);
+                        part = 0.f;
+                    }
                 }
             }
             ff_add(acc, part);
         }
-        const double v = block_sum_ff(acc, s_red);
-        if (t == 0) {
-            E[(long long)am * M + b] = v;
-            E[(long long)b * M + am] = v;
-        }
-    }
-    if (t == 0)
-        E[(long long)am * M + am] = 0.0;
-    FF iacc{0.f, 0.f};
-    if (mol.flags & kMolFlexible) {
-        for (int j = t; j < n; j += T) {
-            const float4 pj = s_ipos[j];
-            const float2 qj = s_iq[j];
-            const int4 ej = s_iexcl[j];
-            float part = 0.f;
-            for (int i = 0; i < j; ++i) {
-                if (!intra_excluded(s_iexcl[i], ej))
-                    part += pair_kcal(s_ipos[i], s_iq[i], pj, qj, s_table, L, invL);
-                if ((i & 31) == 31) {
-                    ff_add(iacc, part);
-                    part = 0.f;
-                }
-            }
-            ff_add(iacc, part);
-        }
+        __syncthreads();
         for (int k = t; k < mol.nind; k += T) {
             const int2 pr = a.indsub[mol.ind_off + k];
-            ff_add(iacc, -pair_kcal(s_ipos[pr.x], s_iq[pr.x], s_ipos[pr.y], s_iq[pr.y], s_table, L, invL));
+            const float4 pa = p[pr.x], pb = p[pr.y], sa = stat[mol.start + pr.x], sb = stat[mol.start + pr.y];
+            ff_add(acc, -pair_kcal(make_float4(pa.x, pa.y, pa.z, sa.x), make_float2(sa.y, sa.z),
+                                   make_float4(pb.x, pb.y, pb.z, sb.x), make_float2(sb.y, sb.z), s_table, L, invL));
         }
-        bonded_terms(global_lists(a), mol, s_ipos, L, invL, t, T, iacc);
+        bonded_terms(global_lists(a), mol, p, L, invL, t, T, acc);
+        const double v = block_sum_ff(acc, s_red);
+        if (t == 0)
+            a.intra[S.molst_off + (long long)r * M + task.a0] = v;
+        return;
     }
-    const double v = block_sum_ff(iacc, s_red);
-    if (t == 0)
-        a.intra[S.molst_off + (long long)r * M + am] = (mol.flags & kMolFlexible) ? v : 0.0;
+
+    const int a1 = task.a0 + task.na, b1 = task.b0 + task.nb;
+    const int i0 = mols[task.a0].start, i1 = mols[a1 - 1].start + mols[a1 - 1].count;
+    const int j0 = mols[task.b0].start, j1 = mols[b1 - 1].start + mols[b1 - 1].count;
+    for (int k = t; k < task.na * task.nb; k += T)
+        s_sum[k / task.nb][k % task.nb] = FF{0.f, 0.f};
+    // middle and half extent of each molecule of the first group
+    for (int k = warp; k < task.na; k += NW) {
+        const DevMol &mk = mols[task.a0 + k];
+        float3 lo = make_float3(3e38f, 3e38f, 3e38f), hi = make_float3(-3e38f, -3e38f, -3e38f);
+        for (int i = lane; i < mk.count; i += 32) {
+            const float4 p = pos[mk.start + i];
+            lo = make_float3(fminf(lo.x, p.x), fminf(lo.y, p.y), fminf(lo.z, p.z));
+            hi = make_float3(fmaxf(hi.x, p.x), fmaxf(hi.y, p.y), fmaxf(hi.z, p.z));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, o));
+            lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, o));
+            lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, o));
+            hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, o));
+            hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, o));
+            hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, o));
+        }
+        if (lane == 0) {
+            s_mol[k] = make_int2(mk.start, mk.start + mk.count);
+            s_mid[k] = make_float4(0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z), 0.f);
+            s_half[k] = make_float4(0.5f * (hi.x - lo.x), 0.5f * (hi.y - lo.y), 0.5f * (hi.z - lo.z), 0.f);
+        }
+    }
+    for (int jc = j0; jc < j1; jc += kInitJ) {
+        // this thread's residues (past the end: the last one, its sums are not read)
+        const int ja = jc + 2 * t, jb = ja + 1;
+        const int ka = min(ja, j1 - 1), kb = min(jb, j1 - 1);
+        const float4 pa = pos[ka], pb = pos[kb], sa = stat[ka], sb = stat[kb];
+        const int ma = __float_as_int(sa.w), mb = __float_as_int(sb.w);
+        Other2 o;
+        o.nx = f2_pack(-pa.x, -pb.x), o.ny = f2_pack(-pa.y, -pb.y), o.nz = f2_pack(-pa.z, -pb.z);
+        o.w = f2_pack(sa.x, sb.x), o.q = f2_pack(sa.y, sb.y);
+        o.c0 = reinterpret_cast<const char *>(s_table + __float_as_int(sa.z));
+        o.c1 = reinterpret_cast<const char *>(s_table + __float_as_int(sb.z));
+        f2 part = 0ull;
+        FF e0{0.f, 0.f}, e1{0.f, 0.f};
+        for (int ib = i0; ib < i1; ib += kInitI) {
+            __syncthreads();
+            const int nb = min(kInitI, i1 - ib);
+            for (int k = t; k < nb; k += T) {
+                const float4 p = pos[ib + k], sr = stat[ib + k];
+                s_xy[k] = make_float4(p.x, p.x, p.y, p.y);
+                s_zw[k] = make_float4(p.z, p.z, sr.x, sr.x);
+                s_qt[k] = make_float2(sr.y, __int_as_float(__float_as_int(sr.z) * kTableStride * 4));
+            }
+            __syncthreads();
+            for (int k = 0; k < task.na; ++k) {
+                const int am = task.a0 + k;
+                const bool use_a = ja < j1 && ma > am, use_b = jb < j1 && mb > am;
+                if (!__any_sync(0xffffffffu, use_a || use_b))
+                    continue;
+                const int2 span = s_mol[k];
+                const int si = max(span.x, ib) - ib, se = min(span.y, ib + nb) - ib;
+                // whole molecules start at phase 0; a larger one goes on from block to block
+                const int phase = ib + si - span.x;
+                const bool crowd_a = use_a && crowd_start >= 0 && (am >= non_crowders || ma >= non_crowders);
+                const bool crowd_b = use_b && crowd_start >= 0 && (am >= non_crowders || mb >= non_crowders);
+                if (__any_sync(0xffffffffu, crowd_a || crowd_b)) {
+                    // repulsive crowding (or a warp with such pairs): one residue at a time
+                    float xa, xb;
+                    f2_unpack(part, xa, xb);
+                    const float4 ra = make_float4(pa.x, pa.y, pa.z, sa.x), rb = make_float4(pb.x, pb.y, pb.z, sb.x);
+                    const float2 qa = make_float2(sa.y, sa.z), qb = make_float2(sb.y, sb.z);
+                    for (int i = si; i < se; ++i) {
+                        const float4 xy = s_xy[i], zw = s_zw[i];
+                        const float4 ri = make_float4(xy.x, xy.z, zw.x, zw.z);
+                        const float2 qi = make_float2(
+                            s_qt[i].x, __int_as_float(__float_as_int(s_qt[i].y) / (kTableStride * 4)));
+                        xa += crowd_a ? crowder_kcal(ri, ra, L, invL) : pair_kcal(ri, qi, ra, qa, s_table, L, invL);
+                        xb += crowd_b ? crowder_kcal(ri, rb, L, invL) : pair_kcal(ri, qi, rb, qb, s_table, L, invL);
+                        if (((phase + i - si) & 31) == 31) {
+                            ff_add(e0, xa);
+                            ff_add(e1, xb);
+                            xa = xb = 0.f;
+                        }
+                    }
+                    part = f2_pack(xa, xb);
+                } else {
+                    // each j's image nearest the molecule's middle; it is every pair's image
+                    // where it lies inside the half box less the molecule's half extent
+                    const float4 mid = s_mid[k], half = s_half[k];
+                    auto image = [&](float x, float m) {
+                        return __fadd_rn(__fmaf_rn(m - x, invL, 12582912.0f), -12582912.0f);
+                    };
+                    const float kxa = image(pa.x, mid.x), kya = image(pa.y, mid.y), kza = image(pa.z, mid.z);
+                    const float kxb = image(pb.x, mid.x), kyb = image(pb.y, mid.y), kzb = image(pb.z, mid.z);
+                    auto inside = [&](float x, float m, float kk, float h) {
+                        return fabsf(fmaf(-L, kk, m - x)) + h < 0.5f * L - kImageMargin;
+                    };
+                    const bool one_a = inside(pa.x, mid.x, kxa, half.x) && inside(pa.y, mid.y, kya, half.y) &&
+                                       inside(pa.z, mid.z, kza, half.z);
+                    const bool one_b = inside(pb.x, mid.x, kxb, half.x) && inside(pb.y, mid.y, kyb, half.y) &&
+                                       inside(pb.z, mid.z, kzb, half.z);
+                    const bool zero = kxa == 0.f && kya == 0.f && kza == 0.f && kxb == 0.f && kyb == 0.f && kzb == 0.f;
+                    if (__any_sync(0xffffffffu, (use_a && !one_a) || (use_b && !one_b)) || L == 0.0f) {
+                        init_span<2>(s_xy, s_zw, s_qt, si, se, phase, o, L, invL, part, e0, e1);
+                    } else if (__any_sync(0xffffffffu, (use_a || use_b) && !zero)) {
+                        o.sx = f2_pack(-L * kxa, -L * kxb), o.sy = f2_pack(-L * kya, -L * kyb);
+                        o.sz = f2_pack(-L * kza, -L * kzb);
+                        init_span<1>(s_xy, s_zw, s_qt, si, se, phase, o, L, invL, part, e0, e1);
+                    } else {
+                        init_span<0>(s_xy, s_zw, s_qt, si, se, phase, o, L, invL, part, e0, e1);
+                    }
+                }
+                if (ib + se == span.y) {  // the molecule is done
+                    float xa, xb;
+                    f2_unpack(part, xa, xb);
+                    ff_add(e0, xa);
+                    ff_add(e1, xb);
+                    s_e[k][2 * t] = make_float2(e0.hi, e0.lo);
+                    s_e[k][2 * t + 1] = make_float2(e1.hi, e1.lo);
+                    part = 0ull;
+                    e0 = e1 = FF{0.f, 0.f};
+                }
+            }
+        }
+        __syncthreads();
+        // per pair of molecules: the chunk's residues of the second one, 32 at a time
+        for (int k = warp; k < task.na * task.nb; k += NW) {
+            const int ka2 = k / task.nb, kb2 = k - ka2 * task.nb, am = task.a0 + ka2, bm = task.b0 + kb2;
+            if (bm <= am)
+                continue;
+            const int lo = max(mols[bm].start, jc), hi = min(mols[bm].start + mols[bm].count, jc + kInitJ);
+            FF sum = s_sum[ka2][kb2];
+            for (int j = lo; j < hi; j += 32) {
+                FF v{0.f, 0.f};
+                if (j + lane < hi) {
+                    const float2 e = s_e[ka2][j + lane - jc];
+                    v = FF{e.x, e.y};
+                }
+                ff_add_ff(sum, ff_warp_sum(v));
+            }
+            if (lane == 0)
+                s_sum[ka2][kb2] = sum;
+        }
+    }
+    __syncthreads();
+    double *E = a.emat + S.emat_off + (long long)r * M * M;
+    for (int k = t; k < task.na * task.nb; k += T) {
+        const int am = task.a0 + k / task.nb, bm = task.b0 + k % task.nb;
+        if (bm <= am)
+            continue;
+        const double v = ff_value(s_sum[k / task.nb][k % task.nb]);
+        E[(long long)am * M + bm] = v;
+        E[(long long)bm * M + am] = v;
+    }
 }
 
-// potential[g] = sum_{a<b} E[a][b] + sum_a intra[a]
-__global__ void k_sum_potential(EngineArgs a, double *out)
+// potential[g] = sum_{a<b} E[a][b] + sum_a intra[a]: a CTA of 8 warps per replica, rows
+// of the matrix dealt to warps (one warp per replica, with a division per entry, took 31
+// us for 64 molecules).
+__global__ void __launch_bounds__(256) k_sum_potential(EngineArgs a, double *out)
 {
-    const int g = blockIdx.x, lane = threadIdx.x;
-    const DevSim S = a.sims[a.rep_sim[g]];
+    __shared__ double s_part[8];
+    const int g = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const DevSim &S = a.sims[a.rep_sim[g]];
     const int r = g - S.rep_off, M = S.M;
     const double *E = a.emat + S.emat_off + (long long)r * M * M;
     const double *in = a.intra + S.molst_off + (long long)r * M;
     double v = 0.0;
-    for (int k = lane; k < M * M; k += 32) {
-        const int x = k / M, y = k % M;
-        if (x < y)
-            v += E[k];
+    for (int x = warp; x < M; x += 8) {
+        for (int y = x + 1 + lane; y < M; y += 32)
+            v += E[(long long)x * M + y];
+        if (lane == 0)
+            v += in[x];
     }
-    for (int k = lane; k < M; k += 32)
-        v += in[k];
     v = warp_sum_d(v);
     if (lane == 0)
+        s_part[warp] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w)
+            v += s_part[w];
         out[g] = v;
+    }
 }
 
 // ------------------------------------------------------------------ exchange
@@ -2314,19 +2601,18 @@ cudaError_t set_mc_smem_limit(size_t smem)
     for (const void *f : mc_kernels())
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_init_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     return e;
 }
 
-cudaError_t launch_init_energy(const EngineArgs &a, int total_replicas, size_t smem, double *potential_out,
+cudaError_t launch_init_energy(const EngineArgs &a, int total_replicas, int n_work, double *potential_out,
                                cudaStream_t stream)
 {
-    k_init_rows<<<total_replicas * a.max_m, 256, smem, stream>>>(a);
+    if (n_work > 0)
+        k_init_pairs<<<n_work, kInitThreads, 0, stream>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return e;
-    k_sum_potential<<<total_replicas, 32, 0, stream>>>(a, potential_out);
+    k_sum_potential<<<total_replicas, 256, 0, stream>>>(a, potential_out);
     return cudaGetLastError();
 }
 

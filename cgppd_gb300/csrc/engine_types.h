@@ -101,6 +101,17 @@ struct SampleRec {
     int step;
 };
 
+// One CTA's share of a replica's energies from scratch: the pairs of the molecules
+// [a0, a0 + na) with those of [b0, b0 + nb) that follow them, or (nb = 0) the internal
+// energy of the flexible molecule a0.
+struct InitTask {
+    int a0, na, b0, nb;
+};
+
+// Limits of a task's two groups of whole molecules: residues (a larger molecule is a group
+// of its own) and molecules.
+constexpr int kInitI = 128, kInitJ = 256, kInitSegs = 8, kInitMols = 64;
+
 struct EngineArgs {
     const DevSim *sims;
     const int *rep_sim;          // global replica -> simulation
@@ -121,6 +132,8 @@ struct EngineArgs {
     const int *localres;
     const int *crankres;
     const int2 *tiles;           // active intra tiles (ta, tb) of flexible molecules
+    const InitTask *init_tasks;  // of every simulation
+    const int2 *init_work;       // (global replica, task), the most pairs first
     const float *table;          // -4 Eij in kcal/mol, ntypes x ntypes (row stride 32)
     float4 *pos;
     float4 *rel;
