@@ -1968,13 +1968,13 @@ __device__ __forceinline__ Pair2 pair2(ulonglong2 xy, ulonglong2 zw, int trow, c
     return p;
 }
 
-// Whether a pair of p lies in the repulsive branch's range (s6 > 1/2: closer than
-// 2^(1/6) sigma; rare, so the branch is taken out of the straight path).
-__device__ __forceinline__ bool close2(const Pair2 &p)
+// The larger s6 of the two pairs: above 1/2 (closer than 2^(1/6) sigma) one may lie in the
+// repulsive branch's range; rare, so the branch is taken out of the straight path.
+__device__ __forceinline__ float closest2(const Pair2 &p)
 {
     float a, b;
     f2_unpack(p.s6, a, b);
-    return fmaxf(a, b) > 0.5f;
+    return fmaxf(a, b);
 }
 
 __device__ __forceinline__ void repulsive2(Pair2 &p)
@@ -2015,17 +2015,21 @@ __device__ __forceinline__ void init_span(const float4 *s_xy, const float4 *s_zw
     while (i < end) {
         const int stop = min(end, i + 32 - (phase & 31));
         phase += stop - i;
-        for (; i + 1 < stop; i += 2) {
-            Pair2 p = pair2<MI>(xy[i], zw[i], __float_as_int(s_qt[i].y), o, L2, invL2);
-            Pair2 q = pair2<MI>(xy[i + 1], zw[i + 1], __float_as_int(s_qt[i + 1].y), o, L2, invL2);
-            if (close2(p) || close2(q)) {
-                repulsive2(p);
-                repulsive2(q);
+        for (; i + 3 < stop; i += 4) {
+            Pair2 p[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                p[k] = pair2<MI>(xy[i + k], zw[i + k], __float_as_int(s_qt[i + k].y), o, L2, invL2);
+            if (fmaxf(fmaxf(closest2(p[0]), closest2(p[1])), fmaxf(closest2(p[2]), closest2(p[3]))) > 0.5f) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    repulsive2(p[k]);
             }
-            add(p, i);
-            add(q, i + 1);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                add(p[k], i + k);
         }
-        if (i < stop) {
+        while (i < stop) {
             Pair2 p = pair2<MI>(xy[i], zw[i], __float_as_int(s_qt[i].y), o, L2, invL2);
             repulsive2(p);
             add(p, i);
