@@ -39,6 +39,7 @@
 // Replica::fraction_bound / acceptance_ratio (src/Replica.cpp:1095-1122) and the
 // surrogate's fallback check.
 #include <array>
+#include <type_traits>
 #include <cooperative_groups.h>
 
 #include "cgppd_common.cuh"
@@ -49,10 +50,13 @@ namespace cg = cooperative_groups;
 
 namespace cgppd {
 
-constexpr int kTableStride = 32;
+constexpr int kTypes = 32;        // rows and columns of the contact table in global memory
+// Words from row to row of the table in shared memory: odd, so that the lanes that share
+// a residue j (one column) and take residues i of different types read different banks.
+constexpr int kTableStride = kTypes + 1;
 // Contact table in shared memory: -4 Eij in kcal/mol per type pair (4 bytes: a warp's
 // lookups of one row fall in one 128-byte line).
-constexpr int kTableBytes = kTableStride * kTableStride * (int)sizeof(float);
+constexpr int kTableBytes = kTypes * kTableStride * (int)sizeof(float);
 constexpr int kMaxThreads = 512;
 constexpr int kMaxWarps = kMaxThreads / 32;
 // Slack (A) on top of two bounding radii before a molecule pair skips the per-pair
@@ -90,7 +94,7 @@ struct MovePre {
 constexpr int kRing = 64;
 
 struct SmemLayout {
-    int table, mols, ipos, irel, iexcl, idisp, iq, ipq, iqq, ej, rowp, row;  // always
+    int table, mols, ipos, irel, iexcl, idisp, iq, ipq, ej, rowp, row;  // always
     int rcv;                                                         // clusters: pushed partial rows
     int rad;                                                         // bounding radius per molecule
     int ring;                                                        // draw-only decisions (kRing)
@@ -105,6 +109,10 @@ struct SmemLayout {
 // padded to multiples of 16 (one mma.sync m-tile); BF16 rows are padded to 264 elements
 // so that the fragment loads of 8 consecutive rows hit distinct banks.
 constexpr int kDaWS = kSurH + 8;
+
+// Records of a MoverView for molecules of up to n residues: each of its two spans rounds
+// up to an even number of rows of g <= min(32, n) lanes.
+__host__ __device__ inline int mover_records(int n) { return (n + 1) / 2 + 2 * (n < 32 ? n : 32); }
 
 __host__ __device__ inline int da_rows(int max_m) { return (((max_m - 1 > 1 ? max_m - 1 : 1) + 15) / 16) * 16; }
 
@@ -147,11 +155,12 @@ __host__ __device__ inline SmemLayout smem_layout(int max_mol, int slice, int ma
     L.mols = off;   off = align16(off + (int)sizeof(DevMol) * max_m);
     L.ipos = off;   off += 16 * max_mol;
     L.irel = off;   off += 16 * max_mol;
-    L.iexcl = off;  off += 16 * max_mol;
-    L.idisp = off;  off += 16 * max_mol;
+    L.iexcl = off;  off += any_flexible ? 16 * max_mol : 0;
     L.iq = off;     off = align16(off + 8 * max_mol);
-    L.ipq = off;    off += 16 * max_mol;  // the rigid mover in charged-first order
-    L.iqq = off;    off = align16(off + 8 * max_mol);
+    // the mover's records (MoverView); a flex move's displacements stand in their positions
+    // until these are written
+    L.ipq = off;    off += 48 * mover_records(max_mol);
+    L.idisp = L.ipq;
     L.ej = off;     off = align16(off + 8 * slice);
     L.rowp = off;   off = align16(off + 8 * (max_m + 1));
     L.row = off;    off = align16(off + 8 * (max_m + 1));
@@ -366,8 +375,8 @@ __device__ __forceinline__ float3 normalized(float x, float y, float z)
 
 __device__ __forceinline__ void load_table(float *s_table, const float *table, int t, int T)
 {
-    for (int k = t; k < kTableStride * kTableStride; k += T)
-        s_table[k] = table[k];
+    for (int k = t; k < kTypes * kTypes; k += T)
+        s_table[k / kTypes * kTableStride + k % kTypes] = table[k];
 }
 
 // Pair energy in kcal/mol of residue records a (position, sigma/2) and b, with the
@@ -406,45 +415,232 @@ __device__ __forceinline__ float pair_kcal(float4 a, float2 qa, float4 b, float2
     return pair_term<DH, 7>(a, qa, b, qb.x, table + __float_as_int(qb.y), L, invL);
 }
 
-// Pair terms of residues i = i0, i0 + g, ... < i1 of the mover (records ipv / iqv) with
-// one residue b of another molecule: four independent partial sums, folded into the
-// float-float accumulator every 32 terms.  Returns the first index of the sequence at or
-// past i1 (where the next span of the same sequence starts).
-template <bool DH, int MI>
-__device__ __forceinline__ int pair_span(const float4 *ipv, const float2 *iqv, int i0, int i1, int g, float4 b,
-                                          float qb, const float *col, float L, float invL, FF &acc, float &p0,
-                                          float &p1, float &p2, float &p3)
+// ------------------------------------------------------------------ packed pair terms
+
+// Two Lennard-Jones terms (pair_term's arithmetic on packed halves, the repulsive branch
+// left to repulsive2) and what the Debye-Hueckel terms need.
+struct Pair2 {
+    f2 u, r2, inv, m4, s6;
+};
+
+// min_image of two differences; nL holds -L.
+__device__ __forceinline__ f2 min_image2(f2 d, f2 nL, f2 invL)
 {
-    int i = i0, cntp = 0;
-    for (; i + 3 * g < i1; i += 4 * g) {
-        p0 += pair_term<DH, MI>(ipv[i], iqv[i], b, qb, col, L, invL);
-        p1 += pair_term<DH, MI>(ipv[i + g], iqv[i + g], b, qb, col, L, invL);
-        p2 += pair_term<DH, MI>(ipv[i + 2 * g], iqv[i + 2 * g], b, qb, col, L, invL);
-        p3 += pair_term<DH, MI>(ipv[i + 3 * g], iqv[i + 3 * g], b, qb, col, L, invL);
-        if (++cntp == 8) {
-            ff_add(acc, (p0 + p1) + (p2 + p3));
-            p0 = p1 = p2 = p3 = 0.f;
-            cntp = 0;
-        }
-    }
-    for (; i < i1; i += g)
-        p0 += pair_term<DH, MI>(ipv[i], iqv[i], b, qb, col, L, invL);
-    return i;
+    return f2_fma(nL, f2_add(f2_fma(d, invL, f2_dup(12582912.0f)), f2_dup(-12582912.0f)), d);
 }
 
-// Every pair of the mover (its charged residues first: the full term, then the
-// Lennard-Jones part alone) with the residue b, residues i = sub, sub + g, ... of the
-// mover, into acc.
-template <int MI>
-__device__ __forceinline__ void mover_spans(const float4 *ipv, const float2 *iqv, int sub, int nqm, int n, int g,
-                                            float4 b, float qb, const float *col, float L, float invL, FF &acc)
+__device__ __forceinline__ Pair2 lj2(f2 dx, f2 dy, f2 dz, f2 sigma, f2 m4)
 {
-    float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
-    const int i2 = pair_span<true, MI>(ipv, iqv, sub, nqm, g, b, qb, col, L, invL, acc, p0, p1, p2, p3);
-    ff_add(acc, (p0 + p1) + (p2 + p3));
-    p0 = p1 = p2 = p3 = 0.f;
-    pair_span<false, MI>(ipv, iqv, i2, n, g, b, qb, col, L, invL, acc, p0, p1, p2, p3);
-    ff_add(acc, (p0 + p1) + (p2 + p3));
+    Pair2 p;
+    p.r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
+    float ra, rb;
+    f2_unpack(p.r2, ra, rb);
+    p.inv = f2_pack(rsqrt_sfu(ra), rsqrt_sfu(rb));
+    p.m4 = m4;
+    const f2 so = f2_mul(sigma, p.inv), s2 = f2_mul(so, so);
+    p.s6 = f2_mul(f2_mul(s2, s2), s2);
+    float sa, sb;
+    f2_unpack(p.s6, sa, sb);
+    p.u = f2_mul(m4, f2_fma(p.s6, p.s6, f2_pack(-sa, -sb)));
+    return p;
+}
+
+// The larger s6 of the two pairs: above 1/2 (closer than 2^(1/6) sigma) one may lie in the
+// repulsive branch's range; rare, so the branch is taken out of the straight path.
+__device__ __forceinline__ float closest2(const Pair2 &p)
+{
+    float a, b;
+    f2_unpack(p.s6, a, b);
+    return fmaxf(a, b);
+}
+
+__device__ __forceinline__ void repulsive2(Pair2 &p)
+{
+    float a, b, ma, mb, ua, ub;
+    f2_unpack(p.s6, a, b);
+    f2_unpack(p.m4, ma, mb);
+    f2_unpack(p.u, ua, ub);
+    if (ma < 0.0f && a > 0.5f)
+        ua = fmaf(-0.5f, ma, -ua);
+    if (mb < 0.0f && b > 0.5f)
+        ub = fmaf(-0.5f, mb, -ub);
+    p.u = f2_pack(ua, ub);
+}
+
+// The terms with the Debye-Hueckel part, qq = q_i q_j of each pair.
+__device__ __forceinline__ f2 with_dh2(const Pair2 &p, f2 qq)
+{
+    const f2 arg = f2_mul(f2_mul(p.r2, p.inv), f2_dup(-kLog2e / kXi));
+    float ea, eb;
+    f2_unpack(arg, ea, eb);
+    return f2_fma(f2_mul(qq, f2_pack(ex2_sfu(ea), ex2_sfu(eb))), p.inv, p.u);
+}
+
+// The mover as the inter pair loop reads it.  Of a span of its residues (all of them, or
+// first the charged ones, then the rest) the g lanes that share a residue j take every
+// g-th; a lane's successive residues stand two to a record, so that one packed operation
+// serves two pairs.  Record (k / 2) g + slot holds the lane's k-th residue in half k % 2:
+//   xy = (x0, x1, y0, y1), zw = (z0, z1, sigma0/2, sigma1/2), qt = (q0, q1, row0, row1),
+// row the residue type's row of the contact table in bytes.  (Batched uneven blocks of 40
+// steps, 768 replicas: 6.86 ms with one residue a record and scalar arithmetic, 6.55 with
+// these records and four residues in flight, 6.30 with eight, 6.06 with the odd table
+// stride.  Bound by issue slots and the latency of 16 warps an SM: 23 instructions a
+// warp's pair, issue slots 53 % busy.)
+struct MoverView {
+    float4 *xy, *zw, *qt;
+};
+
+__device__ __forceinline__ void put_mover(const MoverView &v, int at, float4 p, float q, int type)
+{
+    const int h = at & 1, k = at >> 1;
+    float *a = reinterpret_cast<float *>(v.xy + k), *b = reinterpret_cast<float *>(v.zw + k),
+          *c = reinterpret_cast<float *>(v.qt + k);
+    a[h] = p.x, a[2 + h] = p.y;
+    b[h] = p.z, b[2 + h] = p.w;
+    c[h] = q, c[2 + h] = __int_as_float(type * kTableStride * 4);
+}
+
+// The residue j of a lane: negated position (or its image), half radius, charge, column of
+// the contact table.
+struct MoverOther {
+    f2 nx, ny, nz, w, q;
+    const char *col;
+};
+
+template <int MI>
+__device__ __forceinline__ Pair2 mover_pair2(const MoverView &v, int p, const MoverOther &o, f2 nL, f2 invL)
+{
+    const ulonglong2 xy = reinterpret_cast<const ulonglong2 *>(v.xy)[p],
+                     zw = reinterpret_cast<const ulonglong2 *>(v.zw)[p];
+    const int2 row = reinterpret_cast<const int2 *>(v.qt + p)[1];
+    f2 dx = f2_add(xy.x, o.nx), dy = f2_add(xy.y, o.ny), dz = f2_add(zw.x, o.nz);
+    if (MI & 1)
+        dx = min_image2(dx, nL, invL);
+    if (MI & 2)
+        dy = min_image2(dy, nL, invL);
+    if (MI & 4)
+        dz = min_image2(dz, nL, invL);
+    return lj2(dx, dy, dz, f2_add(zw.y, o.w),
+               f2_pack(*reinterpret_cast<const float *>(o.col + row.x), *reinterpret_cast<const float *>(o.col + row.y)));
+}
+
+// The K residues of a span that a lane takes, from record p on, with its residue j: four
+// independent partial sums, folded into the float-float accumulator every 32 terms; the
+// last (K % 4) go to the first sum, in order.  DH: with the Debye-Hueckel terms.
+template <bool DH, int MI>
+__device__ __forceinline__ void mover_span(const MoverView &v, int p, int K, int g, const MoverOther &o, f2 nL, f2 invL,
+                                           FF &acc)
+{
+    f2 p01 = 0ull, p23 = 0ull;
+    float x0, x1, x2, x3;
+    auto energy = [&](const Pair2 &e, int at) {
+        return DH ? with_dh2(e, f2_mul(reinterpret_cast<const f2 *>(v.qt + at)[0], o.q)) : e.u;
+    };
+    // R records (2 R residues) at once
+    auto records = [&](auto count) {
+        constexpr int R = decltype(count)::value;
+        Pair2 e[R];
+        float closest = 0.0f;
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            e[q] = mover_pair2<MI>(v, p + q * g, o, nL, invL);
+            closest = fmaxf(closest, closest2(e[q]));
+        }
+        if (closest > 0.5f) {
+#pragma unroll
+            for (int q = 0; q < R; ++q)
+                repulsive2(e[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < R; q += 2) {
+            p01 = f2_add(p01, energy(e[q], p + q * g));
+            p23 = f2_add(p23, energy(e[q + 1], p + (q + 1) * g));
+        }
+        p += R * g;
+    };
+    int k = 0, cnt = 0;
+    for (; k + 7 < K; k += 8) {
+        records(std::integral_constant<int, 4>());
+        if ((cnt += 2) == 8) {
+            f2_unpack(p01, x0, x1);
+            f2_unpack(p23, x2, x3);
+            ff_add(acc, (x0 + x1) + (x2 + x3));
+            p01 = p23 = 0ull;
+            cnt = 0;
+        }
+    }
+    if (k + 3 < K) {
+        records(std::integral_constant<int, 2>());
+        k += 4;
+    }
+    f2_unpack(p01, x0, x1);
+    f2_unpack(p23, x2, x3);
+    if (k < K) {
+        Pair2 e = mover_pair2<MI>(v, p, o, nL, invL);
+        repulsive2(e);
+        float a, b;
+        f2_unpack(energy(e, p), a, b);
+        x0 += a;
+        if (k + 1 < K)
+            x0 += b;
+        if (k + 2 < K) {
+            e = mover_pair2<MI>(v, p + g, o, nL, invL);
+            repulsive2(e);
+            f2_unpack(energy(e, p + g), a, b);
+            x0 += a;
+        }
+    }
+    ff_add(acc, (x0 + x1) + (x2 + x3));
+}
+
+// The plan of a molecule's inter pair loop: g lanes per residue j, and the two spans of n1
+// and n - n1 residues as k g + r; packed into the launch's copy of its DevMol.
+struct MoverPlan {
+    int g, k1, r1, k2, r2;
+    int inv;  // ceil(1024 / g): x / g = x inv >> 10 for x <= 32
+};
+
+__device__ __forceinline__ void pack_plan(DevMol &m, int g, int n1)
+{
+    const int n2 = m.count - n1, k1 = n1 / g, k2 = n2 / g;
+    m.pair_lanes = g | (n1 - k1 * g) << 6 | (n2 - k2 * g) << 11 | ((1023 + g) / g) << 16;
+    m.nq = k1 | k2 << 16;
+}
+
+__device__ __forceinline__ MoverPlan mover_plan(const DevMol &m)
+{
+    return MoverPlan{m.pair_lanes & 63, m.nq & 0xffff, (m.pair_lanes >> 6) & 31, (int)((unsigned)m.nq >> 16),
+                     (m.pair_lanes >> 11) & 31, m.pair_lanes >> 16};
+}
+
+// First record of the second span.
+__device__ __forceinline__ int second_span(const MoverPlan &m) { return ((m.k1 + (m.r1 > 0 ? 1 : 0) + 1) >> 1) * m.g; }
+
+// Where the residue with place o in the mover's order goes: 2 x record + half.
+__device__ __forceinline__ int mover_slot(int o, const MoverPlan &m)
+{
+    const int n1 = m.k1 * m.g + m.r1;
+    const int base = o < n1 ? 0 : second_span(m), oo = o < n1 ? o : o - n1;
+    const int k = oo / m.g, slot = oo - k * m.g;
+    return 2 * (base + (k >> 1) * m.g + slot) + (k & 1);
+}
+
+// A lane's share of the mover: its residues of the two spans.
+struct MoverLane {
+    int g, p1, K1, p2, K2;
+};
+
+// Every pair of a lane's share of the mover with its residue j into acc: the first span
+// with the full term, the second (of charged-first movers) with the Lennard-Jones part
+// alone.
+template <int MI, bool QF>
+__device__ __forceinline__ void mover_spans(const MoverView &v, const MoverLane &m, const MoverOther &o, float L,
+                                            float invL, FF &acc)
+{
+    const f2 nL = f2_dup(-L), invL2 = f2_dup(invL);
+    mover_span<true, MI>(v, m.p1, m.K1, m.g, o, nL, invL2, acc);
+    if (QF)
+        mover_span<false, MI>(v, m.p2, m.K2, m.g, o, nL, invL2, acc);
 }
 
 // Repulsive crowder pair in kcal/mol, the reference's REPULSIVE_CROWDING build
@@ -1073,8 +1269,9 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
     int4 *s_iexcl = reinterpret_cast<int4 *>(smem + Ly.iexcl);
     float4 *s_disp = reinterpret_cast<float4 *>(smem + Ly.idisp);
     float2 *s_iq = reinterpret_cast<float2 *>(smem + Ly.iq);
+    const int records = mover_records(a.max_mol);
     float4 *s_ipq = reinterpret_cast<float4 *>(smem + Ly.ipq);
-    float2 *s_iqq = reinterpret_cast<float2 *>(smem + Ly.iqq);
+    const MoverView mover{s_ipq, s_ipq + records, s_ipq + 2 * records};
     unsigned short *s_qpos = reinterpret_cast<unsigned short *>(smem + Ly.QP);
     float *s_rad = reinterpret_cast<float *>(smem + Ly.rad);
     float2 *s_ej = reinterpret_cast<float2 *>(smem + Ly.ej);
@@ -1108,9 +1305,13 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
     FF *ROWSUMf = reinterpret_cast<FF *>(smem + Ly.ROWSUM);
 
     load_table(s_table, a.table, t, T);
+    // a record half that no residue takes is read (and dropped) beside its neighbour: its
+    // table row has to be one
+    for (int k = t; k < records; k += T)
+        mover.qt[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int k = t; k < M; k += T) {
         DevMol mk = a.mols[S.mol_off + k];
-        mk.pair_lanes = pair_lanes(mk.count, N, C, NW);
+        pack_plan(mk, pair_lanes(mk.count, N, C, NW), QF ? mk.nq : mk.count);
         s_mols[k] = mk;
     }
     if (RES) {
@@ -1121,8 +1322,6 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
             sP[i] = make_float4(p.x, p.y, p.z, sr.x);
             sQ[i] = make_float4(q.x, q.y, q.z, sr.y);
             sTY[i] = (unsigned char)__float_as_int(sr.z);
-            if (QF)
-                s_qpos[i] = a.rqpos[S.res_off + i];
         }
         if (a.any_flexible) {
             int4 *sEX = reinterpret_cast<int4 *>(smem + Ly.EX);
@@ -1136,6 +1335,12 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
         for (int k = t; k < M * M; k += T)
             EMf[k] = ff_from(__ldcg(&gE[k]));
         __syncthreads();
+        // where each residue goes when its molecule moves
+        for (int i = t; i < N; i += T) {
+            const DevMol &mk = s_mols[__float_as_int(gST[i].w)];
+            const int o = QF ? a.rqpos[S.res_off + i] : i - mk.start;
+            s_qpos[i] = (unsigned short)mover_slot(o, mover_plan(mk));
+        }
     }
     // bounding radius of every rigid molecule about its centre (rotations keep it up to
     // float rounding, which kImageMargin covers); flexible molecules change shape and get
@@ -1341,6 +1546,12 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
         }
 
         // ---- proposal of the moved molecule
+        // residue i's place among the mover's records
+        auto place = [&](int i) -> int {
+            if (RES)
+                return s_qpos[start + i];
+            return mover_slot(QF ? a.rqpos[S.res_off + start + i] : i, mover_plan(s_mols[m]));
+        };
         for (int i = t; i < n; i += T) {
             const float4 p = ld_state<RES>(&P[start + i]);
             const float4 q = ld_state<RES>(&Q[start + i]);
@@ -1371,11 +1582,8 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
             np.w = sr.x;
             s_ipos[i] = np;
             s_irel[i] = nq;
-            if (QF && !flexmol) {  // the rigid mover also in charged-first order (its final positions)
-                const int k = RES ? s_qpos[start + i] : a.rqpos[S.res_off + start + i];
-                s_ipq[k] = np;
-                s_iqq[k] = make_float2(sr.y, sr.z);
-            }
+            if (N > n && (nullm || type != kFlex))
+                put_mover(mover, place(i), np, sr.y, __float_as_int(sr.z));
         }
         __syncthreads();
         if (type == kFlex && !nullm) {
@@ -1430,6 +1638,11 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
                 s_irel[i] = q;
             }
             __syncthreads();
+            if (N > n) {  // the displacements are read: their place takes the mover's records
+                for (int i = t; i < n; i += T)
+                    put_mover(mover, place(i), s_ipos[i], s_iq[i].x, __float_as_int(s_iq[i].y));
+                __syncthreads();
+            }
         }
 
         // ---- inter-molecule pairs: this CTA's slice of the other residues
@@ -1439,103 +1652,106 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
         const int sl = (nother + C - 1) / C;
         const int o0 = rank * sl, o1 = min(nother, o0 + sl);
         const int cnt = max(0, o1 - o0);
-        // g lanes per j (each takes every g-th i), floor(32 / g) groups of lanes per warp;
-        // the lanes past the last whole group idle
-        const int g = s_mols[m].pair_lanes, jw = 32 / g;
-        // a rigid mover is read in charged-first order: its first nqm residues take the
-        // full pair term, the rest the Lennard-Jones part alone (no charge, no Debye-Hueckel)
-        const bool qfirst = QF && !flexmol;
-        const float4 *ipv = qfirst ? s_ipq : s_ipos;
-        const float2 *iqv = qfirst ? s_iqq : s_iq;
-        const int nqm = qfirst ? s_mols[m].nq : n;
-        // repulsive crowding: pairs with a crowder (j >= cstart, or a crowder mover) take
-        // the crowder term
-        const int cstart = (S.crowd_start >= 0) ? S.crowd_start : 0x7fffffff;
-        const bool mcrowd = S.crowd_start >= 0 && m >= S.non_crowders;
-        const int sub = lane % g, grp = lane / g;
-        const int jl = warp * jw + grp, jstride = NW * jw;
-        const bool lane_on = grp < jw;
-        // Periodic images without a minimum image per pair: each other residue j is moved
-        // once to its image nearest the mover's centre.  Where that image lies more than
-        // the mover's bounding radius inside the half box around the centre on every
-        // axis, no mover residue is more than half a box from it, so the per-pair rule
-        // (src/CudaFunctions.cu:321-333) takes exactly that image for every pair and the
-        // loop takes the plain differences; on an axis where some j of the warp lies in the
-        // outer shell the warp keeps the per-pair minimum image for that axis.  (Flexible
-        // movers have no fixed radius: always the per-pair rule.)
-        const float hlim = (L != 0.0f && !flexmol) ? 0.5f * L - (s_rad[m] + kImageMargin) : -1.0f;
-        auto stat_of = [&](int j) -> float4 {
-            return RES ? make_float4(0.f, Q[j].w, __int_as_float((int)TY[j]), 0.f) : ST[j];
-        };
-        // residue record of this thread's next j, loaded one iteration ahead
-        float4 npj = make_float4(0.f, 0.f, 0.f, 0.f), nsj = npj;
-        if (lane_on && jl < cnt) {
-            const int o = o0 + jl, j = (o < start) ? o : o + n;
-            npj = ld_state<RES>(&P[j]);
-            nsj = stat_of(j);
-        }
-        for (int base = 0; base < cnt; base += jstride) {
-            const int o = o0 + base + jl;
-            const bool valid = lane_on && (base + jl) < cnt;
-            const bool crowd = mcrowd || ((o < start) ? o : o + n) >= cstart;
-            const float4 pj = npj, sj = nsj;
-            if (lane_on && base + jstride + jl < cnt) {
-                const int on = o + jstride, jn = (on < start) ? on : on + n;
-                npj = ld_state<RES>(&P[jn]);
-                nsj = stat_of(jn);
+        if (cnt > 0) {
+            // g lanes per j (each takes every g-th i), floor(32 / g) groups of lanes per warp;
+            // the lanes past the last whole group idle
+            const MoverPlan plan = mover_plan(s_mols[m]);
+            const int g = plan.g, jw = 32 * plan.inv >> 10;
+            // repulsive crowding: pairs with a crowder (j >= cstart, or a crowder mover) take
+            // the crowder term
+            const int cstart = (S.crowd_start >= 0) ? S.crowd_start : 0x7fffffff;
+            const bool mcrowd = S.crowd_start >= 0 && m >= S.non_crowders;
+            const int grp = lane * plan.inv >> 10, sub = lane - grp * g;
+            int slot2 = sub - plan.r1;  // the second span goes on where the first ends
+            slot2 += slot2 < 0 ? g : 0;
+            const MoverLane ml{g, sub, plan.k1 + (sub < plan.r1 ? 1 : 0), second_span(plan) + slot2,
+                               QF ? plan.k2 + (slot2 < plan.r2 ? 1 : 0) : 0};
+            const int jl = warp * jw + grp, jstride = NW * jw;
+            const bool lane_on = grp < jw;
+            // Periodic images without a minimum image per pair: each other residue j is moved
+            // once to its image nearest the mover's centre.  Where that image lies more than
+            // the mover's bounding radius inside the half box around the centre on every
+            // axis, no mover residue is more than half a box from it, so the per-pair rule
+            // (src/CudaFunctions.cu:321-333) takes exactly that image for every pair and the
+            // loop takes the plain differences; on an axis where some j of the warp lies in the
+            // outer shell the warp keeps the per-pair minimum image for that axis.  (Flexible
+            // movers have no fixed radius: always the per-pair rule.)
+            const float hlim = (L != 0.0f && !flexmol) ? 0.5f * L - (s_rad[m] + kImageMargin) : -1.0f;
+            auto stat_of = [&](int j) -> float4 {
+                return RES ? make_float4(0.f, Q[j].w, __int_as_float((int)TY[j]), 0.f) : ST[j];
+            };
+            // residue record of this thread's next j, loaded one iteration ahead
+            float4 npj = make_float4(0.f, 0.f, 0.f, 0.f), nsj = npj;
+            if (lane_on && jl < cnt) {
+                const int o = o0 + jl, j = (o < start) ? o : o + n;
+                npj = ld_state<RES>(&P[j]);
+                nsj = stat_of(j);
             }
-            // j's image nearest the mover's centre (the minimum-image rule applied once;
-            // exactly pj where that image is pj itself)
-            const float kx = __fadd_rn(__fmaf_rn(pj.x - mv.wcx, invL, 12582912.0f), -12582912.0f);
-            const float ky = __fadd_rn(__fmaf_rn(pj.y - mv.wcy, invL, 12582912.0f), -12582912.0f);
-            const float kz = __fadd_rn(__fmaf_rn(pj.z - mv.wcz, invL, 12582912.0f), -12582912.0f);
-            const float bx = fmaf(-L, kx, pj.x), by = fmaf(-L, ky, pj.y), bz = fmaf(-L, kz, pj.z);
-            // the axes on which some j of the warp lies outside the inner region
-            const bool use = valid && !crowd && L != 0.0f;
-            const int outer = (__any_sync(0xffffffffu, use && !(fabsf(bx - mv.wcx) < hlim)) ? 1 : 0) |
-                              (__any_sync(0xffffffffu, use && !(fabsf(by - mv.wcy) < hlim)) ? 2 : 0) |
-                              (__any_sync(0xffffffffu, use && !(fabsf(bz - mv.wcz) < hlim)) ? 4 : 0);
-            FF acc{0.f, 0.f};
-            if (valid && crowd) {
-                float p0 = 0.f;
-                int cntp = 0;
-                for (int i = sub; i < n; i += g) {
-                    p0 += crowder_kcal(ipv[i], pj, L, invL);
-                    if (++cntp == 32) {
-                        ff_add(acc, p0);
-                        p0 = 0.f;
-                        cntp = 0;
-                    }
+            for (int base = 0; base < cnt; base += jstride) {
+                const int o = o0 + base + jl;
+                const bool valid = lane_on && (base + jl) < cnt;
+                const bool crowd = mcrowd || ((o < start) ? o : o + n) >= cstart;
+                const float4 pj = npj, sj = nsj;
+                if (lane_on && base + jstride + jl < cnt) {
+                    const int on = o + jstride, jn = (on < start) ? on : on + n;
+                    npj = ld_state<RES>(&P[jn]);
+                    nsj = stat_of(jn);
                 }
-                ff_add(acc, p0);
-            } else if (valid) {
-                const float qj = sj.y;
-                const float *col = s_table + __float_as_int(sj.z);
-                const float sw = RES ? pj.w : sj.x;
-                // j's image nearest the mover's centre; the minimum image per pair only on
-                // the axes where the warp needs it (most outer warps are outer on one axis)
-                const float4 rj = make_float4(bx, by, bz, sw);
-                if (outer == 0)
-                    mover_spans<0>(ipv, iqv, sub, nqm, n, g, rj, qj, col, L, invL, acc);
-                else if (outer == 1)
-                    mover_spans<1>(ipv, iqv, sub, nqm, n, g, rj, qj, col, L, invL, acc);
-                else if (outer == 2)
-                    mover_spans<2>(ipv, iqv, sub, nqm, n, g, rj, qj, col, L, invL, acc);
-                else if (outer == 4)
-                    mover_spans<4>(ipv, iqv, sub, nqm, n, g, rj, qj, col, L, invL, acc);
-                else
-                    mover_spans<7>(ipv, iqv, sub, nqm, n, g, make_float4(pj.x, pj.y, pj.z, sw), qj, col, L, invL,
-                                   acc);
+                // j's image nearest the mover's centre (the minimum-image rule applied once;
+                // exactly pj where that image is pj itself)
+                const float kx = __fadd_rn(__fmaf_rn(pj.x - mv.wcx, invL, 12582912.0f), -12582912.0f);
+                const float ky = __fadd_rn(__fmaf_rn(pj.y - mv.wcy, invL, 12582912.0f), -12582912.0f);
+                const float kz = __fadd_rn(__fmaf_rn(pj.z - mv.wcz, invL, 12582912.0f), -12582912.0f);
+                const float bx = fmaf(-L, kx, pj.x), by = fmaf(-L, ky, pj.y), bz = fmaf(-L, kz, pj.z);
+                // the axes on which some j of the warp lies outside the inner region
+                const bool use = valid && !crowd && L != 0.0f;
+                const unsigned out3 = (fabsf(bx - mv.wcx) < hlim ? 0u : 1u) | (fabsf(by - mv.wcy) < hlim ? 0u : 2u) |
+                                      (fabsf(bz - mv.wcz) < hlim ? 0u : 4u);
+                const int outer = (int)__reduce_or_sync(0xffffffffu, use ? out3 : 0u);
+                FF acc{0.f, 0.f};
+                if (valid && crowd) {
+                    float p0 = 0.f;
+                    int cntp = 0;
+                    for (int k = 0; k < ml.K1 + ml.K2; ++k) {
+                        const int kk = k < ml.K1 ? k : k - ml.K1, at = (k < ml.K1 ? ml.p1 : ml.p2) + (kk >> 1) * g;
+                        const float *xy = reinterpret_cast<const float *>(mover.xy + at) + (kk & 1);
+                        const float *zw = reinterpret_cast<const float *>(mover.zw + at) + (kk & 1);
+                        p0 += crowder_kcal(make_float4(xy[0], xy[2], zw[0], zw[2]), pj, L, invL);
+                        if (++cntp == 32) {
+                            ff_add(acc, p0);
+                            p0 = 0.f;
+                            cntp = 0;
+                        }
+                    }
+                    ff_add(acc, p0);
+                } else if (valid) {
+                    // j's image nearest the mover's centre; the minimum image per pair only on
+                    // the axes where the warp needs it (most outer warps are outer on one axis)
+                    const bool any_image = outer != 0 && outer != 1 && outer != 2 && outer != 4;
+                    const float ox = any_image ? pj.x : bx, oy = any_image ? pj.y : by, oz = any_image ? pj.z : bz;
+                    const MoverOther oj{f2_dup(-ox), f2_dup(-oy), f2_dup(-oz), f2_dup(RES ? pj.w : sj.x), f2_dup(sj.y),
+                                        reinterpret_cast<const char *>(s_table + __float_as_int(sj.z))};
+                    if (outer == 0)
+                        mover_spans<0, QF>(mover, ml, oj, L, invL, acc);
+                    else if (outer == 1)
+                        mover_spans<1, QF>(mover, ml, oj, L, invL, acc);
+                    else if (outer == 2)
+                        mover_spans<2, QF>(mover, ml, oj, L, invL, acc);
+                    else if (outer == 4)
+                        mover_spans<4, QF>(mover, ml, oj, L, invL, acc);
+                    else
+                        mover_spans<7, QF>(mover, ml, oj, L, invL, acc);
+                }
+                // segmented tree sum towards the group's first lane: after the step with offset
+                // d, lane sub holds the lanes [sub, min(sub + 2d, g)) of its group
+                for (int d = 1; d < g; d <<= 1) {
+                    const FF w{__shfl_down_sync(0xffffffffu, acc.hi, d), __shfl_down_sync(0xffffffffu, acc.lo, d)};
+                    if (sub + d < g)
+                        ff_add_ff(acc, w);
+                }
+                if (valid && sub == 0)
+                    s_ej[o - o0] = make_float2(acc.hi, acc.lo);
             }
-            // segmented tree sum towards the group's first lane: after the step with offset
-            // d, lane sub holds the lanes [sub, min(sub + 2d, g)) of its group
-            for (int d = 1; d < g; d <<= 1) {
-                const FF w{__shfl_down_sync(0xffffffffu, acc.hi, d), __shfl_down_sync(0xffffffffu, acc.lo, d)};
-                if (sub + d < g)
-                    ff_add_ff(acc, w);
-            }
-            if (valid && sub == 0)
-                s_ej[o - o0] = make_float2(acc.hi, acc.lo);
         }
 
         // ---- internal energy of a flexible molecule (intra pairs split over the cluster).
@@ -1650,7 +1866,8 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
                 const float2 e = s_ej[o - o0];
                 ff_add_ff(acc, FF{e.x, e.y});
             }
-            acc = ff_warp_sum(acc);
+            if (lo < hi)
+                acc = ff_warp_sum(acc);
             // lane 0's value for every receiver (lanes may differ in the low word)
             const FF v{__shfl_sync(0xffffffffu, acc.hi, 0), __shfl_sync(0xffffffffu, acc.lo, 0)};
             if (C > 1) {
@@ -1918,15 +2135,8 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
 
 constexpr int kInitThreads = kInitJ / 2;  // two residues j a thread
 
-// Lennard-Jones terms of one residue i with a thread's two residues j (pair_term's
-// arithmetic on packed halves; the repulsive branch is left to repulsive2), and what the
-// Debye-Hueckel term needs.
-struct Pair2 {
-    f2 u, r2, inv, m4, s6;
-};
-
-// The two residues j: negated positions, the image shift -L k, half radii, charges and
-// their columns of the contact table (bytes).
+// The two residues j of a thread: negated positions, the image shift -L k, half radii,
+// charges and their columns of the contact table (bytes).
 struct Other2 {
     f2 nx, ny, nz, sx, sy, sz, w, q;
     const char *c0, *c1;
@@ -1936,67 +2146,22 @@ struct Other2 {
 // segment's middle), the shift added to each difference; 2: the minimum image per pair.
 // The difference is min_image's in all three, bit for bit.
 template <int MI>
-__device__ __forceinline__ f2 image2(f2 xi, f2 nxj, f2 shift, f2 L, f2 invL)
+__device__ __forceinline__ f2 image2(f2 xi, f2 nxj, f2 shift, f2 nL, f2 invL)
 {
     f2 d = f2_add(xi, nxj);
     if (MI == 1)
         d = f2_add(d, shift);
-    if (MI == 2) {
-        const f2 magic = f2_dup(12582912.0f), back = f2_dup(-12582912.0f);
-        d = f2_fma(L, f2_add(f2_fma(d, invL, magic), back), d);  // (L holds -L)
-    }
+    if (MI == 2)
+        d = min_image2(d, nL, invL);
     return d;
 }
 
 template <int MI>
-__device__ __forceinline__ Pair2 pair2(ulonglong2 xy, ulonglong2 zw, int trow, const Other2 &o, f2 L, f2 invL)
+__device__ __forceinline__ Pair2 pair2(ulonglong2 xy, ulonglong2 zw, int trow, const Other2 &o, f2 nL, f2 invL)
 {
-    Pair2 p;
-    const f2 dx = image2<MI>(xy.x, o.nx, o.sx, L, invL);
-    const f2 dy = image2<MI>(xy.y, o.ny, o.sy, L, invL);
-    const f2 dz = image2<MI>(zw.x, o.nz, o.sz, L, invL);
-    p.r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
-    float ra, rb;
-    f2_unpack(p.r2, ra, rb);
-    p.inv = f2_pack(rsqrt_sfu(ra), rsqrt_sfu(rb));
-    p.m4 = f2_pack(*reinterpret_cast<const float *>(o.c0 + trow), *reinterpret_cast<const float *>(o.c1 + trow));
-    const f2 so = f2_mul(f2_add(zw.y, o.w), p.inv), s2 = f2_mul(so, so);
-    p.s6 = f2_mul(f2_mul(s2, s2), s2);
-    float sa, sb;
-    f2_unpack(p.s6, sa, sb);
-    p.u = f2_mul(p.m4, f2_fma(p.s6, p.s6, f2_pack(-sa, -sb)));
-    return p;
-}
-
-// The larger s6 of the two pairs: above 1/2 (closer than 2^(1/6) sigma) one may lie in the
-// repulsive branch's range; rare, so the branch is taken out of the straight path.
-__device__ __forceinline__ float closest2(const Pair2 &p)
-{
-    float a, b;
-    f2_unpack(p.s6, a, b);
-    return fmaxf(a, b);
-}
-
-__device__ __forceinline__ void repulsive2(Pair2 &p)
-{
-    float a, b, ma, mb, ua, ub;
-    f2_unpack(p.s6, a, b);
-    f2_unpack(p.m4, ma, mb);
-    f2_unpack(p.u, ua, ub);
-    if (ma < 0.0f && a > 0.5f)
-        ua = fmaf(-0.5f, ma, -ua);
-    if (mb < 0.0f && b > 0.5f)
-        ub = fmaf(-0.5f, mb, -ub);
-    p.u = f2_pack(ua, ub);
-}
-
-__device__ __forceinline__ f2 with_dh2(const Pair2 &p, float qi, f2 qj)
-{
-    const f2 arg = f2_mul(f2_mul(p.r2, p.inv), f2_dup(-kLog2e / kXi));
-    float ea, eb;
-    f2_unpack(arg, ea, eb);
-    const f2 e = f2_mul(f2_mul(f2_dup(qi), qj), f2_pack(ex2_sfu(ea), ex2_sfu(eb)));
-    return f2_fma(e, p.inv, p.u);
+    return lj2(image2<MI>(xy.x, o.nx, o.sx, nL, invL), image2<MI>(xy.y, o.ny, o.sy, nL, invL),
+               image2<MI>(zw.x, o.nz, o.sz, nL, invL), f2_add(zw.y, o.w),
+               f2_pack(*reinterpret_cast<const float *>(o.c0 + trow), *reinterpret_cast<const float *>(o.c1 + trow)));
 }
 
 // The residues [i, end) of one segment with a thread's two residues j, summed in order of
@@ -2010,7 +2175,7 @@ __device__ __forceinline__ void init_span(const float4 *s_xy, const float4 *s_zw
     const f2 L2 = f2_dup(-L), invL2 = f2_dup(invL);
     auto add = [&](const Pair2 &p, int k) {
         const float qi = s_qt[k].x;
-        part = f2_add(part, qi != 0.0f ? with_dh2(p, qi, o.q) : p.u);
+        part = f2_add(part, qi != 0.0f ? with_dh2(p, f2_mul(f2_dup(qi), o.q)) : p.u);
     };
     while (i < end) {
         const int stop = min(end, i + 32 - (phase & 31));
@@ -2058,7 +2223,7 @@ __device__ __forceinline__ void init_span(const float4 *s_xy, const float4 *s_zw
 // reduction per other molecule took 1243 us.
 __global__ void __launch_bounds__(kInitThreads) k_init_pairs(EngineArgs a)
 {
-    __shared__ __align__(16) float s_table[kTableStride * kTableStride];
+    __shared__ float s_table[kTypes * kTableStride];
     __shared__ float4 s_xy[kInitI], s_zw[kInitI];  // (x, x, y, y), (z, z, sigma/2, sigma/2)
     __shared__ float2 s_qt[kInitI];                // charge, table row (bytes)
     __shared__ float2 s_e[kInitSegs][kInitJ];      // per molecule of the first group and residue j

@@ -66,8 +66,9 @@ struct DevMol {
     int fr0, fr1, fr2;           // residues (molecule-relative) spanning the body frame
     int tile_off, ntile;         // 32 x 32 intra tiles (ta <= tb) holding an unexcluded pair
     float tors_const;            // sum of V_n over the molecule's torsions (kcal/mol)
-    int pair_lanes;              // lanes per other residue in the inter pair loop (set per launch)
-    int nq;                      // charged residues: the inter pair loop takes them first
+    // charged residues (the inter pair loop takes them first); in a launch's own copy the
+    // loop's plan instead, see mover_plan
+    int nq, pair_lanes;
 };
 
 // Delayed-acceptance counters of one replica slot (not swapped on exchange).
