@@ -906,11 +906,14 @@ __device__ void predecide_move(const Lists &a, const DevSim &S, const DevMol *mo
     pre.w_stage1 = w[9];
 }
 
-// The move of this step from its draw-only part and the current state: the centre,
-// the translation and its wrap, the flex pivot, the crankshaft rotation.
+// The move of a step from its draw-only part and the state: the centre, the translation
+// and its wrap, the flex pivot, the crankshaft rotation.  `last` (or null): an accepted
+// move that is being committed meanwhile, its positions in `lastpos`; the state of every
+// other molecule is at rest.
 template <bool RES>
 __device__ void finish_move(const DevSim &S, const DevMol *mols, const float4 *CEN, const float4 *P, float tstep,
-                            const float4 rsc, const MovePre &pre, MoveDesc &mv)
+                            const float4 rsc, const MovePre &pre, MoveDesc &mv, const MoveDesc *last,
+                            const float4 *lastpos)
 {
     const int m = pre.m;
     const DevMol &mol = mols[m];
@@ -931,10 +934,11 @@ __device__ void finish_move(const DevSim &S, const DevMol *mols, const float4 *C
     mv.w_metro = pre.w_metro;
     mv.w_stage1 = pre.w_stage1;
     const float box = S.box;
-    const float4 c = ld_state<RES>(&CEN[m]);
+    const bool moved = last != nullptr && last->m == m;
+    const float4 c = moved ? make_float4(last->wcx, last->wcy, last->wcz, 0.f) : ld_state<RES>(&CEN[m]);
     mv.cx = c.x, mv.cy = c.y, mv.cz = c.z;
     mv.wcx = c.x, mv.wcy = c.y, mv.wcz = c.z;
-    const float4 *Pm = P + mv.start;
+    const float4 *Pm = moved ? lastpos : P + mv.start;
     switch (ptype) {
     case kTranslate:
         mv.vx = pre.R[0] * tstep, mv.vy = pre.R[1] * tstep, mv.vz = pre.R[2] * tstep;
@@ -1226,7 +1230,7 @@ template <bool RES, bool DA, bool QF>
 __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ MoveDesc mv;
+    __shared__ MoveDesc s_mv[2];   // this step's move and (resident) the next one's
     __shared__ FF s_red[kMaxWarps];
     __shared__ float s_fred[3 * kMaxWarps];
     // running total, old/new row of the moved molecule and its internal energy, all as
@@ -1484,17 +1488,23 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
     if (warp == NW - 1)
         fill_ring(0);
     __syncthreads();
+    if (RES) {
+        if (t == 0)
+            finish_move<RES>(S, s_mols, CEN, P, tstep, rsc, s_ring[0], s_mv[0], nullptr, nullptr);
+        __syncthreads();
+    }
 
     for (int step = 0; step < nsteps; ++step) {
         const unsigned long long mcstep = step0 + (unsigned long long)step;
-        // ---- the move decision (thread 0): the state-dependent part of the decision
-        // whose draw-only part waits in the ring
-        if (t == 0) {
-            finish_move<RES>(S, s_mols, CEN, P, tstep, rsc, s_ring[step & (kRing - 1)], mv);
-            if (RES)
-                s_old_row = ROWSUMf[mv.m];
+        // ---- the move decision: the state-dependent part of the decision whose draw-only
+        // part waits in the ring.  Resident launches take it during the previous step's
+        // commit (below); otherwise that commit has to be visible first.
+        MoveDesc &mv = s_mv[RES ? step & 1 : 0];
+        if (!RES) {
+            if (t == 0)
+                finish_move<RES>(S, s_mols, CEN, P, tstep, rsc, s_ring[step & (kRing - 1)], mv, nullptr, nullptr);
+            __syncthreads();
         }
-        __syncthreads();
         const int n = mv.n, start = mv.start, type = mv.type, m = mv.m;
         const bool nullm = mv.null_move != 0;
         const bool flexmol = mv.flexible != 0;
@@ -1937,7 +1947,8 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
                 ff_add_ff(new_row, intra_new);
                 s_new_row = new_row;
                 FF dEf = new_row;  // newPotential - oldPotential = new row - old row
-                ff_add_ff(dEf, FF{-s_old_row.hi, -s_old_row.lo});
+                const FF old_row = RES ? ROWSUMf[m] : s_old_row;
+                ff_add_ff(dEf, FF{-old_row.hi, -old_row.lo});
                 float delta = dEf.hi + dEf.lo;
                 if (DA && screened)  // stage 2: exact change less the surrogate's
                     delta = (float)(ff_value(dEf) - s_ds);
@@ -2042,6 +2053,12 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
         // (the end-of-step barrier publishes it)
         if (skip && warp == NW - 1 && (step & 31) == 15)
             fill_ring(step + 17);
+        // the next step's move, by the last warp while the others commit (a rigid mover leaves
+        // it no residues): its thread waited for on its own took a barrier and about 750
+        // cycles of every step
+        if (RES && t == T - 32 && step + 1 < nsteps)
+            finish_move<RES>(S, s_mols, CEN, P, tstep, rsc, s_ring[(step + 1) & (kRing - 1)], s_mv[(step + 1) & 1],
+                             (!skip && s_accept) ? &mv : nullptr, s_ipos);
         // fraction-bound sample (src/Simulation.cpp:1063-1073, src/Replica.cpp:1037-1063)
         const int freq = S.sample_freq;
         if (freq > 0 && (long long)(mcstep % (unsigned long long)freq) == freq - 1 &&
