@@ -135,48 +135,6 @@ __device__ __forceinline__ float dh_term(float qq, float r, float inv_r)
     return qq * ex2_sfu(r * (-kLog2e / kXi)) * inv_r;
 }
 
-// ------------------------------------------------------------------ packed pairs
-// Two FP32 values in one 64-bit register pair.  The packed add, multiply and fma round
-// each half as the scalar instruction does; an FMA pipe takes two cycles for one, so the
-// FP32 peak is the scalar one, but a loop that is bound by issue slots (28 of them per
-// Lennard-Jones pair, 14 on the FMA pipes) gets half of its arithmetic slots back.
-typedef unsigned long long f2;
-
-__device__ __forceinline__ f2 f2_pack(float lo, float hi)
-{
-    f2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-
-__device__ __forceinline__ f2 f2_dup(float v) { return f2_pack(v, v); }
-
-__device__ __forceinline__ void f2_unpack(f2 v, float &lo, float &hi)
-{
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-
-__device__ __forceinline__ f2 f2_add(f2 a, f2 b)
-{
-    f2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
-__device__ __forceinline__ f2 f2_mul(f2 a, f2 b)
-{
-    f2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
-__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c)
-{
-    f2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
 // ------------------------------------------------------------------ Philox4x32-10
 // Counter-based generator (Salmon et al., SC'11).  Engine draws are
 // philox(key = {seed ^ stream, seed_hi}, ctr = {step, step_hi, block, domain}).

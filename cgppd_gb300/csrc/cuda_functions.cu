@@ -6,21 +6,15 @@
 // (type, charge, vdW radius, w) with w = molecule_id + chain_fraction (-1 for a
 // crowder).  The pair rules are those of the reference's flexible-linker build.
 //
-// Kernel: one CTA per (y-tile, x-tile) pair of 128-residue tiles on or above the
-// diagonal, two (one per 64-residue half of the y tile) for the diagonal pairs.  The x
-// tile is decoded once into shared memory (position and radius; the exclusion keys of
-// its w fields; charge, type and flags) next to the 20x20 table, and copied in the
-// order [charged | uncharged] real residues (padding left out), each part split into
-// the residues that cannot form an excluded pair with this CTA's y residues (their keys
-// outside the y residues' key ranges) and those that may: the Debye-Hueckel term is
-// taken for charged x residues only, and only the second kind takes the exclusion tests.
-// Per warp of y residues the tests are dropped altogether when none of its residues can
-// meet an excluded pair, or when the others share every x residue's domain (their sums
-// are discarded); the crowder forms keep a general loop where pairs may be excluded.
-// Two or four threads own each y residue and sweep alternate x residues.  Pair terms
-// are FP32, summed per 32 pairs and folded into float-float accumulators, reduced per
-// CTA in float-float.  The last CTA to finish (ticket counter) reduces all CTA partials
-// in a fixed order, so the total is deterministic.  Scratch (partials + ticket +
+// Kernel: a CTA takes 128 residues y (four warps of 32) against one, two or four blocks
+// of 32 residues x on or after them.  Per block the 32 x are copied charged first, two to a
+// record (one packed operation serves two pairs); each warp then decides once per block:
+// nothing to do (all pairs excluded), no pair excluded (the packed loop, Debye-Hueckel for
+// the charged records only, the minimum image only on the axes where the block's bounding
+// box and the warp's residues leave more than one image), or a mixture (a scalar loop with
+// the exclusion tests per pair).  Pair terms are FP32, at most eight to a partial sum,
+// folded into float-float accumulators, reduced per CTA in float-float.  The last CTA to finish (ticket counters) reduces all CTA partials
+// in a fixed order, so the total is deterministic.  Scratch (partials + tickets +
 // result) is per (device, stream), allocated on first use and reused.
 #include <cstdio>
 #include <atomic>
@@ -31,6 +25,7 @@
 
 #include "cgppd_common.cuh"
 #include "host/amino_acids.h"
+#include "pair_terms.cuh"
 #include "status.h"
 #include "cgppd_cuda_functions.h"
 
@@ -38,11 +33,16 @@ using namespace cgppd;
 
 namespace {
 
-// (64-residue tiles, four times the CTAs for a one-wave call, measured no faster:
-// 26.5-27.5 us against 24.7 us for a 6 M-pair call, with 12 % more instructions.)
-constexpr int kTile = 128;                 // residues per tile side
-constexpr int kThreads = 2 * kTile;        // two threads per y residue (four for a half y tile)
+constexpr int kTile = 128;                 // residues y of a CTA, one per thread
+constexpr int kThreads = kTile;
 constexpr int kWarps = kThreads / 32;
+constexpr int kBlock = 32;                 // residues of an x block and of a warp's y block
+constexpr int kTypes = 20;
+// Tiles of a call from which a CTA takes four (two) x blocks, see x_blocks.
+constexpr int kFourBlocks = 40, kTwoBlocks = 28;
+// Slack (A) on the box test that drops the minimum image: covers the rounding of the
+// relative positions.
+constexpr float kImageSlack = 0.05f;
 
 __constant__ float c_boxdim;  // CUDA_setBoxDimension, module state per device
 // cgppd_set_repulsive_crowding: the reference's compile-time REPULSIVE_CROWDING
@@ -92,14 +92,6 @@ __device__ __forceinline__ float frac_int(float w, float &ip)
     return w - ip;
 }
 
-// 1/x on the SFU (PTX rcp.approx.ftz.f32, max relative error about 2^-23).
-__device__ __forceinline__ float rcp_sfu(float x)
-{
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // The Lennard-Jones part of lj_term with the table value m4e = -4 Eij (RT units) and the
 // mixed radius sigma_ij: u = m4e s6 (s6 - 1), and 2 Eij - u on the repulsive branch
 // (Eij > 0, s6 > 1/2); one multiplication less than lj_term.
@@ -113,201 +105,228 @@ __device__ __forceinline__ float lj_m4(float m4e, float sigma_ij, float inv_r2)
     return u;
 }
 
-// What the charged-first loop needs of its y residue.
-struct PairCtx {
-    float4 py;
-    float yh, yq;             // half radius, charge
-    const float *m4row;       // -4 Eij (RT units) row of the y type
-    float L, invL;
-    int yl, x0, y;            // y's place in its tile, the x tile's first index, y's index
-    bool diag, near;
-    float ydom, ybond, ychain;
-    bool ydom_nz, ybond_nz;
+// The keys of the exclusion rules over 32 residues, as ranges of their bit patterns (two
+// sets of floats whose bit-pattern ranges are disjoint share no value): nonzero rigid
+// domain, nonzero bond fraction, chain fraction, molecule id (>= 0); an empty range has
+// lo > hi.  flags: bit 0 padding, 1 crowder, 2 a residue without a rigid domain.
+struct Keys {
+    int dlo, dhi, blo, bhi, clo, chi, mlo, mhi, flags;
 };
 
-// The y residue against a span of the copied x tile, the S threads of a y residue
-// taking every S-th x residue of the sequence j, j + S, ... below `end` (returns where
-// the sequence continues).  Charged spans take the full term, the others the
-// Lennard-Jones part alone (1/r^2 from the SFU reciprocal: no 1/r needed there).
-// TESTED spans hold the x residues that may form a pair the reference excludes (same
-// rigid domain, same bond, chain neighbours |x - y| < 4, the diagonal tile's lower
-// half), with the rules of the general loop: charged spans skip those pairs (a warp's y
-// residues mostly share a molecule, so the branch is mostly uniform), the others
-// evaluate them two at a time and select them away.
-template <bool TESTED>
-__device__ __forceinline__ bool pair_excluded(const PairCtx &c, const float4 *s_qk, int j)
+__device__ __forceinline__ Keys warp_keys(bool real, bool crowd, float dom, float bond, float chain, float mol)
 {
-    if (!TESTED)
-        return false;
-    const float4 k = s_qk[j];
-    const int xi = __float_as_int(k.w);
-    return (c.diag && xi <= c.yl) || (c.ydom_nz && k.x == c.ydom) || (c.ybond_nz && k.y == c.ybond) ||
-           (c.near && k.z == c.ychain && abs(c.x0 + xi - c.y) < 4);
-}
-
-template <bool TESTED, int S>
-__device__ __forceinline__ int charged_span(const PairCtx &c, const float4 *s_pq, const float2 *s_qt,
-                                            const float4 *s_qk, int j, int end, FF &lj, FF &dh)
-{
-    const float4 py = c.py;
-    const float L = c.L, invL = c.invL;
-    float l0 = 0.f, d0 = 0.f;
-    int cnt = 0;
-    for (; j < end; j += S) {
-        if (pair_excluded<TESTED>(c, s_qk, j))
-            continue;
-        const float4 px = s_pq[j];
-        const float2 qt = s_qt[j];
-        const float dx = min_image(py.x - px.x, L, invL);
-        const float dyy = min_image(py.y - px.y, L, invL);
-        const float dz = min_image(py.z - px.z, L, invL);
-        const float r2 = fmaf(dx, dx, fmaf(dyy, dyy, dz * dz));
-        const float inv_r = rsqrt_sfu(r2);
-        const float u = lj_m4(c.m4row[__float_as_int(qt.y)], c.yh + px.w, inv_r * inv_r);
-        const float d = dh_term(c.yq * qt.x, r2 * inv_r, inv_r);
-        l0 += u;
-        d0 += d;
-        if (++cnt == 32) {
-            ff_add(lj, l0);
-            ff_add(dh, d0);
-            l0 = d0 = 0.f;
-            cnt = 0;
-        }
-    }
-    ff_add(lj, l0);
-    ff_add(dh, d0);
-    return j;
-}
-
-template <bool TESTED, int S>
-__device__ __forceinline__ int lj_span(const PairCtx &c, const float4 *s_pq, const float2 *s_qt, const float4 *s_qk,
-                                       int j, int end, FF &lj)
-{
-    const float4 py = c.py;
-    const float L = c.L, invL = c.invL;
-    float l0 = 0.f, l1 = 0.f;
-    int cnt = 0;
-    for (; j + S < end; j += 2 * S) {
-        const float4 pa = s_pq[j], pb = s_pq[j + S];
-        const int ta = __float_as_int(s_qt[j].y), tb = __float_as_int(s_qt[j + S].y);
-        const float ax = min_image(py.x - pa.x, L, invL), bx = min_image(py.x - pb.x, L, invL);
-        const float ay = min_image(py.y - pa.y, L, invL), by = min_image(py.y - pb.y, L, invL);
-        const float az = min_image(py.z - pa.z, L, invL), bz = min_image(py.z - pb.z, L, invL);
-        const float ra = fmaf(ax, ax, fmaf(ay, ay, az * az)), rb = fmaf(bx, bx, fmaf(by, by, bz * bz));
-        const float ua = lj_m4(c.m4row[ta], c.yh + pa.w, rcp_sfu(ra));
-        const float ub = lj_m4(c.m4row[tb], c.yh + pb.w, rcp_sfu(rb));
-        l0 += pair_excluded<TESTED>(c, s_qk, j) ? 0.f : ua;
-        l1 += pair_excluded<TESTED>(c, s_qk, j + S) ? 0.f : ub;
-        if (++cnt == 16) {
-            ff_add(lj, l0 + l1);
-            l0 = l1 = 0.f;
-            cnt = 0;
-        }
-    }
-    for (; j < end; j += S) {
-        const float4 pa = s_pq[j];
-        const float ax = min_image(py.x - pa.x, L, invL);
-        const float ay = min_image(py.y - pa.y, L, invL);
-        const float az = min_image(py.z - pa.z, L, invL);
-        const float ra = fmaf(ax, ax, fmaf(ay, ay, az * az));
-        const float ua = lj_m4(c.m4row[__float_as_int(s_qt[j].y)], c.yh + pa.w, rcp_sfu(ra));
-        l0 += pair_excluded<TESTED>(c, s_qk, j) ? 0.f : ua;
-    }
-    ff_add(lj, l0 + l1);
-    return j;
-}
-
-// The y residue against the copied x tile: its real residues in the order [charged
-// safe | charged tested | uncharged safe | uncharged tested] with the group ends e[0..3]
-// (padding after e[3] is not visited); TESTED: the tested groups take the exclusion
-// tests (else the warp's y residues need none, and skip_tested residues skip them).
-template <int S, bool TESTED>
-__device__ __forceinline__ void charged_first_pairs(const PairCtx &c, const float4 *s_pq, const float2 *s_qt,
-                                                    const float4 *s_qk, const int *e, int sub, bool skip_tested,
-                                                    FF &lj, FF &dh)
-{
-    // the first index of the sequence j, j + S, ... at or past `end`
-    auto past = [](int j, int end) { return j < end ? j + ((end - j + S - 1) / S) * S : j; };
-    int j = sub;
-    j = charged_span<false, S>(c, s_pq, s_qt, s_qk, j, e[0], lj, dh);
-    j = skip_tested ? past(j, e[1]) : charged_span<TESTED, S>(c, s_pq, s_qt, s_qk, j, e[1], lj, dh);
-    j = lj_span<false, S>(c, s_pq, s_qt, s_qk, j, e[2], lj);
-    if (!skip_tested)
-        lj_span<TESTED, S>(c, s_pq, s_qt, s_qk, j, e[3], lj);
-}
-
-// One warp's residues' exclusion-key ranges and flags, stored by lane 0 into wk[0..8]:
-// [nonzero domain min/max, nonzero bond min/max, chain min/max, molecule min/max] as
-// bit patterns, then the OR of the flags (bit 0 padding, bit 1 crowder).  Ranges are of
-// the keys' bit patterns: two sets of floats whose bit-pattern ranges are disjoint share
-// no value.
-__device__ __forceinline__ void warp_keys(int *wk, float dom, float bond, float chain, float mol, int flags)
-{
-    const int inf = 0x7fffffff;
+    const int none_lo = 0x7fffffff, none_hi = (int)0x80000000;
     // + 0.0f turns -0 into +0: the exclusion tests compare keys as floats, where -0 == +0
     const int d = __float_as_int(dom + 0.0f), b = __float_as_int(bond + 0.0f), c = __float_as_int(chain + 0.0f),
               m = __float_as_int(mol + 0.0f);
-    const bool real = (flags & 1) == 0;  // padding records carry no keys
-    const int v[8] = {real && dom != 0.f ? d : inf, real && dom != 0.f ? d : -1,
-                      real && bond != 0.f ? b : inf, real && bond != 0.f ? b : -1,
-                      real ? c : inf, real ? c : -1, real && mol >= 0.f ? m : inf, real && mol >= 0.f ? m : -1};
-    int r[8];
+    const bool hd = real && dom != 0.0f, hb = real && bond != 0.0f, hm = real && mol >= 0.0f;
+    Keys k;
+    k.dlo = __reduce_min_sync(0xffffffffu, hd ? d : none_lo), k.dhi = __reduce_max_sync(0xffffffffu, hd ? d : none_hi);
+    k.blo = __reduce_min_sync(0xffffffffu, hb ? b : none_lo), k.bhi = __reduce_max_sync(0xffffffffu, hb ? b : none_hi);
+    k.clo = __reduce_min_sync(0xffffffffu, real ? c : none_lo);
+    k.chi = __reduce_max_sync(0xffffffffu, real ? c : none_hi);
+    k.mlo = __reduce_min_sync(0xffffffffu, hm ? m : none_lo), k.mhi = __reduce_max_sync(0xffffffffu, hm ? m : none_hi);
+    k.flags = (int)__reduce_or_sync(0xffffffffu, (real ? 0u : 1u) | (crowd ? 2u : 0u) |
+                                                     (real && dom == 0.0f ? 4u : 0u));
+    return k;
+}
+
+__device__ __forceinline__ bool disjoint(int alo, int ahi, int blo, int bhi) { return ahi < blo || bhi < alo; }
+
+// One block of 32 residues x.
+struct XBlock {
+    float4 xy[16], zw[16], qt[16];  // records of two: (x0, x1, y0, y1), (z0, z1, s0/2, s1/2), (q0, q1, row0, row1)
+    float4 pos[32];                 // as given: position, half radius
+    float4 key[32];                 // domain, bond, chain, molecule
+    float4 meta[32];                // charge, table row (bytes), flags (1 padding, 2 crowder)
+    Keys keys;
+    int k1, k2;                     // residues in charged and uncharged records (multiples of 4)
+    float3 mid, half;               // of the bounding box
+};
+
+// Orders floats as signed integers.
+__device__ __forceinline__ int ordered(float f)
+{
+    const int i = __float_as_int(f);
+    return i ^ ((i >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ float unordered(int i) { return __int_as_float(i ^ ((i >> 31) & 0x7fffffff)); }
+
+__device__ __forceinline__ void box_axis(float v, bool use, float &mid, float &half)
+{
+    const float lo = unordered(__reduce_min_sync(0xffffffffu, use ? ordered(v) : 0x7f7fffff));
+    const float hi = unordered(__reduce_max_sync(0xffffffffu, use ? ordered(v) : (int)0x80800000));
+    mid = 0.5f * (lo + hi);
+    half = 0.5f * (hi - lo);
+}
+
+// Warp: the block's copies from the residue (p, m) of each lane.  `copied`: the residue
+// takes part in the packed loop.
+__device__ __forceinline__ void build_block(XBlock &X, float4 p, float4 m, int type, bool copied, bool pad, bool crowd)
+{
+    const int lane = threadIdx.x & 31;
+    float dom, mol;
+    const float bond = frac_int(p.w, dom), chain = frac_int(m.w, mol);
+    const Keys k = warp_keys(!pad, crowd, dom, bond, chain, mol);
+    float3 mid, half;
+    box_axis(p.x, copied, mid.x, half.x);
+    box_axis(p.y, copied, mid.y, half.y);
+    box_axis(p.z, copied, mid.z, half.z);
+    const int row = type * kTypes * 4;
+    X.pos[lane] = make_float4(p.x, p.y, p.z, 0.5f * m.z);
+    X.key[lane] = make_float4(dom, bond, chain, mol);
+    X.meta[lane] = make_float4(m.y, __int_as_float(row), __int_as_float((pad ? 1 : 0) | (crowd ? 2 : 0)), 0.f);
+    // charged residues first, then the others, filled up to a multiple of four with the last
+    // one's place and radius, no charge and the table's row of zeros
+    const unsigned all = __ballot_sync(0xffffffffu, copied), chg = __ballot_sync(0xffffffffu, copied && m.y != 0.0f);
+    const unsigned below = (1u << lane) - 1u;
+    const int n = __popc(all), nq = __popc(chg);
+    const int at = (chg >> lane & 1u) ? __popc(chg & below) : nq + __popc(all & ~chg & below);
+    const int n4 = (n + 3) & ~3, k1 = min((nq + 3) & ~3, n4);
+    auto put = [&](int k, float q, int r) {
+        const int h = k & 1;
+        float *a = reinterpret_cast<float *>(&X.xy[k >> 1]), *b = reinterpret_cast<float *>(&X.zw[k >> 1]),
+              *c = reinterpret_cast<float *>(&X.qt[k >> 1]);
+        a[h] = p.x, a[2 + h] = p.y;
+        b[h] = p.z, b[2 + h] = 0.5f * m.z;
+        c[h] = q, c[2 + h] = __int_as_float(r);
+    };
+    if (copied) {
+        put(at, m.y, row);
+        if (at == n - 1)
+            for (int e = n; e < n4; ++e)
+                put(e, 0.0f, kTypes * kTypes * 4);
+    }
+    if (lane == 0) {
+        X.keys = k;
+        X.k1 = k1;
+        X.k2 = n4 - k1;
+        X.mid = mid;
+        X.half = half;
+    }
+}
+
+// A thread's residue y: negated position, shift -L k to its image nearest the block's
+// middle, half radius, charge, its column of the table.
+struct YLane {
+    f2 nx, ny, nz, sx, sy, sz, w, q;
+    const char *col;
+};
+
+// Which differences x - y need what.  The difference of the positions as given is exact for
+// close residues and the shift is exact, so all forms give min_image's bits (positions
+// relative to the block's middle save the shift's addition, but round: ten times the
+// error of a contact's energy).
+constexpr int kPlain = 0, kShift = 8;  // bits 0, 1, 2: the minimum image per pair on that axis
+
+template <int MODE, int AXIS>
+__device__ __forceinline__ f2 difference(f2 x, f2 ny, f2 shift, f2 nL, f2 invL)
+{
+    const f2 d = f2_add(x, ny);
+    if (MODE & AXIS)
+        return min_image2(d, nL, invL);
+    return (MODE & kShift) ? f2_add(d, shift) : d;
+}
+
+// R records of a block with y, terms added in order to four partial sums each of the
+// Lennard-Jones and (DH) Debye-Hueckel part.
+template <bool DH, int MODE, int R>
+__device__ __forceinline__ void block_records(const XBlock &X, int r, const YLane &y, f2 nL, f2 invL, f2 *lj, f2 *dh)
+{
+    Pair2 e[R];
+    float closest = 0.0f;
 #pragma unroll
-    for (int k = 0; k < 8; ++k)
-        r[k] = (k & 1) ? __reduce_max_sync(0xffffffffu, v[k]) : __reduce_min_sync(0xffffffffu, v[k]);
-    const int f = (int)__reduce_or_sync(0xffffffffu, (unsigned)flags);
-    if ((threadIdx.x & 31) == 0) {
+    for (int k = 0; k < R; ++k) {
+        const ulonglong2 xy = reinterpret_cast<const ulonglong2 *>(X.xy)[r + k],
+                         zw = reinterpret_cast<const ulonglong2 *>(X.zw)[r + k];
+        const int2 row = reinterpret_cast<const int2 *>(&X.qt[r + k])[1];
+        e[k] = lj2_sq<DH>(difference<MODE, 1>(xy.x, y.nx, y.sx, nL, invL),
+                          difference<MODE, 2>(xy.y, y.ny, y.sy, nL, invL),
+                          difference<MODE, 4>(zw.x, y.nz, y.sz, nL, invL), f2_add(zw.y, y.w),
+                          f2_pack(*reinterpret_cast<const float *>(y.col + row.x),
+                                  *reinterpret_cast<const float *>(y.col + row.y)));
+        closest = fmaxf(closest, closest2(e[k]));
+    }
+    if (closest > 0.5f) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
-            wk[k] = r[k];
-        wk[8] = f;
+        for (int k = 0; k < R; ++k)
+            repulsive2(e[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        lj[k & 1] = f2_add(lj[k & 1], e[k].u);
+        if (DH)
+            dh[k & 1] = f2_add(dh[k & 1], dh2(e[k], f2_mul(reinterpret_cast<const f2 *>(&X.qt[r + k])[0], y.q)));
     }
 }
 
-constexpr int kKeys = 9;
-
-// Key k of a tile from the nw warps that stored theirs (min for even k, max for odd k,
-// OR for the flags, k = 8).
-__device__ __forceinline__ int tile_key(const int (*wk)[kKeys], int nw, int k)
+__device__ __forceinline__ float sum4(const f2 *v)
 {
-    int v = wk[0][k];
-    for (int w = 1; w < nw; ++w)
-        v = (k == 8) ? (v | wk[w][k]) : (k & 1) ? max(v, wk[w][k]) : min(v, wk[w][k]);
-    return v;
+    float a, b, c, d;
+    f2_unpack(v[0], a, b);
+    f2_unpack(v[1], c, d);
+    return (a + b) + (c + d);
 }
 
-__device__ __forceinline__ bool ranges_disjoint(int amin, int amax, int bmin, int bmax)
+// A whole block (no pair of it excluded) with y: the charged records in full, the others
+// the Lennard-Jones part alone.  Two records at a time and rolled loops: with four, and
+// one more copy of each loop for the odd pair, the warps of an SM were spread over more
+// code than its instruction caches hold (69 M pairs: 100 us, 6 of 13 stall cycles an
+// instruction waiting for instructions; 71 us like this, issue slots 74 % busy while the
+// SMs are, FMA pipes 57 %).
+template <int MODE>
+__device__ __forceinline__ void clean_block(const XBlock &X, const YLane &y, float L, float invL, FF &lj, FF &dh)
 {
-    return amax < bmin || bmax < amin;  // an empty range (min > max) is disjoint from all
+    const f2 nL = f2_dup(-L), invL2 = f2_dup(invL);
+    f2 u[2] = {0ull, 0ull}, d[2] = {0ull, 0ull};
+    const int r1 = X.k1 >> 1, r2 = r1 + (X.k2 >> 1);
+    int r = 0;
+#pragma unroll 1
+    for (; r < r1; r += 2)
+        block_records<true, MODE, 2>(X, r, y, nL, invL2, u, d);
+#pragma unroll 1
+    for (; r < r2; r += 2)
+        block_records<false, MODE, 2>(X, r, y, nL, invL2, u, d);
+    ff_add(lj, sum4(u));
+    ff_add(dh, sum4(d));
 }
 
-// CTAs of a call on nt tiles: every tile pair on or above the diagonal, the nt diagonal
-// pairs twice.
-__host__ __device__ constexpr int energy_ctas(int nt) { return nt * (nt + 1) / 2 + nt; }
+// ------------------------------------------------------------------ work of a call
 
-// CTA b -> tile pair (ty <= tx) and y part: part 1, 2 are the halves of the y tile of a
-// diagonal pair (CTAs 0 .. 2 nt - 1), part 0 the whole y tile of an off-diagonal pair
-// (row-major).
-__device__ __forceinline__ void cta_work(int b, int nt, int &ty, int &tx, int &part)
+// x blocks of a CTA for nt tiles of 128 residues: the blocks of a CTA are a serial chain, so
+// one while that leaves SMs short of warps, more once the copies and keys of a CTA cost
+// more than the chain (us a call on three streams with 1 / 2 / 4 blocks: 21 tiles 5.6 /
+// 6.5 / 8.7, 26 tiles 7.1 / 7.3 / 9.6, 39 tiles - / 13.5 / 12.6 but 40 / 43 for one call
+// alone, 55 tiles - / 26.5 / 22.3).
+__host__ __device__ constexpr int x_blocks(int nt) { return nt >= kFourBlocks ? 4 : nt >= kTwoBlocks ? 2 : 1; }
+
+// CTAs of a call: for each tile ty the chunks of x blocks on or after it, rows of
+// decreasing length.
+__host__ __device__ constexpr int chunks(int nt, int nx) { return 4 * nt / nx; }
+__host__ __device__ constexpr int energy_ctas(int nt)
 {
-    if (b < 2 * nt) {
-        part = 1 + (b & 1);
-        ty = tx = b >> 1;
-        return;
-    }
-    part = 0;
-    int rem = b - 2 * nt;
-    ty = 0;
-    while (ty < nt - 1 && rem >= nt - ty - 1) {  // row ty holds nt - ty - 1 such pairs
-        rem -= nt - ty - 1;
-        ++ty;
-    }
-    tx = ty + 1 + rem;
+    const int nx = x_blocks(nt), nc = chunks(nt, nx), step = 4 / nx;
+    return nt * nc - step * (nt * (nt - 1) / 2);
+}
+// CTA b -> tile ty and chunk: row ty starts at f(ty) = ty nc - step ty (ty - 1) / 2.
+__device__ __forceinline__ void cta_work(int b, int nt, int nx, int &ty, int &chunk)
+{
+    const int nc = chunks(nt, nx), step = 4 / nx;
+    auto first = [&](int r) { return r * nc - step * (r * (r - 1) / 2); };
+    const float h = (float)nc / (float)step + 0.5f;
+    int r = (int)(h - sqrtf(fmaxf(0.0f, h * h - 2.0f * (float)b / (float)step)));
+    r = max(0, min(nt - 1, r));
+    while (r > 0 && first(r) > b)
+        --r;
+    while (r < nt - 1 && first(r + 1) <= b)
+        ++r;
+    ty = r;
+    chunk = step * r + (b - first(r));
 }
 
 // kNC: non-crowder pairs of different molecules only (E_TiledKernelNC).  kRC: the
 // REPULSIVE_CROWDING form of the crowder pairs.
-template <bool kNC, bool kRC>
+template <bool kNC, bool kRC, int NX>
 __global__ void __launch_bounds__(kThreads) k_tile_energy(const float4 *__restrict__ pos, const float4 *__restrict__ meta,
                                                           int P, int nt, const float *__restrict__ lj_raw,
                                                           double *__restrict__ partials, unsigned *__restrict__ ticket,
@@ -315,51 +334,32 @@ __global__ void __launch_bounds__(kThreads) k_tile_energy(const float4 *__restri
                                                           float4 *__restrict__ gsums, unsigned *__restrict__ gtickets,
                                                           float *__restrict__ async_out, int async_count)
 {
-    // x tile, decoded once per CTA: position and vdW radius; exclusion keys (rigid
-    // domain, bond fraction, chain fraction, molecule id); charge, type, flags
-    __shared__ float4 s_px[kTile];
-    __shared__ float4 s_xk[kTile];
-    __shared__ float4 s_xm[kTile];
-    __shared__ float s_eij[400];
-    __shared__ float s_m4[400];   // -4 Eij in RT units (the clean-tile loop's form)
+    __shared__ XBlock s_x[NX];
+    __shared__ float s_m4[(kTypes + 1) * kTypes];  // -4 Eij in RT units, [x type][y type]; a row of zeros
     __shared__ FF s_red[2][kWarps];
-    __shared__ bool s_last, s_last_group;
-    // the x tile's real residues again in charged-first order (position + half radius,
-    // charge + type), for the charged-first loop
-    __shared__ float4 s_pq[kTile];
-    __shared__ float2 s_qt[kTile];
-    // ... and their exclusion keys (domain, bond, chain, original index), for the pairs
-    // that take the exclusion tests
-    __shared__ float4 s_qk[kTile];
-    // per-warp key ranges and flags of the x tile and of this CTA's y residues (warp_keys)
-    __shared__ int s_wk[2][kTile / 32][kKeys];
-    // per x warp, key ranges of its residues that take the exclusion tests: [nonzero domain
-    // min/max, nonzero bond min/max, chain min/max, domain min/max] (bit patterns)
-    __shared__ int s_tk[kTile / 32][8];
-    // counts of the x tile's copy groups per warp (charged safe, charged tested, uncharged
-    // safe, uncharged tested, padding)
-    __shared__ int s_gcnt[kTile / 32][5];
+    __shared__ bool s_last;
 
     // a dependent launch (see launch_energy): nothing global is touched before the
     // stream's previous kernel has completed
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    int ty, tx, part;
-    cta_work(blockIdx.x, nt, ty, tx, part);
-    const int t = threadIdx.x;
-    // y residue of this thread (place in its tile) and its share of the x tile: the
-    // whole y tile with two threads per residue, or one half with four
-    const int ny = part ? kTile / 2 : kTile;
-    const int yl = (part ? (part - 1) * (kTile / 2) : 0) + (t & (ny - 1)), sub = t / ny;
+    int ty, chunk;
+    cta_work(blockIdx.x, nt, NX, ty, chunk);
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     // the x and y records first, so that their loads overlap the table's
-    const int x0 = tx * kTile;
-    const int y = ty * kTile + yl;
-    float4 px_in = make_float4(0.f, 0.f, 0.f, kPadder), mx_in = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (t < kTile && x0 + t < P) {
-        px_in = pos[x0 + t];
-        mx_in = meta[x0 + t];
+    const int x = (chunk * NX + warp) * kBlock + lane, y = ty * kTile + t;
+    float4 px = make_float4(0.f, 0.f, 0.f, kPadder), mx = make_float4(0.f, 0.f, 0.f, 0.f), py = px, my = mx;
+    if (warp < NX && x < P) {
+        px = pos[x];
+        mx = meta[x];
     }
-    const float4 py = (y < P) ? pos[y] : make_float4(0.f, 0.f, 0.f, kPadder);
-    const float4 my = (y < P) ? meta[y] : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (y < P) {
+        py = pos[y];
+        my = meta[y];
+    }
+    for (int k = t; k < kTypes * kTypes; k += kThreads)
+        s_m4[k % kTypes * kTypes + k / kTypes] = -4.0f * (kLambda * (lj_raw[k] - kE0));
+    if (t < kTypes)
+        s_m4[kTypes * kTypes + t] = 0.0f;
     // the async form's output other than the total: zeroed by every CTA, a slice each
     if (async_out != nullptr && async_count > 1) {
         const int per = (async_count - 1 + (int)gridDim.x - 1) / (int)gridDim.x;
@@ -367,258 +367,131 @@ __global__ void __launch_bounds__(kThreads) k_tile_energy(const float4 *__restri
         for (int k = k0 + t; k < k1; k += kThreads)
             async_out[k] = 0.0f;
     }
-
-    for (int k = t; k < 400; k += kThreads)
-    {
-        const float e = kLambda * (lj_raw[k] - kE0);  // Eij in RT units, as the kernel forms it
-        s_eij[k] = e;
-        s_m4[k] = -4.0f * e;
-    }
-    __syncthreads();
-    // residue types are checked once per residue (0..19; padding is excluded anyway):
-    // the pair loop then indexes the table without a bounds test
+    // residue types are checked once per residue (0..19; padding is excluded anyway): the
+    // pair loops then index the table without a bounds test
     unsigned bad = 0;
-    unsigned qb = 0, rb = 0;  // this x warp's charged and real (not padding) residues
-    if (t < kTile) {
-        const float4 px = px_in, mx = mx_in;
-        float xdom, xmol;
-        const float xbond = frac_int(px.w, xdom);
-        const float xchain = frac_int(mx.w, xmol);
-        const bool pad = px.w == kPadder;
-        const bool crowd = mx.w == kCrowder;
+    if (warp < NX) {
+        const bool pad = px.w == kPadder, crowd = mx.w == kCrowder;
         int xt = __float2int_rn(mx.x);
-        if ((unsigned)xt >= 20u) {
+        if ((unsigned)xt >= (unsigned)kTypes) {
             // crowders read no table entry where they are excluded (kNC) or repulsive
             // only (kRC; the reference then gives them the type -1)
             bad |= (pad || (crowd && (kNC || kRC))) ? 0u : 1u;
             xt = 0;
         }
-        const int xflags = (pad ? 1 : 0) | (crowd ? 2 : 0);
-        s_px[t] = make_float4(px.x, px.y, px.z, mx.z);
-        s_xk[t] = make_float4(xdom, xbond, xchain, xmol);
-        s_xm[t] = make_float4(mx.y, __int_as_float(xt), __int_as_float(xflags), 0.f);
-        warp_keys(s_wk[0][t >> 5], xdom, xbond, xchain, xmol, xflags);
-        qb = __ballot_sync(0xffffffffu, !pad && mx.y != 0.0f);
-        rb = __ballot_sync(0xffffffffu, !pad);
+        build_block(s_x[warp], px, mx, xt, !pad && !(kNC && crowd), pad, crowd);
     }
-    if (sub == 0) {
-        float ydom0, ymol0;
-        const float ybond0 = frac_int(py.w, ydom0);
-        const float ychain0 = frac_int(my.w, ymol0);
-        warp_keys(s_wk[1][t >> 5], ydom0, ybond0, ychain0, ymol0,
-                  (py.w == kPadder ? 1 : 0) | (my.w == kCrowder ? 2 : 0));
-    }
-    __syncthreads();
-    const int nyw = ny / 32;  // warps that stored y keys
-    // No pair of the two tiles can be excluded when they are different tiles (where
-    // crowders are treated apart, without crowders), their nonzero rigid-domain and bond
-    // keys share no value, and the chain rule (|x - y| < 4 on one chain) cannot apply
-    // (tiles two or more apart, or no common chain key); for the non-crowder sum also no
-    // common molecule.  Disjoint key ranges show the first ones.  (Padding carries no
-    // keys and is left out of the charged-first copy.)
-    // (Only the crowder forms decide per tile pair; the default potential per x residue.)
-    bool clean = false;
-    if (kNC || kRC) {
-        auto kx = [&](int k) { return tile_key(s_wk[0], kTile / 32, k); };
-        auto ky = [&](int k) { return tile_key(s_wk[1], nyw, k); };
-        clean = tx != ty && ((kx(8) | ky(8)) & 2) == 0;
-        if (kNC)
-            clean = clean && ranges_disjoint(kx(6), kx(7), ky(6), ky(7));
-        else
-            clean = clean && ranges_disjoint(kx(0), kx(1), ky(0), ky(1)) && ranges_disjoint(kx(2), kx(3), ky(2), ky(3)) &&
-                    (tx - ty >= 2 || ranges_disjoint(kx(4), kx(5), ky(4), ky(5)));
-    }
-    // The default potential always takes the charged-first loop: each x residue that may
-    // form an excluded pair with this CTA's y residues (a diagonal tile; its nonzero domain
-    // or bond key inside the y residues' ranges; its chain key inside theirs where the
-    // chain rule can apply) is tested per pair, the others are not.  The crowder forms
-    // take it for clean tile pairs only, the general loop otherwise.
-    const bool cfirst = clean || (!kNC && !kRC);
-    int e[4] = {0, 0, 0, 0};  // ends of the copy's groups (see charged_first_pairs)
-    if (cfirst) {
-        // the x tile's real residues in the order [charged safe | charged tested | uncharged
-        // safe | uncharged tested] (stable within each group), padding after them: the
-        // Debye-Hueckel term is then taken for the charged x residues only
-        unsigned gm[5] = {0u, 0u, 0u, 0u, 0u};  // this x warp's residues by group
-        if (t < kTile) {
-            bool u = false;
-            if (!kNC && !kRC) {
-                const float4 xk = s_xk[t];
-                const int d = __float_as_int(xk.x + 0.0f), b = __float_as_int(xk.y + 0.0f),
-                          ch = __float_as_int(xk.z + 0.0f);
-                u = tx == ty || (xk.x != 0.f && tile_key(s_wk[1], nyw, 0) <= d && d <= tile_key(s_wk[1], nyw, 1)) ||
-                    (xk.y != 0.f && tile_key(s_wk[1], nyw, 2) <= b && b <= tile_key(s_wk[1], nyw, 3)) ||
-                    (tx - ty <= 1 && tile_key(s_wk[1], nyw, 4) <= ch && ch <= tile_key(s_wk[1], nyw, 5));
-            }
-            const unsigned ub = __ballot_sync(0xffffffffu, u);
-            {
-                const float4 xk = s_xk[t];
-                const bool tst = u && ((rb >> (t & 31)) & 1u);
-                const int inf = 0x7fffffff;
-                const int d = __float_as_int(xk.x + 0.0f), b = __float_as_int(xk.y + 0.0f),
-                          ch = __float_as_int(xk.z + 0.0f);
-                const int v[8] = {tst && xk.x != 0.f ? d : inf, tst && xk.x != 0.f ? d : -1,
-                                  tst && xk.y != 0.f ? b : inf, tst && xk.y != 0.f ? b : -1,
-                                  tst ? ch : inf, tst ? ch : -1, tst ? d : inf, tst ? d : -1};
-                int r[8];
-#pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    r[k] = (k & 1) ? __reduce_max_sync(0xffffffffu, v[k]) : __reduce_min_sync(0xffffffffu, v[k]);
-                if ((t & 31) == 0)
-#pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        s_tk[t >> 5][k] = r[k];
-            }
-            gm[0] = qb & ~ub;
-            gm[1] = qb & ub;
-            gm[2] = rb & ~qb & ~ub;
-            gm[3] = rb & ~qb & ub;
-            gm[4] = ~rb;
-            if ((t & 31) == 0)
-#pragma unroll
-                for (int g = 0; g < 5; ++g)
-                    s_gcnt[t >> 5][g] = __popc(gm[g]);
-        }
-        __syncthreads();
-        int acc = 0;
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-            for (int w = 0; w < kTile / 32; ++w)
-                acc += s_gcnt[w][g];
-            e[g] = acc;
-        }
-        if (t < kTile) {
-            // this residue's group g, its members in this warp (mg) and the group's start
-            const int w0 = t >> 5;
-            const unsigned me = 1u << (t & 31);
-            const int g = (gm[0] & me) ? 0 : (gm[1] & me) ? 1 : (gm[2] & me) ? 2 : (gm[3] & me) ? 3 : 4;
-            const unsigned mg = g == 0 ? gm[0] : g == 1 ? gm[1] : g == 2 ? gm[2] : g == 3 ? gm[3] : gm[4];
-            int k = (g == 0 ? 0 : g == 1 ? e[0] : g == 2 ? e[1] : g == 3 ? e[2] : e[3]) + __popc(mg & (me - 1u));
-            for (int w = 0; w < w0; ++w)
-                k += s_gcnt[w][g];
-            const float4 xm = s_xm[t];
-            float4 pw = s_px[t];
-            pw.w *= 0.5f;  // half the radius: sigma_ij = half_y + half_x
-            s_pq[k] = pw;
-            s_qt[k] = make_float2(xm.x, xm.y);
-            const float4 xk = s_xk[t];
-            s_qk[k] = make_float4(xk.x, xk.y, xk.z, __int_as_float(t));
-        }
-        __syncthreads();
-    }
-
-    FF lj{0.f, 0.f}, dh{0.f, 0.f};
-    const bool ycrowd = my.w == kCrowder;
+    // this thread's y residue and its warp's keys
+    const bool ypad = py.w == kPadder, ycrowd = my.w == kCrowder;
     const bool active = (py.w > kPadder) && (!kNC || !ycrowd);
-    // Default potential, per y residue against the tested x residues (keys s_tk): it is
-    // safe when none of its keys can meet theirs (an off-diagonal tile; its nonzero domain
-    // and bond keys outside their ranges; its chain key too where the chain rule can
-    // apply), and all-excluded when they all share its nonzero domain.  A warp whose y
-    // residues are all one or the other takes the tested groups without tests (the
-    // all-excluded residues skip them); otherwise it tests per pair.
-    bool skip_tested = false, wtested = true;
-    if (!kNC && !kRC && cfirst) {
-        // the tested residues' key k: lane k combines the x warps' values, then a broadcast
-        int tk = 0;
-        if ((t & 31) < 8) {
-            const int k = t & 31;
-            tk = s_tk[0][k];
-            for (int w = 1; w < kTile / 32; ++w)
-                tk = (k & 1) ? max(tk, s_tk[w][k]) : min(tk, s_tk[w][k]);
-        }
-        int T[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            T[k] = __shfl_sync(0xffffffffu, tk, k);
-        float yd0, ym0;
-        const float yb0 = frac_int(py.w, yd0);
-        const float yc0 = frac_int(my.w, ym0);
-        const int yd = __float_as_int(yd0 + 0.0f), yb = __float_as_int(yb0 + 0.0f), yc = __float_as_int(yc0 + 0.0f);
-        const bool lsafe = tx != ty && !(yd0 != 0.f && T[0] <= yd && yd <= T[1]) &&
-                           !(yb0 != 0.f && T[2] <= yb && yb <= T[3]) && !(tx - ty <= 1 && T[4] <= yc && yc <= T[5]);
-        skip_tested = yd0 != 0.f && T[6] == yd && T[7] == yd;
-        wtested = __any_sync(0xffffffffu, active && !lsafe && !skip_tested);
+    float ydom, ymol;
+    const float ybond = frac_int(py.w, ydom), ychain = frac_int(my.w, ymol);
+    const Keys yk = warp_keys(!ypad, ycrowd, ydom, ybond, ychain, ymol);
+    int yt = __float2int_rn(my.x);
+    if ((unsigned)yt >= (unsigned)kTypes) {
+        bad |= (!active || (kRC && ycrowd)) ? 0u : 1u;
+        yt = 0;
     }
-    if (active) {
-        const float L = c_boxdim;
-        const float invL = (L != 0.0f) ? 1.0f / L : 0.0f;
-        float ydom, ymol;
-        const float ybond = frac_int(py.w, ydom);
-        const float ychain = frac_int(my.w, ymol);
-        const bool ydom_nz = ydom != 0.f, ybond_nz = ybond != 0.f;
-        const bool diag = (tx == ty);
-        // the chain rule (|x - y| < 4) can only hold on and next to the diagonal
-        const bool near = (tx - ty) <= 1;
-        int yt = __float2int_rn(my.x);
-        if ((unsigned)yt >= 20u) {
-            bad |= (kRC && ycrowd) ? 0u : 1u;
-            yt = 0;
+    const float L = c_boxdim, invL = (L != 0.0f) ? 1.0f / L : 0.0f;
+    const char *col = reinterpret_cast<const char *>(s_m4 + yt);
+    const bool any_active = __any_sync(0xffffffffu, active);
+    FF lj{0.f, 0.f}, dh{0.f, 0.f};
+    __syncthreads();
+
+    const int ys = ty * (kTile / kBlock) + warp;
+    for (int b = 0; any_active && b < NX; ++b) {
+        const int xs = chunk * NX + b;
+        const XBlock &X = s_x[b];
+        const Keys &xk = X.keys;
+        if (xs < ys || X.k1 + X.k2 == 0)
+            continue;
+        bool none, clean;  // every pair excluded; no pair excluded
+        if (kNC) {
+            none = xk.mlo == xk.mhi && yk.mlo == yk.mhi && xk.mlo == yk.mlo;
+            clean = xs != ys && disjoint(xk.mlo, xk.mhi, yk.mlo, yk.mhi);
+        } else {
+            none = xk.dlo == xk.dhi && yk.dlo == yk.dhi && xk.dlo == yk.dlo && ((xk.flags | yk.flags) & 4) == 0;
+            clean = xs != ys && disjoint(xk.dlo, xk.dhi, yk.dlo, yk.dhi) && disjoint(xk.blo, xk.bhi, yk.blo, yk.bhi) &&
+                    (xs - ys > 1 || disjoint(xk.clo, xk.chi, yk.clo, yk.chi));
+            if (kRC)
+                clean = clean && ((xk.flags | yk.flags) & 2) == 0;
         }
-        const float *erow = s_eij + 20 * yt;
-        const float yq = my.y, ys = my.z;
-        if (cfirst) {
-            const PairCtx c{py, 0.5f * ys, yq, s_m4 + 20 * yt, L, invL, yl, x0, y, diag, near, ydom, ybond, ychain,
-                            ydom_nz, ybond_nz};
-            if (wtested) {
-                if (part == 0)
-                    charged_first_pairs<2, true>(c, s_pq, s_qt, s_qk, e, sub, false, lj, dh);
-                else
-                    charged_first_pairs<4, true>(c, s_pq, s_qt, s_qk, e, sub, false, lj, dh);
+        if (none)
+            continue;
+        if (clean) {
+            // y's image nearest the block's middle; on the axes where that lies inside the half
+            // box less the block's half extent for the whole warp, it is the image of every pair
+            auto image = [&](float d) { return __fadd_rn(__fmaf_rn(d, invL, 12582912.0f), -12582912.0f); };
+            const float3 d = make_float3(X.mid.x - py.x, X.mid.y - py.y, X.mid.z - py.z);
+            const float3 k = make_float3(image(d.x), image(d.y), image(d.z));
+            const float lim = 0.5f * L - kImageSlack;
+            auto outside = [&](float dd, float kk, float half) {
+                return !(fabsf(fmaf(-L, kk, dd)) + half < lim && fabsf(kk) <= 2.0f);  // (-L k is exact)
+            };
+            const unsigned mode = (outside(d.x, k.x, X.half.x) ? 1u : 0u) | (outside(d.y, k.y, X.half.y) ? 2u : 0u) |
+                                  (outside(d.z, k.z, X.half.z) ? 4u : 0u) |
+                                  (k.x != 0.0f || k.y != 0.0f || k.z != 0.0f ? 8u : 0u);
+            const unsigned any = __reduce_or_sync(0xffffffffu, active && L != 0.0f ? mode : 0u);
+            const YLane yl{f2_dup(-py.x), f2_dup(-py.y), f2_dup(-py.z), f2_dup(-L * k.x), f2_dup(-L * k.y),
+                           f2_dup(-L * k.z), f2_dup(0.5f * my.z), f2_dup(my.y), col};
+            if (any == 0u)
+                clean_block<kPlain>(X, yl, L, invL, lj, dh);
+            else if (any == 8u)
+                clean_block<kShift>(X, yl, L, invL, lj, dh);
+            else if ((any & 7u) == 1u)
+                clean_block<kShift | 1>(X, yl, L, invL, lj, dh);
+            else if ((any & 7u) == 2u)
+                clean_block<kShift | 2>(X, yl, L, invL, lj, dh);
+            else if ((any & 7u) == 4u)
+                clean_block<kShift | 4>(X, yl, L, invL, lj, dh);
+            else
+                clean_block<7>(X, yl, L, invL, lj, dh);
+            continue;
+        }
+        // branch-free: every pair is evaluated and the excluded ones (padding, the pair
+        // itself on the diagonal: possibly inf / NaN) are selected away
+        const bool ydom_nz = ydom != 0.f, ybond_nz = ybond != 0.f, near = xs - ys <= 1, diag = xs == ys;
+        float l0 = 0.f, l1 = 0.f, d0 = 0.f, d1 = 0.f;
+#pragma unroll 2
+        for (int j = 0; j < kBlock; ++j) {
+            const float4 xkey = X.key[j], xm = X.meta[j], xp = X.pos[j];
+            const int xflags = __float_as_int(xm.z);
+            bool excl = (xflags & 1) || (diag && j <= lane);
+            if (kNC)
+                excl = excl || (xflags & 2) || xkey.w == ymol;
+            else
+                excl = excl || (ydom_nz && xkey.x == ydom) || (ybond_nz && xkey.y == ybond) ||
+                       (near && xkey.z == ychain && abs(xs * kBlock + j - y) < 4);
+            const float dx = min_image(py.x - xp.x, L, invL);
+            const float dy = min_image(py.y - xp.y, L, invL);
+            const float dz = min_image(py.z - xp.z, L, invL);
+            const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+            const float inv_r = rsqrt_sfu(r2);
+            const float m4 = *reinterpret_cast<const float *>(col + __float_as_int(xm.y));
+            float lt = lj_m4(m4, 0.5f * my.z + xp.w, rcp_sfu(r2));
+            float dt = dh_term(my.y * xm.x, r2 * inv_r, inv_r);
+            if (kRC && (ycrowd || (xflags & 2))) {
+                // REPULSIVE_CROWDING (src/CudaFunctions.cu:335-338, :492-498): (6/r)^12 in RT
+                // units below 15 A, no Debye-Hueckel term
+                const float sc = 6.0f * inv_r, s2 = sc * sc, s6 = s2 * s2 * s2;
+                lt = (r2 * inv_r < kRepulsiveCutoff) ? s6 * s6 : 0.f;
+                dt = 0.f;
+            }
+            lt = excl ? 0.f : lt;
+            dt = excl ? 0.f : dt;
+            if (j & 1) {
+                l1 += lt;
+                d1 += dt;
             } else {
-                if (part == 0)
-                    charged_first_pairs<2, false>(c, s_pq, s_qt, s_qk, e, sub, skip_tested, lj, dh);
-                else
-                    charged_first_pairs<4, false>(c, s_pq, s_qt, s_qk, e, sub, skip_tested, lj, dh);
+                l0 += lt;
+                d0 += dt;
             }
         }
-        // the general loop: this thread's share of the x tile, kTile / S consecutive residues
-        const int jw = part ? kTile / 4 : kTile / 2, jb0 = sub * jw;
-        for (int jb = jb0; !cfirst && jb < jb0 + jw; jb += 32) {
-            float l0 = 0.f, l1 = 0.f, d0 = 0.f, d1 = 0.f;
-            // branch-free: every pair is evaluated and the excluded ones (padding, the
-            // pair itself on the diagonal: possibly inf / NaN) are selected away
-#pragma unroll 4
-            for (int jj = 0; jj < 32; ++jj) {
-                const int j = jb + jj;
-                const float4 xk = s_xk[j];
-                const float4 xm = s_xm[j];
-                const float4 px = s_px[j];
-                const int xflags = __float_as_int(xm.z);
-                bool excl = (xflags & 1) || (diag && j <= yl);
-                if (kNC)
-                    excl = excl || (xflags & 2) || xk.w == ymol;
-                else
-                    excl = excl || (ydom_nz && xk.x == ydom) || (ybond_nz && xk.y == ybond) ||
-                           (near && xk.z == ychain && abs(x0 + j - y) < 4);
-                const float dx = min_image(py.x - px.x, L, invL);
-                const float dyy = min_image(py.y - px.y, L, invL);
-                const float dz = min_image(py.z - px.z, L, invL);
-                const float r2 = fmaf(dx, dx, fmaf(dyy, dyy, dz * dz));
-                const float inv_r = rsqrt_sfu(r2);
-                const float r = r2 * inv_r;
-                float lt = lj_term(erow[__float_as_int(xm.y)], (ys + px.w) * 0.5f, inv_r * inv_r);
-                float dt = dh_term(yq * xm.x, r, inv_r);
-                if (kRC && (ycrowd || (xflags & 2))) {
-                    // REPULSIVE_CROWDING (src/CudaFunctions.cu:335-338, :492-498):
-                    // (6/r)^12 in RT units below 15 A, no Debye-Hueckel term
-                    const float sc = 6.0f * inv_r, s2 = sc * sc, s6 = s2 * s2 * s2;
-                    lt = (r < kRepulsiveCutoff) ? s6 * s6 : 0.f;
-                    dt = 0.f;
-                }
-                lt = excl ? 0.f : lt;
-                dt = excl ? 0.f : dt;
-                if (jj & 1) {
-                    l1 += lt;
-                    d1 += dt;
-                } else {
-                    l0 += lt;
-                    d0 += dt;
-                }
-            }
-            ff_add(lj, l0 + l1);
-            ff_add(dh, d0 + d1);
-        }
+        ff_add(lj, l0 + l1);
+        ff_add(dh, d0 + d1);
     }
+    if (!active)
+        lj = dh = FF{0.f, 0.f};
 
     // the stream's next call may be scheduled once every CTA is past its pair work: its
     // CTAs then spread over SMs that are mostly idle, and wait for this kernel to end
@@ -629,13 +502,15 @@ __global__ void __launch_bounds__(kThreads) k_tile_energy(const float4 *__restri
     lj = ff_warp_sum(lj);
     dh = ff_warp_sum(dh);
     bad = __any_sync(0xffffffffu, bad) ? 1u : 0u;
-    if ((t & 31) == 0) {
-        s_red[0][t >> 5] = lj;
-        s_red[1][t >> 5] = dh;
+    if (lane == 0) {
+        s_red[0][warp] = lj;
+        s_red[1][warp] = dh;
         if (bad)
             atomicOr(flags, 1u);
     }
     __syncthreads();
+    const int ngroups = ((int)gridDim.x + kGroup - 1) / kGroup;
+    const int g = blockIdx.x / kGroup, gsize = min(kGroup, (int)gridDim.x - g * kGroup);
     if (t == 0) {
         FF a = s_red[0][0], b = s_red[1][0];
         for (int w = 1; w < kWarps; ++w) {
@@ -644,60 +519,55 @@ __global__ void __launch_bounds__(kThreads) k_tile_energy(const float4 *__restri
         }
         part4[blockIdx.x] = make_float4(a.hi, a.lo, b.hi, b.lo);
         __threadfence();
-        const int g = blockIdx.x / kGroup, gsize = min(kGroup, (int)gridDim.x - g * kGroup);
-        const unsigned done = atomicAdd(&gtickets[g], 1u);
-        s_last = (done == (unsigned)gsize - 1u);
+        s_last = atomicAdd(&gtickets[g], 1u) == (unsigned)gsize - 1u;
     }
     __syncthreads();
-    if (!s_last)
+    if (!s_last || warp != 0)
         return;
 
-    // Last CTA of its group: the group's partials in a fixed order (float-float, one warp).
+    // Last CTA of its group: the group's partials in a fixed order (float-float, one warp);
+    // a call of one group ends here.
     __threadfence();
-    const int ngroups = ((int)gridDim.x + kGroup - 1) / kGroup;
-    if (t < 32) {
-        const int g = blockIdx.x / kGroup, c0 = g * kGroup, gsize = min(kGroup, (int)gridDim.x - c0);
-        FF a{0.f, 0.f}, b{0.f, 0.f};
-        if (t < gsize) {
-            const float4 p = __ldcg(&part4[c0 + t]);
-            a = FF{p.x, p.y};
-            b = FF{p.z, p.w};
-        }
-        a = ff_warp_sum(a);
-        b = ff_warp_sum(b);
-        if (t == 0) {
+    FF a{0.f, 0.f}, b{0.f, 0.f};
+    if (lane < gsize) {
+        const float4 p = __ldcg(&part4[g * kGroup + lane]);
+        a = FF{p.x, p.y};
+        b = FF{p.z, p.w};
+    }
+    a = ff_warp_sum(a);
+    b = ff_warp_sum(b);
+    if (lane == 0)
+        gtickets[g] = 0u;
+    if (ngroups > 1) {
+        unsigned last = 0;
+        if (lane == 0) {
             gsums[g] = make_float4(a.hi, a.lo, b.hi, b.lo);
-            gtickets[g] = 0u;
             __threadfence();
-            const unsigned done = atomicAdd(ticket, 1u);
-            s_last_group = (done == (unsigned)ngroups - 1u);
+            last = atomicAdd(ticket, 1u) == (unsigned)ngroups - 1u;
         }
-    }
-    __syncthreads();
-    if (!s_last_group)
-        return;
-
-    // Last group: every group's sum in a fixed order, float-float, then FP64 once.
-    __threadfence();
-    if (t < 32) {
-        FF a{0.f, 0.f}, b{0.f, 0.f};
-        for (int g = t; g < ngroups; g += 32) {
-            const float4 p = __ldcg(&gsums[g]);
+        if (!__shfl_sync(0xffffffffu, last, 0))
+            return;
+        // Last group: every group's sum in a fixed order, float-float, then FP64 once.
+        __threadfence();
+        a = b = FF{0.f, 0.f};
+        for (int k = lane; k < ngroups; k += 32) {
+            const float4 p = __ldcg(&gsums[k]);
             ff_add_ff(a, FF{p.x, p.y});
             ff_add_ff(b, FF{p.z, p.w});
         }
         a = ff_warp_sum(a);
         b = ff_warp_sum(b);
-        if (t == 0) {
-            const double lj_raw_sum = ff_value(a), dh_raw_sum = ff_value(b);
-            const double total = lj_raw_sum * (double)kRTtoKcal + dh_raw_sum * (double)kDHFactor;
-            result[0] = lj_raw_sum;
-            result[1] = dh_raw_sum;
-            result[2] = total;
-            if (async_out != nullptr && async_count > 0)
-                async_out[0] = (float)total;
+    }
+    if (lane == 0) {
+        const double lj_raw_sum = ff_value(a), dh_raw_sum = ff_value(b);
+        const double total = lj_raw_sum * (double)kRTtoKcal + dh_raw_sum * (double)kDHFactor;
+        result[0] = lj_raw_sum;
+        result[1] = dh_raw_sum;
+        result[2] = total;
+        if (async_out != nullptr && async_count > 0)
+            async_out[0] = (float)total;
+        if (ngroups > 1)
             *ticket = 0u;
-        }
     }
 }
 
@@ -731,7 +601,6 @@ const float *bound_table()
     return it == g_bound_table.end() ? nullptr : it->second;
 }
 
-// Launch the tile kernel on `stream`.  Returns 0 on success.
 // Launch the tile kernel on `stream`.  Returns 0 on success.  On a stream of the caller
 // (the asynchronous entry point) the launch is a programmatic dependent one: the grid
 // may be scheduled once every CTA of the stream's previous kernel has finished its pair
@@ -744,7 +613,13 @@ int launch_energy(bool nc, const float4 *pos, const float4 *meta, int P, const f
     const int nt = (P + kTile - 1) / kTile;
     // crowders take no part in the non-crowder sum, so its form has no crowder variant
     const bool rc = g_repulsive_crowding.load() != 0;
-    auto kern = nc ? k_tile_energy<true, false> : rc ? k_tile_energy<false, true> : k_tile_energy<false, false>;
+    const int nx = x_blocks(nt);
+    auto kern = nc   ? (nx == 4 ? k_tile_energy<true, false, 4> : nx == 2 ? k_tile_energy<true, false, 2>
+                                                                          : k_tile_energy<true, false, 1>)
+                : rc ? (nx == 4 ? k_tile_energy<false, true, 4> : nx == 2 ? k_tile_energy<false, true, 2>
+                                                                          : k_tile_energy<false, true, 1>)
+                     : (nx == 4 ? k_tile_energy<false, false, 4> : nx == 2 ? k_tile_energy<false, false, 2>
+                                                                           : k_tile_energy<false, false, 1>);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)energy_ctas(nt));
     cfg.blockDim = dim3(kThreads);
@@ -935,9 +810,17 @@ namespace {
 
 constexpr int kNoAllocMaxResidues = 16384;                       // datasetSize limit
 constexpr int kNoAllocMaxTiles = kNoAllocMaxResidues / kTile;    // 128-residue tiles
-constexpr int kNoAllocMaxCtas = energy_ctas(kNoAllocMaxTiles);
+constexpr int kNoAllocMaxCtas = 8384;                            // CTAs the array has room for
 constexpr size_t kNoAllocBytes = scratch_bytes(kNoAllocMaxCtas);  // 139,896 bytes (layout: scratch_view)
 static_assert(kNoAllocBytes == 139896, "the documented size of the static scratch");
+constexpr bool no_alloc_fits()
+{
+    for (int nt = 1; nt <= kNoAllocMaxTiles; ++nt)
+        if (energy_ctas(nt) > kNoAllocMaxCtas)
+            return false;
+    return true;
+}
+static_assert(no_alloc_fits(), "every accepted size fits the static scratch");
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 

@@ -44,6 +44,7 @@
 
 #include "cgppd_common.cuh"
 #include "engine_types.h"
+#include "pair_terms.cuh"
 #include "surrogate.cuh"
 
 namespace cg = cooperative_groups;
@@ -413,67 +414,6 @@ __device__ __forceinline__ float pair_kcal(float4 a, float2 qa, float4 b, float2
                                            float invL)
 {
     return pair_term<DH, 7>(a, qa, b, qb.x, table + __float_as_int(qb.y), L, invL);
-}
-
-// ------------------------------------------------------------------ packed pair terms
-
-// Two Lennard-Jones terms (pair_term's arithmetic on packed halves, the repulsive branch
-// left to repulsive2) and what the Debye-Hueckel terms need.
-struct Pair2 {
-    f2 u, r2, inv, m4, s6;
-};
-
-// min_image of two differences; nL holds -L.
-__device__ __forceinline__ f2 min_image2(f2 d, f2 nL, f2 invL)
-{
-    return f2_fma(nL, f2_add(f2_fma(d, invL, f2_dup(12582912.0f)), f2_dup(-12582912.0f)), d);
-}
-
-__device__ __forceinline__ Pair2 lj2(f2 dx, f2 dy, f2 dz, f2 sigma, f2 m4)
-{
-    Pair2 p;
-    p.r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
-    float ra, rb;
-    f2_unpack(p.r2, ra, rb);
-    p.inv = f2_pack(rsqrt_sfu(ra), rsqrt_sfu(rb));
-    p.m4 = m4;
-    const f2 so = f2_mul(sigma, p.inv), s2 = f2_mul(so, so);
-    p.s6 = f2_mul(f2_mul(s2, s2), s2);
-    float sa, sb;
-    f2_unpack(p.s6, sa, sb);
-    p.u = f2_mul(m4, f2_fma(p.s6, p.s6, f2_pack(-sa, -sb)));
-    return p;
-}
-
-// The larger s6 of the two pairs: above 1/2 (closer than 2^(1/6) sigma) one may lie in the
-// repulsive branch's range; rare, so the branch is taken out of the straight path.
-__device__ __forceinline__ float closest2(const Pair2 &p)
-{
-    float a, b;
-    f2_unpack(p.s6, a, b);
-    return fmaxf(a, b);
-}
-
-__device__ __forceinline__ void repulsive2(Pair2 &p)
-{
-    float a, b, ma, mb, ua, ub;
-    f2_unpack(p.s6, a, b);
-    f2_unpack(p.m4, ma, mb);
-    f2_unpack(p.u, ua, ub);
-    if (ma < 0.0f && a > 0.5f)
-        ua = fmaf(-0.5f, ma, -ua);
-    if (mb < 0.0f && b > 0.5f)
-        ub = fmaf(-0.5f, mb, -ub);
-    p.u = f2_pack(ua, ub);
-}
-
-// The terms with the Debye-Hueckel part, qq = q_i q_j of each pair.
-__device__ __forceinline__ f2 with_dh2(const Pair2 &p, f2 qq)
-{
-    const f2 arg = f2_mul(f2_mul(p.r2, p.inv), f2_dup(-kLog2e / kXi));
-    float ea, eb;
-    f2_unpack(arg, ea, eb);
-    return f2_fma(f2_mul(qq, f2_pack(ex2_sfu(ea), ex2_sfu(eb))), p.inv, p.u);
 }
 
 // The mover as the inter pair loop reads it.  Of a span of its residues (all of them, or
