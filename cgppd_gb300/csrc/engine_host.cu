@@ -195,6 +195,7 @@ struct cgppd_engine {
     DevBuf<int> d_sim_da;
     DevBuf<DAStats> d_dastats;
     int report_capacity = 0;
+    int exchanges = 0;  // exchange sweeps enqueued so far (every simulation's count on the device)
     int last_launches = 0;
 
     cudaStream_t own_stream = nullptr;
@@ -1061,7 +1062,9 @@ static int ensure_reports(cgppd_engine *e, int rows)
 {
     if (rows <= e->report_capacity)
         return 0;
-    // keep existing rows
+    // keep existing rows, once the blocks under way have written theirs
+    if (e->report_capacity > 0 && cgppd_check(cudaDeviceSynchronize(), "report rows") != 0)
+        return -1;
     const int cap = std::max(rows, 2 * e->report_capacity);
     DevBuf<float4> nr;
     DevBuf<int2> ne;
@@ -1073,6 +1076,9 @@ static int ensure_reports(cgppd_engine *e, int rows)
         cudaMemcpy(ne.ptr, e->d_exch_report.ptr, sizeof(int2) * (size_t)e->report_capacity * e->sims.size(),
                    cudaMemcpyDeviceToDevice);
     }
+    // (device-to-device copies and clears return early, and not in the blocks' streams)
+    if (cgppd_check(cudaDeviceSynchronize(), "report rows") != 0)
+        return -1;
     std::swap(e->d_report.ptr, nr.ptr);
     std::swap(e->d_report.n, nr.n);
     std::swap(e->d_exch_report.ptr, ne.ptr);
@@ -1084,13 +1090,6 @@ static int ensure_reports(cgppd_engine *e, int rows)
     return 0;
 }
 
-static int exchanges_done(cgppd_engine *e)
-{
-    int st[4] = {0, 0, 0, 0};
-    cudaMemcpy(st, e->d_sim_state.ptr, sizeof(st), cudaMemcpyDeviceToHost);
-    return st[1];
-}
-
 int cgppd_engine_run(cgppd_engine *e, int n_blocks, int steps_per_block, int exchange_after_last, void *stream)
 {
     if (!e->finalized)
@@ -1099,7 +1098,7 @@ int cgppd_engine_run(cgppd_engine *e, int n_blocks, int steps_per_block, int exc
         return 0;
     cudaStream_t st = stream ? (cudaStream_t)stream : e->own_stream;
     // report rows: one per exchange (+1 for a closing report)
-    const int need = exchanges_done(e) + n_blocks + 1;
+    const int need = e->exchanges + n_blocks + 1;
     if (ensure_reports(e, need) != 0)
         return -1;
     EngineArgs a = e->args();
@@ -1128,6 +1127,7 @@ int cgppd_engine_run(cgppd_engine *e, int n_blocks, int steps_per_block, int exc
         if (cgppd_check(cudaGraphLaunch(it->second, st), "graph launch") != 0)
             return -1;
         launches += exch ? 2 : 1;
+        e->exchanges += exch ? 1 : 0;
     }
     e->last_launches = launches;
     return 0;
@@ -1144,10 +1144,8 @@ int cgppd_engine_final_report(cgppd_engine *e, int row, void *stream)
 
 int cgppd_engine_synchronize(cgppd_engine *e)
 {
-    int rc = cgppd_check(cudaStreamSynchronize(e->own_stream), "engine synchronize");
-    if (rc == 0)
-        rc = cgppd_check(cudaDeviceSynchronize(), "engine synchronize");
-    return rc;
+    (void)e;  // (the caller's streams included)
+    return cgppd_check(cudaDeviceSynchronize(), "engine synchronize");
 }
 
 int cgppd_engine_total_replicas(const cgppd_engine *e) { return e->total_replicas; }
@@ -1172,8 +1170,6 @@ int cgppd_engine_recompute(cgppd_engine *e, double *out, int write_state)
 {
     if (!e->finalized)
         return cgppd_fail("cgppd_engine_recompute: engine not finalized");
-    if (cgppd_check(cudaStreamSynchronize(e->own_stream), "recompute") != 0)
-        return -1;
     EngineArgs a = e->args();
     double *dst = write_state ? e->d_potential.ptr : e->d_scratch_pot.ptr;
     if (!write_state) {
@@ -1187,12 +1183,11 @@ int cgppd_engine_recompute(cgppd_engine *e, double *out, int write_state)
     }
     if (cgppd_check(launch_init_energy(a, e->total_replicas, e->init_work, dst, e->own_stream), "recompute") != 0)
         return -1;
-    if (cgppd_check(cudaStreamSynchronize(e->own_stream), "recompute") != 0)
+    if (out && cgppd_check(cudaMemcpyAsync(out, dst, sizeof(double) * e->total_replicas, cudaMemcpyDeviceToHost,
+                                           e->own_stream),
+                           "recompute copy") != 0)
         return -1;
-    if (out)
-        return cgppd_check(cudaMemcpy(out, dst, sizeof(double) * e->total_replicas, cudaMemcpyDeviceToHost),
-                           "recompute copy");
-    return 0;
+    return cgppd_check(cudaStreamSynchronize(e->own_stream), "recompute");
 }
 
 int cgppd_engine_get_replicas(cgppd_engine *e, int sim, double *potentials, float *temperatures, int *labels,
@@ -1466,6 +1461,10 @@ extern "C" int cgppd_engine_restore(cgppd_engine *e, const char *path)
     std::fclose(fp);
     if (rc != 0 || !ok)
         return cgppd_fail("cgppd_engine_restore: truncated or mismatched checkpoint");
+    int st[4] = {0, 0, 0, 0};
+    if (cgppd_check(cudaMemcpy(st, e->d_sim_state.ptr, sizeof(st), cudaMemcpyDeviceToHost), "restore") != 0)
+        return -1;
+    e->exchanges = st[1];
     // rows past the checkpoint's capacity held this engine's earlier run: clear them, as
     // in the engine that wrote the checkpoint (report rows start zeroed)
     if ((int)cap < e->report_capacity) {
