@@ -11,7 +11,6 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
-#include <numeric>
 #include <vector>
 
 #include "cgppd_surrogate.h"
@@ -67,7 +66,9 @@ struct cgppd_surrogate {
     DevBuf<float> stageX, stageO;
     // dataset
     DevBuf<float> dsX, dsY;
-    DevBuf<int> perm;
+    DevBuf<int> perm, partner;
+    DevBuf<unsigned long long> place;
+    DevBuf<unsigned> left;
     std::vector<float> hX, hY;   // host mirror of the dataset (appended by collect/set)
     bool ds_dirty = true;
 
@@ -348,23 +349,22 @@ int cgppd_surrogate_train(cgppd_surrogate *s, int epochs, float lr, float clip, 
         return cgppd_fail("cgppd_surrogate_train: fewer training samples than one batch");
     if (s->upload_dataset())
         return -1;
-    if (s->perm.alloc(ntrain))
+    if (ntrain > INT32_MAX)
+        return cgppd_fail("cgppd_surrogate_train: too many samples");
+    if (s->perm.n < (size_t)ntrain &&
+        (s->perm.alloc(ntrain) || s->partner.alloc(ntrain) || s->place.alloc(ntrain) || s->left.alloc(3)))
         return -1;
-    std::vector<int> perm(ntrain);
     uint64_t rs = s->seed ^ 0x7A11ull;
     const long long nb = ntrain / B;
     if (s->losses.n < (size_t)nb && s->losses.alloc(nb))
         return -1;
     for (int e = 0; e < epochs; ++e) {
-        std::iota(perm.begin(), perm.end(), 0);
-        for (long long i = ntrain - 1; i > 0; --i) {
-            const long long j = (long long)(splitmix64(rs) % (uint64_t)(i + 1));
-            std::swap(perm[i], perm[j]);
-        }
-        if (cgppd_check(cudaMemcpyAsync(s->perm.ptr, perm.data(), ntrain * sizeof(int), cudaMemcpyHostToDevice,
-                                        s->stream),
+        // the order of a sequential shuffle with splitmix64(rs), drawn on the device
+        if (cgppd_check(launch_permutation((int)ntrain, rs, s->perm.ptr, s->partner.ptr, s->place.ptr, s->left.ptr,
+                                           s->max_ctas, s->stream),
                         "permutation"))
             return -1;
+        rs += (uint64_t)(ntrain - 1) * 0x9E3779B97F4A7C15ull;
         for (long long b = 0; b < nb; ++b)
             if (s->enqueue_step(s->dsX.ptr, s->dsY.ptr, s->perm.ptr + b * B, clip, B, true, lr, s->losses.ptr + b))
                 return -1;

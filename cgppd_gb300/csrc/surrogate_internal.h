@@ -4,6 +4,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <cstdint>
+
 #include "surrogate.cuh"
 
 struct cgppd_surrogate;
@@ -61,6 +63,11 @@ cudaError_t launch_net_rows(const NetRowsArgs &a, bool backward, int max_ctas, c
 cudaError_t launch_net_wgrad(const NetWgradArgs &a, cudaStream_t st);
 cudaError_t launch_net_update(const NetUpdateArgs &a, NetUpdateMode mode, cudaStream_t st);
 cudaError_t launch_net_copies(const float *P, __nv_bfloat16 *Wf, __nv_bfloat16 *wtiles, cudaStream_t st);
+
+// perm[0 .. n): the shuffle of 0 .. n - 1 that splitmix64 from `state` gives (permutation.cu;
+// n - 1 words are used).  partner, place: n words each; left: 3 words.
+cudaError_t launch_permutation(int n, uint64_t state, int *perm, int *partner, unsigned long long *place,
+                               unsigned *left, int max_ctas, cudaStream_t st);
 
 // The engine reads a trained surrogate's FP32 parameters and BF16 forward weights.
 const float *surrogate_device_params(const cgppd_surrogate *s);

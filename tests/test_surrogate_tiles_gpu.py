@@ -54,3 +54,35 @@ def test_saturated_units():
     assert np.all(np.isfinite(out))
     assert np.max(np.abs(out - ref)) <= 2e-3 * (1 + np.max(np.abs(ref)))
     s.close()
+
+
+def shuffled(n, seed):
+    """The sequential shuffle of 0..n-1 with splitmix64, as the training order is defined."""
+    mask, s = (1 << 64) - 1, (seed ^ 0x7A11) & ((1 << 64) - 1)
+    p = list(range(n))
+    for i in range(n - 1, 0, -1):
+        s = (s + 0x9E3779B97F4A7C15) & mask
+        z = ((s ^ (s >> 30)) * 0xBF58476D1CE4E5B9) & mask
+        z = ((z ^ (z >> 27)) * 0x94D049BB133111EB) & mask
+        j = (z ^ (z >> 31)) % (i + 1)
+        p[i], p[j] = p[j], p[i]
+    return p
+
+
+@pytest.mark.parametrize("n", [128, 129, 200, 1025, 5000, 152 * 1024 + 7])
+def test_training_order_is_the_sequential_shuffle(n):
+    """Targets that are all zero but for the row number: the mean squared error of a batch of
+    a network that predicts zero names its rows.  (A learning rate that leaves the
+    parameters where they are; history holds the mean over every 16th batch and the last.)"""
+    s = sg.Surrogate(batch=128, seed=17)
+    s.params = np.zeros(sg.N_PARAMS, np.float32)
+    y = (1.0 + np.arange(n, dtype=np.float64) / n).astype(np.float32)
+    s.add_samples(pose_like(np.random.default_rng(2), n), y)
+    hist = s.train(1, lr=1e-30, clip=25.0, val_fraction=0.0)
+    p, nb = shuffled(n, 17), n // 128
+    logged = [b for b in range(nb) if b % 16 == 0 or b == nb - 1]
+    want = np.sqrt(np.mean([np.mean(y[p[128 * b:128 * b + 128]].astype(np.float64) ** 2) for b in logged]))
+    # 128-term float sums and the float32 mean: a few times 2^-24; another order of n rows
+    # differs by about 1e-2 / sqrt(batches)
+    assert hist[0, 0] == pytest.approx(want, rel=2e-6)
+    s.close()
