@@ -184,7 +184,7 @@ struct cgppd_engine {
     int total_replicas = 0;
     int max_n = 0, max_m = 0, max_mol = 0;
     int lmax[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};  // largest per-simulation static list sizes
-    int resident = 0, any_flexible = 0;
+    int resident = 0, early = 0, any_flexible = 0;
     int resident_pref = 1;
     // delayed acceptance
     cgppd_surrogate *sur = nullptr;
@@ -311,6 +311,7 @@ struct cgppd_engine {
             a.lmax[k] = lmax[k];
         a.resident = resident;
         a.any_flexible = any_flexible;
+        a.early = early;
         // the charged-first mover order (Debye-Hueckel terms for charged residues only)
         // pays off for rigid systems with long per-thread i loops; elsewhere it lengthens
         // the kernel for nothing (measured: C2 +6 %, C3 +10 %; C4 -3 % and C1 -3 % when
@@ -698,7 +699,10 @@ static void configure_shape(cgppd_engine *e, int C, int T)
     const size_t s_res = engine_smem_bytes(e->max_mol, e->max_n, e->max_m, C, 1, e->any_flexible, da, e->lmax);
     const size_t s_da = da ? s_res - engine_smem_bytes(e->max_mol, e->max_n, e->max_m, C, 1, e->any_flexible, 0, e->lmax) : 0;
     e->resident = (e->resident_pref != 0) && s_res <= 212 * 1024 + s_da && s_res <= 226 * 1024;
-    e->smem = engine_smem_bytes(e->max_mol, e->max_n, e->max_m, C, e->resident, e->any_flexible, da, e->lmax);
+    // room for the next proposal beside the current one, where that does not cost residency
+    e->early = e->resident && !da &&
+               engine_smem_bytes(e->max_mol, e->max_n, e->max_m, C, 2, e->any_flexible, 0, e->lmax) <= 212 * 1024;
+    e->smem = engine_smem_bytes(e->max_mol, e->max_n, e->max_m, C, e->resident + e->early, e->any_flexible, da, e->lmax);
 }
 
 // Autotuner: time k_mc for each candidate launch shape on scratch copies of the mutable
@@ -857,6 +861,7 @@ static int autotune(cgppd_engine *e, int fixed_cluster, int fixed_threads)
             EngineArgs a = base;
             a.cluster = C;
             a.resident = e->resident;
+            a.early = e->early;
             if (launch_mc_block(a, e->total_replicas, 4, T, e->smem, e->own_stream) != cudaSuccess) {
                 cudaGetLastError();  // a shape the device cannot schedule: skip it
                 continue;

@@ -1,6 +1,6 @@
 // engine_kernels.cu -- device side of the batched replica-exchange Monte Carlo engine.
 //
-// k_mc<RES, DA, QF>: one thread-block cluster per replica runs `nsteps` Monte Carlo steps of
+// k_mc<RES, DA, QF, FLEX>: one thread-block cluster per replica runs `nsteps` Monte Carlo steps of
 // that replica with no inter-replica traffic (replicas are independent between
 // exchanges); every replica of every simulation is in the one launch.  A step restates
 // Replica::MCSearch (src/Replica.cpp:350-414):
@@ -33,6 +33,11 @@
 //
 // QF = true: a rigid mover is also kept in charged-first order, and the pair loop takes
 // the Debye-Hueckel term for its charged residues only (most residues carry no charge).
+//
+// FLEX = false: no molecule is flexible; none of the code for such molecules is there.
+//
+// Resident clusters prepare a rigid mover's proposal while the decision before it is taken
+// (two pairs of proposal buffers), unless the same molecule moves twice in a row.
 //
 // k_exchange: one warp per simulation performs the even/odd temperature exchange of
 // Simulation::run (src/Simulation.cpp:770-795), the per-temperature bookkeeping of
@@ -154,8 +159,9 @@ __host__ __device__ inline SmemLayout smem_layout(int max_mol, int slice, int ma
     int off = 0;
     L.table = off;  off += kTableBytes;
     L.mols = off;   off = align16(off + (int)sizeof(DevMol) * max_m);
-    L.ipos = off;   off += 16 * max_mol;
-    L.irel = off;   off += 16 * max_mol;
+    // the proposal; early launches (resident == 2) prepare the next one beside it
+    L.ipos = off;   off += 16 * max_mol * (resident == 2 ? 2 : 1);
+    L.irel = off;   off += 16 * max_mol * (resident == 2 ? 2 : 1);
     L.iexcl = off;  off += any_flexible ? 16 * max_mol : 0;
     L.iq = off;     off = align16(off + 8 * max_mol);
     // the mover's records (MoverView); a flex move's displacements stand in their positions
@@ -756,6 +762,7 @@ __device__ __forceinline__ T ld_state(const T *p)
     return __ldcg(p);
 }
 
+template <bool FLEX>
 __device__ void predecide_move(const Lists &a, const DevSim &S, const DevMol *mols, const float4 rsc,
                                const uint32_t *w, MovePre &pre)
 {
@@ -766,7 +773,7 @@ __device__ void predecide_move(const Lists &a, const DevSim &S, const DevMol *mo
     pre.ri = 0, pre.br_off = 0, pre.br_cnt = 0;
     int kind = 0, null_move = 0, flip = 0;
     int type;
-    if (mol.flags & kMolFlexible) {
+    if (FLEX && (mol.flags & kMolFlexible)) {
         int k = 0;
         if (M > 1) {
             while (k < 3 && (unsigned long long)w[1] >= S.thr4[k])
@@ -795,6 +802,8 @@ __device__ void predecide_move(const Lists &a, const DevSim &S, const DevMol *mo
         break;
     }
     case kFlex: {
+        if (!FLEX)
+            break;
         // Molecule::flex(rng, step) (src/Molecule.cpp:331-413)
         if (mol.nflex == 0) {
             null_move = 1;
@@ -814,6 +823,8 @@ __device__ void predecide_move(const Lists &a, const DevSim &S, const DevMol *mo
         break;
     }
     case kLocal: {
+        if (!FLEX)
+            break;
         // Molecule::make_local_moves (src/Molecule.cpp:415-448): Bernoulli(0.5) picks a
         // crankshaft (1) or a local translation (0) of one residue.
         kind = (w[5] < 2147483648u) ? 1 : 0;
@@ -850,7 +861,15 @@ __device__ void predecide_move(const Lists &a, const DevSim &S, const DevMol *mo
 // and its wrap, the flex pivot, the crankshaft rotation.  `last` (or null): an accepted
 // move that is being committed meanwhile, its positions in `lastpos`; the state of every
 // other molecule is at rest.
-template <bool RES>
+// The molecule's centre after a translation along the decision's direction (rounded step
+// by step: two places evaluate it, with the same bits).
+__device__ __forceinline__ float3 translated(const MovePre &pre, float4 c, float tstep, float box)
+{
+    const auto axis = [&](float x, float u) { return wrapf(__fadd_rn(x, __fmul_rn(u, tstep)), box); };
+    return make_float3(axis(c.x, pre.R[0]), axis(c.y, pre.R[1]), axis(c.z, pre.R[2]));
+}
+
+template <bool RES, bool FLEX>
 __device__ void finish_move(const DevSim &S, const DevMol *mols, const float4 *CEN, const float4 *P, float tstep,
                             const float4 rsc, const MovePre &pre, MoveDesc &mv, const MoveDesc *last,
                             const float4 *lastpos)
@@ -880,19 +899,18 @@ __device__ void finish_move(const DevSim &S, const DevMol *mols, const float4 *C
     mv.wcx = c.x, mv.wcy = c.y, mv.wcz = c.z;
     const float4 *Pm = moved ? lastpos : P + mv.start;
     switch (ptype) {
-    case kTranslate:
-        mv.vx = pre.R[0] * tstep, mv.vy = pre.R[1] * tstep, mv.vz = pre.R[2] * tstep;
-        mv.wcx = wrapf(c.x + mv.vx, box);
-        mv.wcy = wrapf(c.y + mv.vy, box);
-        mv.wcz = wrapf(c.z + mv.vz, box);
+    case kTranslate: {
+        const float3 w = translated(pre, c, tstep, box);
+        mv.wcx = w.x, mv.wcy = w.y, mv.wcz = w.z;
         break;
+    }
     case kRotate:
 #pragma unroll
         for (int k = 0; k < 9; ++k)
             mv.R[k] = pre.R[k];
         break;
     case kFlex: {
-        if (pnull)
+        if (!FLEX || pnull)
             break;
 #pragma unroll
         for (int k = 0; k < 9; ++k)
@@ -902,7 +920,7 @@ __device__ void finish_move(const DevSim &S, const DevMol *mols, const float4 *C
         break;
     }
     case kLocal: {
-        if (pnull)
+        if (!FLEX || pnull)
             break;
         float vx, vy, vz;
         if (pkind == 0) {
@@ -1166,7 +1184,7 @@ __device__ void da_init_matrix(DaView &v, const DevMol *mols, const float4 *Q, c
 
 // ------------------------------------------------------------------ MC kernel
 
-template <bool RES, bool DA, bool QF>
+template <bool RES, bool DA, bool QF, bool FLEX>
 __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -1186,6 +1204,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
     __shared__ DaView s_dv;
 
     const int C = a.cluster;
+    const int any_flexible = FLEX ? a.any_flexible : 0;
     const int t = threadIdx.x, T = blockDim.x, lane = t & 31, warp = t >> 5, NW = T >> 5;
     int rank = 0;
     if (C > 1)
@@ -1203,13 +1222,11 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
     const int N = S.N, M = S.M;
     const int slice = (a.max_n + C - 1) / C;
     const SmemLayout Ly =
-        smem_layout(a.max_mol, slice, a.max_m, a.max_n, RES ? 1 : 0, a.any_flexible, DA ? 1 : 0, C, a.lmax);
+        smem_layout(a.max_mol, slice, a.max_m, a.max_n, RES ? 1 + a.early : 0, any_flexible, DA ? 1 : 0, C, a.lmax);
     // screening is on for this simulation (uniform over the cluster: one simulation)
     const bool da_on = DA && a.sim_da[s] != 0;
     float *s_table = reinterpret_cast<float *>(smem + Ly.table);
     DevMol *s_mols = reinterpret_cast<DevMol *>(smem + Ly.mols);
-    float4 *s_ipos = reinterpret_cast<float4 *>(smem + Ly.ipos);
-    float4 *s_irel = reinterpret_cast<float4 *>(smem + Ly.irel);
     int4 *s_iexcl = reinterpret_cast<int4 *>(smem + Ly.iexcl);
     float4 *s_disp = reinterpret_cast<float4 *>(smem + Ly.idisp);
     float2 *s_iq = reinterpret_cast<float2 *>(smem + Ly.iq);
@@ -1240,7 +1257,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
     // into a byte (33 instead of 48 bytes per residue)
     const float4 *ST = gST;
     const unsigned char *TY = RES ? reinterpret_cast<const unsigned char *>(smem + Ly.ST) : nullptr;
-    const int4 *EX = (RES && a.any_flexible) ? reinterpret_cast<const int4 *>(smem + Ly.EX) : gEX;
+    const int4 *EX = (RES && any_flexible) ? reinterpret_cast<const int4 *>(smem + Ly.EX) : gEX;
     float4 *CEN = RES ? reinterpret_cast<float4 *>(smem + Ly.CEN) : gCEN;
     // resident copies of the pair matrix, internal energies and row sums are float-float
     // (converted from / to the global doubles at launch start and end)
@@ -1267,7 +1284,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
             sQ[i] = make_float4(q.x, q.y, q.z, sr.y);
             sTY[i] = (unsigned char)__float_as_int(sr.z);
         }
-        if (a.any_flexible) {
+        if (any_flexible) {
             int4 *sEX = reinterpret_cast<int4 *>(smem + Ly.EX);
             for (int i = t; i < N; i += T)
                 sEX[i] = gEX[i];
@@ -1320,7 +1337,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
     unsigned errbits = 0;
     if (t == 0)
         s_lists = global_lists(a);
-    if (RES && a.any_flexible) {
+    if (RES && any_flexible) {
         // this simulation's static lists into shared memory
         int2 *lb = reinterpret_cast<int2 *>(smem + Ly.lst[0]);
         int4 *la = reinterpret_cast<int4 *>(smem + Ly.lst[1]);
@@ -1371,7 +1388,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
         // them from the state once per launch (bounding the float-float accumulation of the
         // increments) and carry the difference into the running total.  Every CTA of the
         // cluster evaluates the same sums in the same order.
-        if (a.any_flexible)
+        if (any_flexible)
             for (int k = 0; k < M; ++k) {
                 if (!(s_mols[k].flags & kMolFlexible))
                     continue;
@@ -1423,17 +1440,24 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
             const U4 res = philox4x32_10(ctr, key0, key1);
             w[4 * b + 0] = res.x, w[4 * b + 1] = res.y, w[4 * b + 2] = res.z, w[4 * b + 3] = res.w;
         }
-        predecide_move(Ls, S, s_mols, rsc, w, s_ring[k & (kRing - 1)]);
+        predecide_move<FLEX>(Ls, S, s_mols, rsc, w, s_ring[k & (kRing - 1)]);
     };
     if (warp == NW - 1)
         fill_ring(0);
     __syncthreads();
     if (RES) {
         if (t == 0)
-            finish_move<RES>(S, s_mols, CEN, P, tstep, rsc, s_ring[0], s_mv[0], nullptr, nullptr);
+            finish_move<RES, FLEX>(S, s_mols, CEN, P, tstep, rsc, s_ring[0], s_mv[0], nullptr, nullptr);
         __syncthreads();
     }
 
+    // residue i of the proposal of molecule m2 (from `start2`): its place among the records
+    auto place = [&](int m2, int start2, int i) -> int {
+        if (RES)
+            return s_qpos[start2 + i];
+        return mover_slot(QF ? a.rqpos[S.res_off + start2 + i] : i, mover_plan(s_mols[m2]));
+    };
+    bool ready = false;  // the step's proposal was prepared during the step before
     for (int step = 0; step < nsteps; ++step) {
         const unsigned long long mcstep = step0 + (unsigned long long)step;
         // ---- the move decision: the state-dependent part of the decision whose draw-only
@@ -1442,12 +1466,15 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
         MoveDesc &mv = s_mv[RES ? step & 1 : 0];
         if (!RES) {
             if (t == 0)
-                finish_move<RES>(S, s_mols, CEN, P, tstep, rsc, s_ring[step & (kRing - 1)], mv, nullptr, nullptr);
+                finish_move<RES, FLEX>(S, s_mols, CEN, P, tstep, rsc, s_ring[step & (kRing - 1)], mv, nullptr, nullptr);
             __syncthreads();
         }
         const int n = mv.n, start = mv.start, type = mv.type, m = mv.m;
-        const bool nullm = mv.null_move != 0;
-        const bool flexmol = mv.flexible != 0;
+        const bool nullm = FLEX && mv.null_move != 0;
+        const bool flexmol = FLEX && mv.flexible != 0;
+        const int buf = RES && a.early ? (step & 1) * a.max_mol : 0;
+        float4 *s_ipos = reinterpret_cast<float4 *>(smem + Ly.ipos) + buf;
+        float4 *s_irel = reinterpret_cast<float4 *>(smem + Ly.irel) + buf;
 
         // ---- delayed acceptance, stage 1: the surrogate's energy change of the proposal
         const bool screened = da_on && !nullm && !flexmol;
@@ -1495,20 +1522,16 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
                 s_old_row = ff_from(v + __ldcg(&gINTRA[m]));
         }
 
-        // ---- proposal of the moved molecule
-        // residue i's place among the mover's records
-        auto place = [&](int i) -> int {
-            if (RES)
-                return s_qpos[start + i];
-            return mover_slot(QF ? a.rqpos[S.res_off + start + i] : i, mover_plan(s_mols[m]));
-        };
+        // ---- proposal of the moved molecule, unless it is there already
+        if (!ready) {
         for (int i = t; i < n; i += T) {
             const float4 p = ld_state<RES>(&P[start + i]);
             const float4 q = ld_state<RES>(&Q[start + i]);
             const float4 sr = RES ? make_float4(p.w, q.w, __int_as_float((int)TY[start + i]), 0.f) : ST[start + i];
-            s_iq[i] = make_float2(sr.y, sr.z);
-            if (flexmol)
+            if (flexmol) {
+                s_iq[i] = make_float2(sr.y, sr.z);
                 s_iexcl[i] = EX[start + i];
+            }
             float4 np = p, nq = q;
             if (!nullm) {
                 if (type == kTranslate) {
@@ -1517,7 +1540,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
                     const float3 rr = rot_apply(mv.R, q.x, q.y, q.z);
                     nq = make_float4(rr.x, rr.y, rr.z, 0.f);
                     np = make_float4(mv.cx + rr.x, mv.cy + rr.y, mv.cz + rr.z, 0.f);
-                } else if (type == kLocal) {
+                } else if (FLEX && type == kLocal) {
                     if (i == mv.ri) {
                         nq = make_float4(q.x + mv.vx, q.y + mv.vy, q.z + mv.vz, 0.f);
                         np = make_float4(p.x + mv.vx, p.y + mv.vy, p.z + mv.vz, 0.f);
@@ -1525,18 +1548,18 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
                     nq = make_float4(nq.x - mv.fx, nq.y - mv.fy, nq.z - mv.fz, 0.f);
                     if (mv.wrapped)
                         np = make_float4(nq.x + mv.wcx, nq.y + mv.wcy, nq.z + mv.wcz, 0.f);
-                } else {  // kFlex: displacement pass below
+                } else if (FLEX) {  // kFlex: displacement pass below
                     s_disp[i] = make_float4(0.f, 0.f, 0.f, 0.f);
                 }
             }
-            np.w = sr.x;
+            np.w = sr.x, nq.w = sr.y;
             s_ipos[i] = np;
             s_irel[i] = nq;
-            if (N > n && (nullm || type != kFlex))
-                put_mover(mover, place(i), np, sr.y, __float_as_int(sr.z));
+            if (N > n && (!FLEX || nullm || type != kFlex))
+                put_mover(mover, place(m, start, i), np, sr.y, __float_as_int(sr.z));
         }
         __syncthreads();
-        if (type == kFlex && !nullm) {
+        if (FLEX && type == kFlex && !nullm) {
             // rotate the branch about the pivot, accumulate the displacement
             for (int k = t; k < mv.br_cnt; k += T) {
                 const int i = Ls.branch[mv.br_off + k - Ls.base[kLBranch]];
@@ -1579,7 +1602,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
             for (int i = t; i < n; i += T) {
                 const float4 d = s_disp[i];
                 float4 p = s_ipos[i], q = s_irel[i];
-                q = make_float4((q.x + d.x) - mv.fx, (q.y + d.y) - mv.fy, (q.z + d.z) - mv.fz, 0.f);
+                q = make_float4((q.x + d.x) - mv.fx, (q.y + d.y) - mv.fy, (q.z + d.z) - mv.fz, q.w);
                 if (mv.wrapped)
                     p = make_float4(q.x + mv.wcx, q.y + mv.wcy, q.z + mv.wcz, p.w);
                 else
@@ -1590,10 +1613,11 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
             __syncthreads();
             if (N > n) {  // the displacements are read: their place takes the mover's records
                 for (int i = t; i < n; i += T)
-                    put_mover(mover, place(i), s_ipos[i], s_iq[i].x, __float_as_int(s_iq[i].y));
+                    put_mover(mover, place(m, start, i), s_ipos[i], s_iq[i].x, __float_as_int(s_iq[i].y));
                 __syncthreads();
             }
         }
+        }  // !ready
 
         // ---- inter-molecule pairs: this CTA's slice of the other residues
         // the other N - n residues split evenly over the cluster for this move (the
@@ -1845,6 +1869,13 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
         // Metropolis decision, all in warp 0 (no CTA barrier before the decision) and in
         // float-float arithmetic (FP32 pipe; the FP64 unit is slow on this part)
         const FF *rowv = (C > 1) ? s_row : s_rowp;
+        // the next step's move is of another, rigid molecule: nothing of it depends on the
+        // decision, and the warps that wait for that prepare its proposal meanwhile, in the
+        // second pair of buffers (the proposal took 1,370 of a step's 11,800 cycles for eight
+        // copies of 76 residues: 595 -> 558 us a block of 100 steps)
+        const MovePre &nx = s_ring[(step + 1) & (kRing - 1)];
+        const bool early = RES && !DA && a.early && NW > 1 && step + 1 < nsteps && nx.m != m &&
+                           (!FLEX || !(s_mols[nx.m].flags & kMolFlexible));
         if (warp == 0) {
             FF v{0.f, 0.f};
             for (int b = lane; b < M; b += 32) {
@@ -1936,9 +1967,34 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
                 if (nullm)
                     errbits |= 1u;
             }
-        } else if (warp == NW - 1 && (step & 31) == 15) {
-            fill_ring(step + 17);  // the steps of the next block of 32, half a ring ahead
+        } else {
+            if (early) {
+                const DevMol &nm = s_mols[nx.m];
+                const int start2 = nm.start, n2 = nm.count;
+                const bool rotate = (nx.bits & 15) == kRotate;
+                const float4 c = CEN[nx.m];
+                const float3 w = translated(nx, c, tstep, L);
+                float4 *ipos = reinterpret_cast<float4 *>(smem + Ly.ipos) + (a.max_mol - buf);
+                float4 *irel = reinterpret_cast<float4 *>(smem + Ly.irel) + (a.max_mol - buf);
+                for (int i = t - 32; i < n2; i += T - 32) {
+                    const float4 p = P[start2 + i], q = Q[start2 + i];
+                    float4 np = make_float4(q.x + w.x, q.y + w.y, q.z + w.z, p.w), nq = q;
+                    if (rotate) {
+                        const float3 rr = rot_apply(nx.R, q.x, q.y, q.z);
+                        nq = make_float4(rr.x, rr.y, rr.z, q.w);
+                        np = make_float4(c.x + rr.x, c.y + rr.y, c.z + rr.z, p.w);
+                    }
+                    ipos[i] = np;
+                    irel[i] = nq;
+                    put_mover(mover, place(nx.m, start2, i), np, q.w, (int)TY[start2 + i]);
+                }
+                if (t == T - 32)
+                    finish_move<RES, FLEX>(S, s_mols, CEN, P, tstep, rsc, nx, s_mv[(step + 1) & 1], nullptr, nullptr);
+            }
+            if (warp == NW - 1 && (step & 31) == 15)
+                fill_ring(step + 17);  // the steps of the next block of 32, half a ring ahead
         }
+        ready = early;
         __syncthreads();
 
         // ---- commit
@@ -1946,9 +2002,9 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
         const bool writer = RES || rank == 0;
         if (acc && writer) {
             for (int i = t; i < n; i += T) {
-                float4 p = s_ipos[i], q = s_irel[i];  // s_ipos.w = sigma/2
+                float4 p = s_ipos[i], q = s_irel[i];  // w: sigma/2, charge
                 p.w = RES ? p.w : 0.f;
-                q.w = RES ? s_iq[i].x : 0.f;
+                q.w = RES ? q.w : 0.f;
                 P[start + i] = p;
                 Q[start + i] = q;
             }
@@ -1996,8 +2052,8 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
         // the next step's move, by the last warp while the others commit (a rigid mover leaves
         // it no residues): its thread waited for on its own took a barrier and about 750
         // cycles of every step
-        if (RES && t == T - 32 && step + 1 < nsteps)
-            finish_move<RES>(S, s_mols, CEN, P, tstep, rsc, s_ring[(step + 1) & (kRing - 1)], s_mv[(step + 1) & 1],
+        if (RES && !ready && t == T - 32 && step + 1 < nsteps)
+            finish_move<RES, FLEX>(S, s_mols, CEN, P, tstep, rsc, s_ring[(step + 1) & (kRing - 1)], s_mv[(step + 1) & 1],
                              (!skip && s_accept) ? &mv : nullptr, s_ipos);
         // fraction-bound sample (src/Simulation.cpp:1063-1073, src/Replica.cpp:1037-1063)
         const int freq = S.sample_freq;
@@ -2662,14 +2718,18 @@ cudaError_t launch_pose_samples(const EngineArgs &a, const int4 *items, int n, u
     return cudaGetLastError();
 }
 
-// Every instantiation of k_mc a launch can pick: resident or not x delayed acceptance x
-// charged-first mover order (the last only without delayed acceptance).
-static const std::array<const void *, 6> &mc_kernels()
+// Every instantiation of k_mc a launch can pick: resident or not x delayed acceptance,
+// and without that x charged-first mover order (rigid only) or rigid only or any molecule.
+// An engine without flexible molecules takes a kernel without their code: with it, preparing
+// proposals early left the crowded replicas slower (1,236 -> 1,386 us a block of 100 steps),
+// without it they gain (1,218).
+static const std::array<const void *, 8> &mc_kernels()
 {
-    static const std::array<const void *, 6> k = {
-        (const void *)k_mc<true, false, false>, (const void *)k_mc<false, false, false>,
-        (const void *)k_mc<true, true, false>,  (const void *)k_mc<false, true, false>,
-        (const void *)k_mc<true, false, true>,  (const void *)k_mc<false, false, true>};
+    static const std::array<const void *, 8> k = {
+        (const void *)k_mc<true, false, false, true>,  (const void *)k_mc<false, false, false, true>,
+        (const void *)k_mc<true, true, false, true>,   (const void *)k_mc<false, true, false, true>,
+        (const void *)k_mc<true, false, true, false>,  (const void *)k_mc<false, false, true, false>,
+        (const void *)k_mc<true, false, false, false>, (const void *)k_mc<false, false, false, false>};
     return k;
 }
 
@@ -2700,19 +2760,16 @@ cudaError_t launch_mc_block(const EngineArgs &a, int total_replicas, int nsteps,
             allowed = true;
         }
     }
-    if (a.da) {
-        if (a.resident)
-            return cudaLaunchKernelEx(&cfg, k_mc<true, true, false>, a, nsteps);
-        return cudaLaunchKernelEx(&cfg, k_mc<false, true, false>, a, nsteps);
-    }
-    if (a.qfirst) {
-        if (a.resident)
-            return cudaLaunchKernelEx(&cfg, k_mc<true, false, true>, a, nsteps);
-        return cudaLaunchKernelEx(&cfg, k_mc<false, false, true>, a, nsteps);
-    }
-    if (a.resident)
-        return cudaLaunchKernelEx(&cfg, k_mc<true, false, false>, a, nsteps);
-    return cudaLaunchKernelEx(&cfg, k_mc<false, false, false>, a, nsteps);
+    const auto launch = [&](auto resident, auto general) {
+        return cudaLaunchKernelEx(&cfg, a.resident ? resident : general, a, nsteps);
+    };
+    if (a.da)
+        return launch(k_mc<true, true, false, true>, k_mc<false, true, false, true>);
+    if (a.qfirst)
+        return launch(k_mc<true, false, true, false>, k_mc<false, false, true, false>);
+    if (!a.any_flexible)
+        return launch(k_mc<true, false, false, false>, k_mc<false, false, false, false>);
+    return launch(k_mc<true, false, false, true>, k_mc<false, false, false, true>);
 }
 
 cudaError_t set_mc_smem_limit(size_t smem)

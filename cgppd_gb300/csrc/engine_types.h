@@ -165,13 +165,14 @@ struct EngineArgs {
     int ntypes;
     int cluster;                 // CTAs per replica
     int resident;                // 1: each CTA keeps its replica's state in shared memory
+    int early;                   // 1: resident, with room to prepare the next step's proposal early
     int any_flexible;            // some molecule carries internal energy terms
-    int qfirst;                  // 1: k_mc<.., .., true> reads rigid movers charged first
+    int qfirst;                  // 1: k_mc<.., .., true, ..> reads rigid movers charged first
     int max_n;                   // largest N
     int max_m;                   // largest M
     int max_mol;                 // largest molecule
     int lmax[10];                // largest per-simulation count of each static list
-    // delayed acceptance with the learned surrogate (da != 0: k_mc<.., true, false> is launched)
+    // delayed acceptance with the learned surrogate (da != 0: k_mc<.., true, .., ..> is launched)
     int da;
     const float *sur_P;          // FP32 master parameters
     const void *sur_wf;          // BF16 Wf[3][256][256] of layers 2..4

@@ -4,6 +4,8 @@ bound of the other energy tests (1e-5 relative).
 * k_mc's mover records (two residues to a record, g lanes a residue j, charged span
   first): molecules from 1 residue up, odd counts, none or all residues charged, rigid
   and flexible movers, cluster and thread shapes that change g, resident or not;
+* proposals prepared a step ahead: movers with more residues than the threads that prepare
+  them, one molecule (never ahead), two (often not), a flexible one among rigid ones;
 * k_init_pairs' groups (128 and 256 residues of whole molecules): molecules at and past
   the limits, many small ones, crowders with and without the repulsive term.
 """
@@ -72,6 +74,26 @@ def test_flexible_mover_among_others(cluster, threads):
         e.synchronize()
         check_state(e, wl, o)
         e.close()
+
+
+# Proposals prepared a step ahead (resident launches) against launches that never do
+# (global state).  Both take the same draws, so they stay together: each of the 60 steps
+# rounds the mover's coordinates (below 256 A, 1.5e-5 A) and no decision is that close.
+@pytest.mark.parametrize("lengths,segments", [([40], {}), ([97, 30], {}), ([230, 1, 96, 98], {}), ([12] * 9, {}),
+                                              ([33, 40, 120], {1: range(20, 31)})])
+@pytest.mark.parametrize("cluster,threads", [(1, 128), (4, 256)])
+def test_proposals_a_step_ahead(lengths, segments, cluster, threads):
+    wl = system(lengths, 200.0, segments=segments, seed=11)
+    state = {}
+    for resident in (True, False):
+        e = engine_for(wl, wl.sims, cluster=cluster, threads=threads, resident=resident)
+        e.run(2, 30)
+        e.synchronize()
+        check_state(e, wl, oracle_for(wl, wl.sims[0]))
+        state[resident] = [e.state(0, r)[0] for r in range(len(wl.sims[0].temperatures))]
+        e.close()
+    for a, b in zip(state[True], state[False]):
+        assert np.abs(a - b).max() < 2e-3
 
 
 @pytest.mark.parametrize("repulsive", [False, True])
