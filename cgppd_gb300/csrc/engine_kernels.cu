@@ -698,20 +698,6 @@ __device__ __forceinline__ bool bonded_has(const Lists &a, const DevMol &mol, in
     return tq.x == ri || tq.y == ri || tq.z == ri || tq.w == ri;
 }
 
-// Change of the bonded terms that involve residue ri between positions pold and pnew
-// (molecule-relative arrays), thread-strided from t0.
-__device__ void bonded_delta(const Lists &a, const DevMol &mol, const float4 *pnew, const float4 *pold, int ri,
-                             float L, float invL, int t0, int stride, FF &acc)
-{
-    const int nb = mol.nbond, na = mol.nang, nt = mol.ntor;
-    for (int k = t0; k < nb + na + nt; k += stride) {
-        const int kind = (k < nb) ? 0 : (k < nb + na) ? 1 : 2;
-        const int kk = (kind == 0) ? k : (kind == 1) ? k - nb : k - nb - na;
-        if (bonded_has(a, mol, kind, kk, ri))
-            ff_add(acc, bonded_item(a, mol, pnew, L, invL, kind, kk) - bonded_item(a, mol, pold, L, invL, kind, kk));
-    }
-}
-
 // Full internal energy (unexcluded pairs over the molecule's active tiles, indirect
 // subtraction, bonded terms) of a molecule at the state's positions, by one CTA; the
 // same value in every thread.
@@ -1585,26 +1571,27 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
                 s_fred[3 * warp + 2] = sz;
             }
             __syncthreads();
+            // every thread takes the sums and the new centre itself (thread 0 for the record):
+            // one barrier less than reading them from it
+            float fx = 0.f, fy = 0.f, fz = 0.f;
+            for (int w = 0; w < NW; ++w)
+                fx += s_fred[3 * w], fy += s_fred[3 * w + 1], fz += s_fred[3 * w + 2];
+            const float nf = (float)n;
+            fx /= nf, fy /= nf, fz /= nf;
+            const float ncx = mv.cx + fx, ncy = mv.cy + fy, ncz = mv.cz + fz;
+            const float wx = wrapf(ncx, L), wy = wrapf(ncy, L), wz = wrapf(ncz, L);
+            const bool wrapped = (wx != ncx) || (wy != ncy) || (wz != ncz);  // (else w equals nc)
             if (t == 0) {
-                float ax = 0.f, ay = 0.f, az = 0.f;
-                for (int w = 0; w < NW; ++w)
-                    ax += s_fred[3 * w], ay += s_fred[3 * w + 1], az += s_fred[3 * w + 2];
-                const float nf = (float)n;
-                mv.fx = ax / nf, mv.fy = ay / nf, mv.fz = az / nf;
-                const float ncx = mv.cx + mv.fx, ncy = mv.cy + mv.fy, ncz = mv.cz + mv.fz;
-                const float wx = wrapf(ncx, L), wy = wrapf(ncy, L), wz = wrapf(ncz, L);
-                mv.wrapped = (wx != ncx) || (wy != ncy) || (wz != ncz);
-                mv.wcx = mv.wrapped ? wx : ncx;
-                mv.wcy = mv.wrapped ? wy : ncy;
-                mv.wcz = mv.wrapped ? wz : ncz;
+                mv.fx = fx, mv.fy = fy, mv.fz = fz;
+                mv.wrapped = wrapped;
+                mv.wcx = wx, mv.wcy = wy, mv.wcz = wz;
             }
-            __syncthreads();
             for (int i = t; i < n; i += T) {
                 const float4 d = s_disp[i];
                 float4 p = s_ipos[i], q = s_irel[i];
-                q = make_float4((q.x + d.x) - mv.fx, (q.y + d.y) - mv.fy, (q.z + d.z) - mv.fz, q.w);
-                if (mv.wrapped)
-                    p = make_float4(q.x + mv.wcx, q.y + mv.wcy, q.z + mv.wcz, p.w);
+                q = make_float4((q.x + d.x) - fx, (q.y + d.y) - fy, (q.z + d.z) - fz, q.w);
+                if (wrapped)
+                    p = make_float4(q.x + wx, q.y + wy, q.z + wz, p.w);
                 else
                     p = make_float4(p.x + d.x, p.y + d.y, p.z + d.z, p.w);
                 s_ipos[i] = p;
@@ -1735,7 +1722,11 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
         // terms.  Other moves recompute it: a rigid rotation or translation changes the
         // float positions, and with them the energy, at rounding level, which a running
         // total must follow to stay within 1e-5 of the energy of its own coordinates.
+        // Its work is dealt to the cluster's warps in slots, round robin over the CTAs (a warp of
+        // mixed bond, angle and torsion terms runs the three in turn, and CTA after CTA the
+        // first one had it all: 4,000 of a linker step's 10,800 cycles).
         FF iacc{0.f, 0.f};
+        const int slot = warp * C + rank, nslots = C * NW;
         const bool incr = RES && flexmol && !nullm && type == kLocal && !mv.wrapped;
         if (incr && type == kLocal) {
             const DevMol &mol = s_mols[m];
@@ -1744,22 +1735,41 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
             const float4 po = make_float4(po4.x, po4.y, po4.z, pn.w);
             const float2 qr = s_iq[ri];
             const int4 er = s_iexcl[ri];
-            for (int j = rank * T + t; j < n; j += C * T) {
-                if (j == ri || intra_excluded(er, s_iexcl[j]))
-                    continue;
-                const float4 pj = s_ipos[j];  // unmoved: the state's position
-                const float2 qj = s_iq[j];
-                ff_add(iacc, pair_kcal(pn, qr, pj, qj, s_table, L, invL) - pair_kcal(po, qr, pj, qj, s_table, L, invL));
+            // slots of 32 terms, one kind each: pairs, indirect neighbours, then the bonded terms
+            // of the new and of the old positions
+            const int wp = (n + 31) >> 5, wi = wp + ((mol.nind + 31) >> 5);
+            const int wb = (mol.nbond + 31) >> 5, wa = (mol.nang + 31) >> 5, wt = (mol.ntor + 31) >> 5,
+                      half = wb + wa + wt;
+            for (int sl32 = slot; sl32 < wi + 2 * half; sl32 += nslots) {
+                if (sl32 < wp) {
+                    const int j = sl32 * 32 + lane;
+                    if (j >= n || j == ri || intra_excluded(er, s_iexcl[j]))
+                        continue;
+                    const float4 pj = s_ipos[j];  // unmoved: the state's position
+                    const float2 qj = s_iq[j];
+                    ff_add(iacc, pair_kcal(pn, qr, pj, qj, s_table, L, invL) -
+                                     pair_kcal(po, qr, pj, qj, s_table, L, invL));
+                } else if (sl32 < wi) {
+                    const int k = (sl32 - wp) * 32 + lane;
+                    if (k >= mol.nind)
+                        continue;
+                    const int2 pr = Ls.indsub[mol.ind_off + k - Ls.base[kLInd]];
+                    if (pr.x != ri && pr.y != ri)
+                        continue;
+                    const int o = (pr.x == ri) ? pr.y : pr.x;
+                    ff_add(iacc, pair_kcal(po, qr, s_ipos[o], s_iq[o], s_table, L, invL) -
+                                     pair_kcal(pn, qr, s_ipos[o], s_iq[o], s_table, L, invL));
+                } else {
+                    const int h = sl32 - wi, old = h >= half, w = old ? h - half : h;
+                    const int kind = w < wb ? 0 : w < wb + wa ? 1 : 2;
+                    const int k = (w - (kind == 0 ? 0 : kind == 1 ? wb : wb + wa)) * 32 + lane;
+                    const int terms = kind == 0 ? mol.nbond : kind == 1 ? mol.nang : mol.ntor;
+                    if (k < terms && bonded_has(Ls, mol, kind, k, ri)) {
+                        const float e = bonded_item(Ls, mol, old ? P + start : s_ipos, L, invL, kind, k);
+                        ff_add(iacc, old ? -e : e);
+                    }
+                }
             }
-            for (int k = rank * T + t; k < mol.nind; k += C * T) {
-                const int2 pr = Ls.indsub[mol.ind_off + k - Ls.base[kLInd]];
-                if (pr.x != ri && pr.y != ri)
-                    continue;
-                const int o = (pr.x == ri) ? pr.y : pr.x;
-                ff_add(iacc, pair_kcal(po, qr, s_ipos[o], s_iq[o], s_table, L, invL) -
-                                 pair_kcal(pn, qr, s_ipos[o], s_iq[o], s_table, L, invL));
-            }
-            bonded_delta(Ls, mol, s_ipos, P + start, ri, L, invL, rank * T + t, C * T, iacc);
         } else if (flexmol && !incr) {
             // the molecule's active 32 x 32 tiles (on and above the diagonal, holding at least
             // one unexcluded pair); when the cluster has spare warps each tile's i range is
@@ -1770,7 +1780,8 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
             while (sf < 4 && ntiles * sf * 2 <= C * NW)
                 sf <<= 1;
             const int il = 32 / sf;
-            for (int k = rank * NW + warp; k < ntiles * sf; k += C * NW) {
+            const int ntask = ntiles * sf;
+            for (int k = slot; k < ntask; k += nslots) {
                 const int tk = k / sf, ck = k - tk * sf;
                 const int2 tl = Ls.tiles[mt.tile_off + tk - Ls.base[kLTile]];
                 const int ta = tl.x, tb = tl.y;
@@ -1803,23 +1814,26 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
                 }
                 ff_add(iacc, part);
             }
-            {
-                // indirect neighbours not caught by the rules above, and the bonded terms:
-                // on the cluster's warps that hold no tile task when there are any (so
-                // no warp carries both), else over every thread
-                const DevMol &mol = s_mols[m];
-                const int gw = rank * NW + warp, ntask = ntiles * sf, nwarps = C * NW;
-                int b0 = rank * T + t, bstride = C * T;
-                if (ntask < nwarps) {
-                    b0 = (gw >= ntask) ? (gw - ntask) * 32 + lane : 0x7fffffff;
-                    bstride = (nwarps - ntask) * 32;
+            // indirect neighbours not caught by the rules above, and the bonded terms, in slots of
+            // 32 of one kind after the tile tasks
+            const int wi = (mt.nind + 31) >> 5, wb = (mt.nbond + 31) >> 5, wa = (mt.nang + 31) >> 5,
+                      wt = (mt.ntor + 31) >> 5;
+            int first = slot - ntask;  // this warp's first slot past the tiles
+            if (first < 0)
+                first += (-first + nslots - 1) / nslots * nslots;
+            for (int w = first; w < wi + wb + wa + wt; w += nslots) {
+                if (w < wi) {
+                    const int k = w * 32 + lane;
+                    if (k < mt.nind) {
+                        const int2 pr = Ls.indsub[mt.ind_off + k - Ls.base[kLInd]];
+                        ff_add(iacc, -pair_kcal(s_ipos[pr.x], s_iq[pr.x], s_ipos[pr.y], s_iq[pr.y], s_table, L, invL));
+                    }
+                } else {
+                    const int u = w - wi, kind = u < wb ? 0 : u < wb + wa ? 1 : 2;
+                    const int k = (u - (kind == 0 ? 0 : kind == 1 ? wb : wb + wa)) * 32 + lane;
+                    if (k < (kind == 0 ? mt.nbond : kind == 1 ? mt.nang : mt.ntor))
+                        ff_add(iacc, bonded_item(Ls, mt, s_ipos, L, invL, kind, k));
                 }
-                for (int k = b0; k < mol.nind; k += bstride) {
-                    const int2 pr = Ls.indsub[mol.ind_off + k - Ls.base[kLInd]];
-                    ff_add(iacc, -pair_kcal(s_ipos[pr.x], s_iq[pr.x], s_ipos[pr.y], s_iq[pr.y], s_table, L, invL));
-                }
-                if (b0 != 0x7fffffff)
-                    bonded_terms(Ls, mol, s_ipos, L, invL, b0, bstride, iacc);
             }
         }
         __syncthreads();
@@ -2053,8 +2067,8 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
         // it no residues): its thread waited for on its own took a barrier and about 750
         // cycles of every step
         if (RES && !ready && t == T - 32 && step + 1 < nsteps)
-            finish_move<RES, FLEX>(S, s_mols, CEN, P, tstep, rsc, s_ring[(step + 1) & (kRing - 1)], s_mv[(step + 1) & 1],
-                             (!skip && s_accept) ? &mv : nullptr, s_ipos);
+            finish_move<RES, FLEX>(S, s_mols, CEN, P, tstep, rsc, s_ring[(step + 1) & (kRing - 1)],
+                                   s_mv[(step + 1) & 1], (!skip && s_accept) ? &mv : nullptr, s_ipos);
         // fraction-bound sample (src/Simulation.cpp:1063-1073, src/Replica.cpp:1037-1063)
         const int freq = S.sample_freq;
         if (freq > 0 && (long long)(mcstep % (unsigned long long)freq) == freq - 1 &&
