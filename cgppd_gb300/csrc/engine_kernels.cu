@@ -129,23 +129,15 @@ __host__ __device__ inline int align16(int v) { return (v + 15) & ~15; }
 // g-th residue i of the mover, a warp holds floor(32 / g) such groups.  Cost of the busiest
 // thread: passes over the CTA's slice x (ceil(n / g) pairs + a per-j overhead for the
 // loads, the periodic image and the log2(g)-step reduction); the cheapest g wins, ties
-// to the smaller g.
-__host__ __device__ inline int pair_lanes(int n, int N, int C, int W) {
-    const int sl = (N - n + C - 1) / C;
-    int best = 1, best_cost = 0x7fffffff;
-    for (int g = 1; g <= 32 && g <= (n > 1 ? n : 1); ++g) {
-        const int per = W * (32 / g);
-        const int passes = (sl + per - 1) / per;
-        int lg = 0;
-        while ((1 << lg) < g)
-            ++lg;
-        const int cost = passes * ((n + g - 1) / g + 2 + lg);
-        if (cost < best_cost) {
-            best_cost = cost;
-            best = g;
-        }
-    }
-    return best;
+// to the smaller g.  One warp, a lane per g.
+__device__ __forceinline__ int pair_lanes(int n, int N, int C, int W)
+{
+    const int g = (threadIdx.x & 31) + 1;
+    const int sl = (N - n + C - 1) / C, per = W * (32 / g), passes = (sl + per - 1) / per;
+    const int lg = 32 - __clz(g - 1);  // ceil(log2 g), 0 for g = 1
+    const int cost = g <= n ? passes * ((n + g - 1) / g + 2 + lg) : 0x7fffffff;
+    const int best = __reduce_min_sync(0xffffffffu, cost);
+    return __ffs(__ballot_sync(0xffffffffu, cost == best));
 }
 
 enum ListId { kLBond = 0, kLAng, kLTor, kLInd, kLFlex, kLFopt, kLBranch, kLLocal, kLCrank, kLTile };
@@ -379,6 +371,12 @@ __device__ __forceinline__ float3 normalized(float x, float y, float z)
     return make_float3(x, y, z);
 }
 
+
+__device__ __forceinline__ void copy_words(void *dst, const void *src, int words, int t, int T)
+{
+    for (int k = t; k < words; k += T)
+        static_cast<int *>(dst)[k] = static_cast<const int *>(src)[k];
+}
 
 __device__ __forceinline__ void load_table(float *s_table, const float *table, int t, int T)
 {
@@ -717,11 +715,19 @@ __device__ FF intra_full_cta(const Lists &Ls, const DevMol &mol, const float4 *P
             const float2 qj = make_float2(Q[st + j].w, __int_as_float((int)TY[st + j]));
             const int4 ej = EX[st + j];
             const int iend = (tl.x == tl.y) ? j : min(n, tl.x * 32 + 32);
-            for (int i = tl.x * 32; i < iend; ++i) {
-                if (intra_excluded(EX[st + i], ej))
-                    continue;
-                part += pair_kcal(P[st + i], make_float2(Q[st + i].w, __int_as_float((int)TY[st + i])), pj, qj, table,
-                                  L, invL);
+            // (excluded pairs are evaluated and dropped, so that four are in flight)
+            for (int i = tl.x * 32; i < iend; i += 4) {
+                float e[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int ii = st + min(i + q, iend - 1);
+                    e[q] = pair_kcal(P[ii], make_float2(Q[ii].w, __int_as_float((int)TY[ii])), pj, qj, table, L, invL);
+                    if (i + q >= iend || intra_excluded(EX[ii], ej))
+                        e[q] = 0.f;
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    part += e[q];
             }
         }
         ff_add(acc, part);
@@ -1197,12 +1203,10 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
         rank = (int)cg::this_cluster().block_rank();
     const int g = a.rep_order[blockIdx.x / C];
     const int s = a.rep_sim[g];
-    if (t == 0) {
-        S = a.sims[s];
-        st = a.stats[g];
-        if (DA)
-            s_da = a.dastats[g];
-    }
+    copy_words(&S, a.sims + s, (int)sizeof(DevSim) / 4, t, T);
+    copy_words(&st, a.stats + g, (int)sizeof(ReplicaStats) / 4, t, T);
+    if (DA && t == 0)
+        s_da = a.dastats[g];
     __syncthreads();
     const int r = g - S.rep_off;
     const int N = S.N, M = S.M;
@@ -1256,11 +1260,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
     // table row has to be one
     for (int k = t; k < records; k += T)
         mover.qt[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int k = t; k < M; k += T) {
-        DevMol mk = a.mols[S.mol_off + k];
-        pack_plan(mk, pair_lanes(mk.count, N, C, NW), QF ? mk.nq : mk.count);
-        s_mols[k] = mk;
-    }
+    copy_words(s_mols, a.mols + S.mol_off, M * (int)sizeof(DevMol) / 4, t, T);
     if (RES) {
         float4 *sP = P, *sQ = Q, *sC = CEN;
         unsigned char *sTY = reinterpret_cast<unsigned char *>(smem + Ly.ST);
@@ -1269,6 +1269,8 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
             sP[i] = make_float4(p.x, p.y, p.z, sr.x);
             sQ[i] = make_float4(q.x, q.y, q.z, sr.y);
             sTY[i] = (unsigned char)__float_as_int(sr.z);
+            if (QF)
+                s_qpos[i] = a.rqpos[S.res_off + i];
         }
         if (any_flexible) {
             int4 *sEX = reinterpret_cast<int4 *>(smem + Ly.EX);
@@ -1281,25 +1283,26 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
         }
         for (int k = t; k < M * M; k += T)
             EMf[k] = ff_from(__ldcg(&gE[k]));
-        __syncthreads();
-        // where each residue goes when its molecule moves
-        for (int i = t; i < N; i += T) {
-            const DevMol &mk = s_mols[__float_as_int(gST[i].w)];
-            const int o = QF ? a.rqpos[S.res_off + i] : i - mk.start;
-            s_qpos[i] = (unsigned short)mover_slot(o, mover_plan(mk));
-        }
     }
-    // bounding radius of every rigid molecule about its centre (rotations keep it up to
-    // float rounding, which kImageMargin covers); flexible molecules change shape and get
-    // none.  One warp per molecule, after every thread has stored its DevMol records (the
-    // resident load above ends with a barrier; the global-state path has none).
     __syncthreads();
+    // per molecule, one warp: the plan of its inter pair loop; the bounding radius of a rigid
+    // one about its centre (rotations keep it up to float rounding, which kImageMargin
+    // covers; flexible molecules change shape and get none); where its residues go among the
+    // mover's records
     for (int k = warp; k < M; k += NW) {
-        const DevMol &mk = s_mols[k];
+        DevMol &mk = s_mols[k];
+        const int gl = pair_lanes(mk.count, N, C, NW);
+        __syncwarp();
+        if (lane == 0)
+            pack_plan(mk, gl, QF ? mk.nq : mk.count);
+        __syncwarp();
+        const MoverPlan plan = mover_plan(mk);
         float rmax = 0.0f;
         for (int i = lane; i < mk.count; i += 32) {
             const float4 q = RES ? Q[mk.start + i] : __ldcg(&gQ[mk.start + i]);
             rmax = fmaxf(rmax, sqrtf(fmaf(q.x, q.x, fmaf(q.y, q.y, q.z * q.z))));
+            if (RES)
+                s_qpos[mk.start + i] = (unsigned short)mover_slot(QF ? s_qpos[mk.start + i] : i, plan);
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
@@ -1338,29 +1341,34 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
         int *lc = reinterpret_cast<int *>(smem + Ly.lst[10]);
         int2 *ltl = reinterpret_cast<int2 *>(smem + Ly.lst[11]);
         const int *B = S.lbase, *Nn = S.lcount;
-        for (int k = t; k < Nn[kLBond]; k += T)
-            lb[k] = a.bonds[B[kLBond] + k];
-        for (int k = t; k < Nn[kLAng]; k += T)
-            la[k] = a.angles[B[kLAng] + k];
-        for (int k = t; k < Nn[kLTor]; k += T) {
-            lt[k] = a.tors[B[kLTor] + k];
-            ltv[k] = a.torsV[B[kLTor] + k];
-            lts[k] = a.torsS[B[kLTor] + k];
+        // one loop over the words of all lists, so that their loads overlap
+        const void *from[12] = {a.bonds + B[kLBond],   a.angles + B[kLAng],     a.tors + B[kLTor],
+                                a.torsV + B[kLTor],    a.torsS + B[kLTor],      a.indsub + B[kLInd],
+                                a.flexres + B[kLFlex], a.flexopt + B[kLFopt],   a.branch + B[kLBranch],
+                                a.localres + B[kLLocal], a.crankres + B[kLCrank], a.tiles + B[kLTile]};
+        void *const to[12] = {lb, la, lt, ltv, lts, li, lf, lfo, lbr, ll, lc, ltl};
+        const int words[12] = {2 * Nn[kLBond], 4 * Nn[kLAng],  4 * Nn[kLTor],  4 * Nn[kLTor],
+                               4 * Nn[kLTor],  2 * Nn[kLInd],  4 * Nn[kLFlex], 4 * Nn[kLFopt],
+                               Nn[kLBranch],   Nn[kLLocal],    Nn[kLCrank],    2 * Nn[kLTile]};
+        int total = 0;
+#pragma unroll
+        for (int j = 0; j < 12; ++j)
+            total += words[j];
+#pragma unroll 4
+        for (int k = t; k < total; k += T) {
+            const int *src = nullptr;
+            int *dst = nullptr;
+            int off = k;
+#pragma unroll
+            for (int j = 0; j < 12; ++j) {
+                if (off >= 0 && off < words[j]) {
+                    src = static_cast<const int *>(from[j]) + off;
+                    dst = static_cast<int *>(to[j]) + off;
+                }
+                off -= words[j];
+            }
+            *dst = *src;
         }
-        for (int k = t; k < Nn[kLInd]; k += T)
-            li[k] = a.indsub[B[kLInd] + k];
-        for (int k = t; k < Nn[kLFlex]; k += T)
-            lf[k] = a.flexres[B[kLFlex] + k];
-        for (int k = t; k < Nn[kLFopt]; k += T)
-            lfo[k] = a.flexopt[B[kLFopt] + k];
-        for (int k = t; k < Nn[kLBranch]; k += T)
-            lbr[k] = a.branch[B[kLBranch] + k];
-        for (int k = t; k < Nn[kLLocal]; k += T)
-            ll[k] = a.localres[B[kLLocal] + k];
-        for (int k = t; k < Nn[kLCrank]; k += T)
-            lc[k] = a.crankres[B[kLCrank] + k];
-        for (int k = t; k < Nn[kLTile]; k += T)
-            ltl[k] = a.tiles[B[kLTile] + k];
         if (t == 0)
             s_lists = Lists{lb, la, lt, ltv, lts, li, lf, lfo, lbr, ll, lc, ltl,
                             {B[0], B[1], B[2], B[3], B[4], B[5], B[6], B[7], B[8], B[9]}};
@@ -1389,13 +1397,17 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
                 }
                 __syncthreads();
             }
-        // row sums: S[m] = intra[m] + sum_b E[m][b]
-        for (int k = t; k < M; k += T) {
-            FF v = INTRAf[k];
-            for (int b = 0; b < M; ++b)
+        // row sums: S[m] = intra[m] + sum_b E[m][b], a warp per row
+        for (int k = warp; k < M; k += NW) {
+            FF v{0.f, 0.f};
+            for (int b = lane; b < M; b += 32)
                 if (b != k)
                     ff_add_ff(v, EMf[(long long)k * M + b]);
-            ROWSUMf[k] = v;
+            v = ff_warp_sum(v);
+            if (lane == 0) {
+                ff_add_ff(v, INTRAf[k]);
+                ROWSUMf[k] = v;
+            }
         }
         __syncthreads();
     }
@@ -2130,21 +2142,22 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
     if (C > 1)  // no CTA leaves while another may still read its shared memory
         cg::this_cluster().sync();
 
-    // ---- write back (rank 0)
+    // ---- write back: every rank holds the whole state and writes a share of it
+    if (RES) {
+        for (int i = rank * T + t; i < N; i += C * T) {
+            const float4 p = P[i], q = Q[i];
+            gP[i] = make_float4(p.x, p.y, p.z, 0.f);
+            gQ[i] = make_float4(q.x, q.y, q.z, 0.f);
+        }
+        for (int k = rank * T + t; k < M * M; k += C * T)
+            gE[k] = ff_value(EMf[k]);
+    }
     if (rank == 0) {
-        if (RES) {
-            for (int i = t; i < N; i += T) {
-                const float4 p = P[i], q = Q[i];
-                gP[i] = make_float4(p.x, p.y, p.z, 0.f);
-                gQ[i] = make_float4(q.x, q.y, q.z, 0.f);
-            }
+        if (RES)
             for (int k = t; k < M; k += T) {
                 gCEN[k] = CEN[k];
                 gINTRA[k] = ff_value(INTRAf[k]);
             }
-            for (int k = t; k < M * M; k += T)
-                gE[k] = ff_value(EMf[k]);
-        }
         if (t == 0) {
             a.potential[g] = ff_value(s_pot);
             a.stats[g] = st;
