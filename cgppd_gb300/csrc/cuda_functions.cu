@@ -39,7 +39,7 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kBlock = 32;                 // residues of an x block and of a warp's y block
 constexpr int kTypes = 20;
 // Tiles of a call from which a CTA takes four (two) x blocks, see x_blocks.
-constexpr int kFourBlocks = 40, kTwoBlocks = 28;
+constexpr int kFourBlocks = 40, kTwoBlocks = 34;
 // Slack (A) on the box test that drops the minimum image: covers the rounding of the
 // relative positions.
 constexpr float kImageSlack = 0.05f;
@@ -296,9 +296,10 @@ __device__ __forceinline__ void clean_block(const XBlock &X, const YLane &y, flo
 
 // x blocks of a CTA for nt tiles of 128 residues: the blocks of a CTA are a serial chain, so
 // one while that leaves SMs short of warps, more once the copies and keys of a CTA cost
-// more than the chain (us a call on three streams with 1 / 2 / 4 blocks: 21 tiles 5.6 /
-// 6.5 / 8.7, 26 tiles 7.1 / 7.3 / 9.6, 39 tiles - / 13.5 / 12.6 but 40 / 43 for one call
-// alone, 55 tiles - / 26.5 / 22.3).
+// more than the chain.  us a call on three streams with 1 / 2 / 4 blocks: 21 tiles 5.6 / 6.5 /
+// 8.7, 28 tiles 8.6 / 9.4, 32 tiles 11.1 / 10.7, 36 tiles 14.2 / 13.1, 39 tiles 16.1 / 14.6 /
+// 12.6, 55 tiles - / 26.5 / 22.3; of a synchronous call with 1 / 2: 28 tiles 28.8 / 31.2, 32
+// tiles 31.0 / 32.9, 36 tiles 34.5 / 35.3, and in bursts on one stream 28 tiles 17.7 / 19.7.
 __host__ __device__ constexpr int x_blocks(int nt) { return nt >= kFourBlocks ? 4 : nt >= kTwoBlocks ? 2 : 1; }
 
 // CTAs of a call: for each tile ty the chunks of x blocks on or after it, rows of

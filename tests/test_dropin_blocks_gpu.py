@@ -77,8 +77,9 @@ def test_block_edges(L, refdata, n, flexible):  # noqa: F811
         check(L, refdata, pos, meta, box)
 
 
-# tiles on both sides of the shapes' limits (28 and 40 tiles), a partial last tile
-@pytest.mark.parametrize("n", [27 * 128, 27 * 128 + 1, 28 * 128 - 31, 39 * 128, 39 * 128 + 5, 41 * 128 + 77])
+# tiles on both sides of the shapes' limits (34 and 40 tiles), a partial last tile
+@pytest.mark.parametrize("n", [27 * 128, 27 * 128 + 1, 28 * 128 - 31, 33 * 128, 33 * 128 + 1, 39 * 128,
+                               39 * 128 + 5, 41 * 128 + 77])
 def test_cta_shapes(L, refdata, n):  # noqa: F811
     rng = np.random.default_rng(n)
     pos, meta = cut(*synthetic_packed(rng, 52, [60, 160, 97], 260.0, 0.1, crowders=4), n)
