@@ -83,10 +83,19 @@ def test_flexible_mover_among_others(cluster, threads):
                                               ([33, 40, 120], {1: range(20, 31)})])
 @pytest.mark.parametrize("cluster,threads", [(1, 128), (4, 256)])
 def test_proposals_a_step_ahead(lengths, segments, cluster, threads):
-    wl = system(lengths, 200.0, segments=segments, seed=11)
+    same_with_and_without_resident_state(system(lengths, 200.0, segments=segments, seed=11), cluster, threads)
+
+
+# 4,600 residues over four CTAs: the replica fits shared memory, a second proposal does not
+def test_no_room_for_a_second_proposal():
+    same_with_and_without_resident_state(system([400] * 11 + [200], 250.0, seed=12), 4, 256)
+
+
+def same_with_and_without_resident_state(wl, cluster, threads):
     state = {}
     for resident in (True, False):
         e = engine_for(wl, wl.sims, cluster=cluster, threads=threads, resident=resident)
+        assert e.launch_shape() == (cluster, threads, resident)
         e.run(2, 30)
         e.synchronize()
         check_state(e, wl, oracle_for(wl, wl.sims[0]))
