@@ -2745,18 +2745,19 @@ cudaError_t launch_pose_samples(const EngineArgs &a, const int4 *items, int n, u
     return cudaGetLastError();
 }
 
-// Every instantiation of k_mc a launch can pick: resident or not x delayed acceptance,
-// and without that x charged-first mover order (rigid only) or rigid only or any molecule.
-// An engine without flexible molecules takes a kernel without their code: with it, preparing
-// proposals early left the crowded replicas slower (1,236 -> 1,386 us a block of 100 steps),
-// without it they gain (1,218).
-static const std::array<const void *, 8> &mc_kernels()
+// Every instantiation of k_mc a launch can pick: resident or not x delayed acceptance or
+// not x any molecule or rigid only, and the charged-first mover order (rigid only, without
+// delayed acceptance).  An engine without flexible molecules takes a kernel without their
+// code: with it, preparing proposals early left the crowded replicas slower (1,236 -> 1,386
+// us a block of 100 steps), without it they gain (1,218).
+static const std::array<const void *, 10> &mc_kernels()
 {
-    static const std::array<const void *, 8> k = {
+    static const std::array<const void *, 10> k = {
         (const void *)k_mc<true, false, false, true>,  (const void *)k_mc<false, false, false, true>,
+        (const void *)k_mc<true, false, false, false>, (const void *)k_mc<false, false, false, false>,
         (const void *)k_mc<true, true, false, true>,   (const void *)k_mc<false, true, false, true>,
-        (const void *)k_mc<true, false, true, false>,  (const void *)k_mc<false, false, true, false>,
-        (const void *)k_mc<true, false, false, false>, (const void *)k_mc<false, false, false, false>};
+        (const void *)k_mc<true, true, false, false>,  (const void *)k_mc<false, true, false, false>,
+        (const void *)k_mc<true, false, true, false>,  (const void *)k_mc<false, false, true, false>};
     return k;
 }
 
@@ -2791,7 +2792,8 @@ cudaError_t launch_mc_block(const EngineArgs &a, int total_replicas, int nsteps,
         return cudaLaunchKernelEx(&cfg, a.resident ? resident : general, a, nsteps);
     };
     if (a.da)
-        return launch(k_mc<true, true, false, true>, k_mc<false, true, false, true>);
+        return a.any_flexible ? launch(k_mc<true, true, false, true>, k_mc<false, true, false, true>)
+                              : launch(k_mc<true, true, false, false>, k_mc<false, true, false, false>);
     if (a.qfirst)
         return launch(k_mc<true, false, true, false>, k_mc<false, false, true, false>);
     if (!a.any_flexible)
