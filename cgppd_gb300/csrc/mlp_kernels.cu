@@ -47,15 +47,7 @@ __device__ __forceinline__ void store16(unsigned char *tile, int unit, int c, co
     *reinterpret_cast<uint4 *>(tile + tc05::tile_offset(unit, c + 1)) = make_uint4(w[4], w[5], w[6], w[7]);
 }
 
-// 2^x on the SFU.  exp(-z) is taken as 2^(-z log2 e), as __expf takes it; flushed
-// results only meet "1 +".
-__device__ __forceinline__ float exp_neg(float z)
-{
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(z * -1.4426950408889634f));
-    return y;
-}
-
+// 1 / x on the SFU: relative error at most 2^-23, results below the normal range flushed.
 __device__ __forceinline__ float rcp_approx(float x)
 {
     float y;
@@ -63,12 +55,13 @@ __device__ __forceinline__ float rcp_approx(float x)
     return y;
 }
 
-// bf16(silu(z)) of 16 values, the same bits as rounding the IEEE quotient z / (1 + exp(-z)):
-// z times the SFU reciprocal is within two units in the last place of it, so the two
-// round to different BF16 values only where the low 16 bits lie that close to a half
-// (0x8000); a pair with such a value (one in 2000; also any for z < -80, where the
-// reciprocal leaves the normal range) takes the divisions.  A third of the division's
-// instructions: the epilogues are bound by issue slots.
+// bf16(silu(z)) of 16 values, the same bits as rounding the quotient z / (1 + exp(-z)).
+// z times the SFU reciprocal is within 2^-22 of that quotient (2^-23 of the reciprocal, half
+// a unit of the product and of the quotient each): four units in the last place.  The two
+// therefore round to different BF16 values only where the low 16 bits lie that close to a
+// half (0x8000); a pair with such a value (one in 2000; also any for z < -80, where the
+// reciprocal nears the end of the normal range) takes the divisions.  A third of the
+// division's instructions: the epilogues are bound by issue slots.
 __device__ __forceinline__ void silu16(const float *z, uint32_t *w)
 {
     // low halves + 0x8008: 0 .. 16 within eight units of the half (the carry into the
@@ -78,7 +71,7 @@ __device__ __forceinline__ void silu16(const float *z, uint32_t *w)
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const float z0 = z[2 * i], z1 = z[2 * i + 1];
-        const float h0 = z0 * rcp_approx(1.0f + exp_neg(z0)), h1 = z1 * rcp_approx(1.0f + exp_neg(z1));
+        const float h0 = z0 * rcp_approx(1.0f + __expf(-z0)), h1 = z1 * rcp_approx(1.0f + __expf(-z1));
         w[i] = pack_bf16(h0, h1);
         near_half[i] = __byte_perm(__float_as_uint(h0), __float_as_uint(h1), 0x5410) + 0x80088008u;
         lows = __vminu2(lows, near_half[i]);
@@ -90,26 +83,6 @@ __device__ __forceinline__ void silu16(const float *z, uint32_t *w)
         for (int i = 0; i < 8; ++i)
             if ((near_half[i] & 0xffffu) < 18u || near_half[i] < (18u << 16) || low)
                 w[i] = pack_bf16(silu(z[2 * i]), silu(z[2 * i + 1]));
-    }
-}
-
-// silu'(z) of 16 values, the same bits as silu_grad: the sigmoid 1 / (1 + exp(-z)) is the
-// SFU reciprocal and one Newton step with the exact residual (equal to the IEEE quotient
-// for every z >= -80, checked over all of them; a thread with a smaller z divides).
-__device__ __forceinline__ void silu_slope16(const float *z, float *g)
-{
-    float zmin = z[0];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const float d = 1.0f + exp_neg(z[i]), y = rcp_approx(d);
-        const float s = fmaf(y, fmaf(-d, y, 1.0f), y);
-        g[i] = s * (1.0f + z[i] * (1.0f - s));
-        zmin = fminf(zmin, z[i]);
-    }
-    if (!(zmin >= -80.0f)) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-            g[i] = silu_grad(z[i]);
     }
 }
 
@@ -377,17 +350,16 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net_rows(NetRowsArgs a)
         if (!mma_warp) {
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
-                float v[16], g4[16];
+                float v[16];
                 tc05::tmem_ld16(lane_base + (uint32_t)(2 * kTmemBlock + q * 16), v);
 #pragma unroll
                 for (int i = 0; i < 16; ++i)
                     v[i] += b4;
-                silu_slope16(v, g4);
                 uint32_t w[8];
 #pragma unroll
                 for (int i = 0; i < 16; i += 2) {
                     const float d0 = s_do[row0 + q * 16 + i], d1 = s_do[row0 + q * 16 + i + 1];
-                    w[i >> 1] = pack_bf16(d0 * w5 * g4[i], d1 * w5 * g4[i + 1]);
+                    w[i >> 1] = pack_bf16(d0 * w5 * silu_grad(v[i]), d1 * w5 * silu_grad(v[i + 1]));
                 }
                 store16(s_h[0], unit, (row0 >> 3) + 2 * q, w);
             }
@@ -395,11 +367,9 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net_rows(NetRowsArgs a)
         if (!publish())
             break;
         auto weighted_slopes = [](const float *v, const float *z, uint32_t *w) {
-            float d[16];
-            silu_slope16(z, d);
 #pragma unroll
             for (int i = 0; i < 16; i += 2)
-                w[i >> 1] = pack_bf16(v[i] * d[i], v[i + 1] * d[i + 1]);
+                w[i >> 1] = pack_bf16(v[i] * silu_grad(z[i]), v[i + 1] * silu_grad(z[i + 1]));
         };
         auto backward_epilogue = [&](int blk, int zblk, float bias, unsigned char *buf) {
 #pragma unroll
