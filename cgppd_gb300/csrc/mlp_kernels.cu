@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net_rows(NetRowsArgs a)
             forward_epilogue(2, b4, s_h[1]);
         if (!publish())
             break;
-        if (BWD && mma_thread)  // (its readers of shared memory are waited for in the next advance)
+        if (BWD && mma_thread)  // (its read of the tile is waited for before the next publish)
             tc05::bulk_store(a.act + ((size_t)(kActH1 + 3) * ntiles + tile) * kNetTileElems, tc05::smem_u32(s_h[1]),
                              kTileBytes);
         // ---- output: warp w takes rows 8 w .. 8 w + 7, lane l the units l, l + 32, ...
@@ -364,6 +364,8 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net_rows(NetRowsArgs a)
                 store16(s_h[0], unit, (row0 >> 3) + 2 * q, w);
             }
         }
+        if (mma_thread)  // the copy of H4 has read its tile before any warp may pass to writing dZ3 there
+            tc05::bulk_store_wait_read();
         if (!publish())
             break;
         auto weighted_slopes = [](const float *v, const float *z, uint32_t *w) {
