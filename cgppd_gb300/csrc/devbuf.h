@@ -33,18 +33,25 @@ struct DevBuf {
     }
     int upload(const std::vector<T> &v)
     {
-        if (alloc(v.size()) != 0)
-            return -1;
         if (v.empty())
-            return cgppd_check(cudaMemset(ptr, 0, sizeof(T)), "device memset");
-        return cgppd_check(cudaMemcpy(ptr, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice), "device upload");
+            return zero(1);
+        if (alloc(v.size()) != 0 ||
+            cgppd_check(cudaMemcpy(ptr, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice), "device upload") != 0)
+            return -1;
+        return settled();
     }
     int zero(size_t count)
     {
-        if (alloc(count) != 0)
+        if (alloc(count) != 0 || cgppd_check(cudaMemset(ptr, 0, n * sizeof(T)), "device memset") != 0)
             return -1;
-        return cgppd_check(cudaMemset(ptr, 0, n * sizeof(T)), "device memset");
+        return settled();
     }
+
+private:
+    // A clear of device memory (and the end of a copy from pageable memory) runs on the
+    // legacy stream after the call has returned, behind whatever is queued there; the
+    // objects' own streams don't wait for that stream, so the host does.
+    static int settled() { return cgppd_check(cudaStreamSynchronize(cudaStreamLegacy), "device buffer set-up"); }
 };
 
 }  // namespace cgppd

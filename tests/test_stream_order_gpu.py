@@ -1,0 +1,35 @@
+"""The engine's calls while the default stream, which its own stream does not wait for, has
+work to do."""
+import numpy as np
+import pytest
+import torch
+
+from cgppd_gb300 import engine as eng
+from cgppd_gb300 import workloads
+
+pytestmark = pytest.mark.gpu
+
+
+def busy():
+    torch.cuda.synchronize()
+    torch.cuda._sleep(200_000_000)  # about 0.1 s on the default stream
+
+
+def build(config="c4", nrep=4):
+    wl = workloads.make(config)
+    s = wl.sims[0]
+    wl.sims = [workloads.Simulation(s.molecules, s.box, s.temperatures[:nrep], s.translate_steps[:nrep],
+                                    s.rotate_steps[:nrep], s.move_weights, s.rigid_rotate_prob)]
+    return eng.from_workload(wl, cluster=2, threads=256)
+
+
+def test_first_recompute():
+    """The scratch energies are cleared before the first evaluation into them."""
+    e = build()
+    want = e.recompute(write_state=True)
+    busy()
+    got = e.recompute(write_state=False)
+    torch.cuda.synchronize()
+    assert np.array_equal(got, want)
+    assert np.array_equal(e.recompute(write_state=False), want)
+    e.close()

@@ -31,3 +31,20 @@ def test_gradient_while_memory_is_busy():
             assert lb == loss and np.array_equal(g, gb)
         side.synchronize()
     s.close()
+
+
+def test_created_behind_a_busy_default_stream():
+    """The set-up clears and fills buffers while the default stream still has work to do."""
+    rng = np.random.default_rng(7)
+    X, y = pose_like(rng, 256), rng.normal(size=256).astype(np.float32)
+    s = sg.Surrogate(batch=256, seed=21)
+    want = s.params, s.predict(X), *s.loss_grad(X, y)
+    s.close()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(200_000_000)  # about 0.1 s on the default stream
+    s = sg.Surrogate(batch=256, seed=21)
+    got = s.predict(X), *s.loss_grad(X, y)
+    torch.cuda.synchronize()
+    for a, b in zip(want, (s.params, *got)):
+        assert np.array_equal(a, b)
+    s.close()
