@@ -28,9 +28,16 @@ struct DevBuf {
     int alloc(size_t count)
     {
         release();
-        n = std::max<size_t>(count, 1);
-        return cgppd_check(cudaMalloc(&ptr, n * sizeof(T)), "device allocation");
+        const size_t want = std::max<size_t>(count, 1);
+        if (cgppd_check(cudaMalloc(&ptr, want * sizeof(T)), "device allocation") != 0) {
+            ptr = nullptr;
+            return -1;
+        }
+        n = want;
+        return 0;
     }
+    // Room for at least `count` elements (the contents are lost if it grows).
+    int reserve(size_t count) { return n >= count ? 0 : alloc(count); }
     int upload(const std::vector<T> &v)
     {
         if (v.empty())

@@ -219,7 +219,7 @@ struct cgppd_surrogate {
     int predict(const float *Xsrc, int n, float *out_host)
     {
         const int chunk = std::min(n, kStageRows);
-        if (stageO.n < (size_t)chunk && (stageX.alloc((size_t)chunk * kSurIn) || stageO.alloc(chunk)))
+        if (n > 0 && (stageX.reserve((size_t)chunk * kSurIn) || stageO.reserve(chunk)))
             return -1;
         for (int s0 = 0; s0 < n; s0 += chunk) {
             const int cnt = std::min(chunk, n - s0);
@@ -351,12 +351,11 @@ int cgppd_surrogate_train(cgppd_surrogate *s, int epochs, float lr, float clip, 
         return -1;
     if (ntrain > INT32_MAX)
         return cgppd_fail("cgppd_surrogate_train: too many samples");
-    if (s->perm.n < (size_t)ntrain &&
-        (s->perm.alloc(ntrain) || s->partner.alloc(ntrain) || s->place.alloc(ntrain) || s->left.alloc(3)))
+    if (s->perm.reserve(ntrain) || s->partner.reserve(ntrain) || s->place.reserve(ntrain) || s->left.reserve(3))
         return -1;
     uint64_t rs = s->seed ^ 0x7A11ull;
     const long long nb = ntrain / B;
-    if (s->losses.n < (size_t)nb && s->losses.alloc(nb))
+    if (s->losses.reserve(nb))
         return -1;
     for (int e = 0; e < epochs; ++e) {
         // the order of a sequential shuffle with splitmix64(rs), drawn on the device
