@@ -598,7 +598,13 @@ Scratch *scratch_for(cudaStream_t stream, size_t blocks)
         unsigned char *base = nullptr;
         if (cgppd_check(cudaMalloc(&base, scratch_bytes(cap)), "scratch allocation") != 0)
             return nullptr;
-        cudaMemset(base, 0, scratch_bytes(cap));
+        // (the clear runs on the legacy stream, which the caller's stream need not wait for)
+        if (cgppd_check(cudaMemset(base, 0, scratch_bytes(cap)), "scratch clear") != 0 ||
+            cgppd_check(cudaStreamSynchronize(cudaStreamLegacy), "scratch clear") != 0) {
+            cudaFree(base);
+            s = Scratch{};
+            return nullptr;
+        }
         scratch_view(base, cap, s);
     }
     return &s;
