@@ -592,19 +592,18 @@ Scratch *scratch_for(cudaStream_t stream, size_t blocks)
 {
     Scratch &s = g_scratch[std::make_pair(current_device(), stream)];
     if (s.capacity < blocks) {
-        if (s.ticket != nullptr)
-            cudaFree(s.ticket);
-        size_t cap = blocks < 256 ? 256 : blocks;
+        const size_t cap = blocks < 256 ? 256 : blocks;
         unsigned char *base = nullptr;
         if (cgppd_check(cudaMalloc(&base, scratch_bytes(cap)), "scratch allocation") != 0)
-            return nullptr;
+            return nullptr;  // (what there is stays: smaller calls still fit)
         // (the clear runs on the legacy stream, which the caller's stream need not wait for)
         if (cgppd_check(cudaMemset(base, 0, scratch_bytes(cap)), "scratch clear") != 0 ||
             cgppd_check(cudaStreamSynchronize(cudaStreamLegacy), "scratch clear") != 0) {
             cudaFree(base);
-            s = Scratch{};
             return nullptr;
         }
+        if (s.ticket != nullptr)
+            cudaFree(s.ticket);
         scratch_view(base, cap, s);
     }
     return &s;

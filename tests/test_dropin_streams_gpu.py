@@ -30,4 +30,5 @@ def test_first_call_on_a_stream_behind_a_busy_default_stream(L):  # noqa: F811
         stream.synchronize()
         cgppd_gb300.check("EonDevice_async")
         torch.cuda.synchronize()
-        assert float(out[0]) == np.float32(want)
+        # (one rounding to FP32; float-float sums, in whatever order, are far below it)
+        assert abs(float(out[0]) - want) <= 2.0 ** -23 * abs(want) + 1e-9

@@ -1,9 +1,9 @@
 """A call that ran out of device memory leaves no buffer behind that counts as allocated: the
 same call again fails the same way, or works once there is memory.
 
-The surrogate's host code is linked against a stand-in for the CUDA runtime that takes
-device memory from the heap and can refuse any one allocation, and against launchers that
-check the pointers they are given.
+The host code is linked against a stand-in for the CUDA runtime that takes device memory
+from the heap and can refuse any one allocation; the surrogate's also against launchers
+that check the pointers they are given, the energy calls against a launch that does.
 """
 import os
 import subprocess
@@ -18,9 +18,11 @@ build = sys.modules["cgppd_gb300.build"]
 RUNTIME = r"""
 #include <cstdlib>
 #include <cstring>
+#include <set>
 #include <cuda_runtime.h>
 
 int allocations = 0, refuse = 0;
+std::set<void *> freed;
 
 extern "C" {
 cudaError_t cudaMalloc(void **p, size_t n)
@@ -32,7 +34,7 @@ cudaError_t cudaMalloc(void **p, size_t n)
     return cudaSuccess;
 }
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { *p = calloc(n, 1); return cudaSuccess; }
-cudaError_t cudaFree(void *p) { free(p); return cudaSuccess; }
+cudaError_t cudaFree(void *p) { freed.insert(p); return cudaSuccess; }  // (kept, so that no address comes twice)
 cudaError_t cudaFreeHost(void *p) { free(p); return cudaSuccess; }
 cudaError_t cudaMemset(void *p, int v, size_t n) { memset(p, v, n); return cudaSuccess; }
 cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) { memcpy(d, s, n); return cudaSuccess; }
@@ -125,20 +127,71 @@ int main()
 """
 
 
-def test_after_a_refused_allocation(tmp_path):
+ENERGY = r"""
+#include <cstdio>
+#include <set>
+#include <cuda_runtime.h>
+#include "cgppd_cuda_functions.h"
+
+extern int allocations, refuse;
+extern std::set<void *> freed;
+static int bad = 0, launches = 0;
+
+extern "C" cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *, const void *, void **args)
+{
+    for (int k : {5, 6, 7, 8, 9, 10}) {  // the scratch pointers (partials .. group tickets)
+        void *p = *static_cast<void **>(args[k]);
+        for (void *f : freed)
+            if (p == nullptr || (p >= f && p < static_cast<char *>(f) + 512))
+                ++bad;
+    }
+    ++launches;
+    return cudaSuccess;
+}
+
+int main()
+{
+    float4 *p = reinterpret_cast<float4 *>(16);
+    float out[1], table[1];
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(32);
+    auto call = [&](int n) { CUDA_EonDevice_async(p, p, 0, 0, 0, 0, out, 1, 32, n, 0, st); };
+    bindLJTexture(table);
+    call(1000);
+    allocations = 0, refuse = 1;
+    call(8000);  // needs more room and is refused it
+    refuse = 0;
+    call(1000);
+    call(8000);
+    printf("launches %d bad %d\n", launches, bad);
+    return bad != 0 || launches != 3;
+}
+"""
+
+
+def compile_and_run(tmp_path, harness, sources):
     try:
         home = build.cuda_home()
     except RuntimeError:
         pytest.skip("no nvcc")
-    (tmp_path / "harness.cu").write_text(HARNESS)
+    (tmp_path / "harness.cu").write_text(harness)
     (tmp_path / "runtime.cpp").write_text(RUNTIME)
     exe = str(tmp_path / "harness")
     inc = ["-I" + build.CSRC, "-I" + os.path.join(build.ROOT, "include")]
     subprocess.run([os.path.join(home, "bin", "nvcc"), build.GENCODE, "-std=c++17", "--expt-relaxed-constexpr",
-                    "-cudart", "shared"] + inc +
-                   ["-o", exe, str(tmp_path / "harness.cu"), str(tmp_path / "runtime.cpp"), os.path.join(build.CSRC, "surrogate_host.cu"),
-                    os.path.join(build.CSRC, "status.cpp")], check=True)
+                    "-cudart", "shared"] + inc + ["-o", exe, str(tmp_path / "harness.cu"),
+                                                  str(tmp_path / "runtime.cpp")] + sources, check=True)
     env = dict(os.environ, LD_LIBRARY_PATH=os.path.join(home, "lib64"))
     r = subprocess.run([exe], env=env, stdout=subprocess.PIPE, stderr=subprocess.PIPE, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
-    assert "0 1: -1" in r.stdout and "1 1: -1" in r.stdout  # the stand-in did refuse
+    return r.stdout
+
+
+def test_surrogate_after_a_refused_allocation(tmp_path):
+    out = compile_and_run(tmp_path, HARNESS, [os.path.join(build.CSRC, f) for f in ("surrogate_host.cu", "status.cpp")])
+    assert "0 1: -1" in out and "1 1: -1" in out  # the stand-in did refuse
+
+
+def test_energy_call_after_a_refused_allocation(tmp_path):
+    build.build()
+    compile_and_run(tmp_path, ENERGY, [os.path.join(build.BUILD, f) for f in
+                                       ("cuda_functions.cu.o", "host_amino_acids.cpp.o", "status.cpp.o")])
