@@ -183,8 +183,11 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net_rows(NetRowsArgs a)
             if (ok)
                 tc05::mma_commit(&done[half]);
         }
-        if (!ok)
+        if (!ok) {  // the MMAs issued so far, for the wait at the end
+            tc05::mma_commit(&done[1]);
+            issued = g + 1;
             return;
+        }
         used = issued = g + 1;
         if (g + 1 < total) {
             for (int c = 0; c < kRing && ok; ++c)
