@@ -199,6 +199,7 @@ struct cgppd_engine {
     int last_launches = 0;
 
     cudaStream_t own_stream = nullptr;
+    cudaEvent_t ordinary = nullptr;  // see after_ordinary_streams
     std::map<std::pair<int, int>, cudaGraphExec_t> graphs;  // (steps, exchange) -> graph
 
     // device buffers
@@ -248,6 +249,8 @@ struct cgppd_engine {
             cudaGraphExecDestroy(kv.second);
         if (own_stream)
             cudaStreamDestroy(own_stream);
+        if (ordinary)
+            cudaEventDestroy(ordinary);
     }
 
     EngineArgs args() const
@@ -1033,7 +1036,8 @@ int cgppd_engine_finalize(cgppd_engine *e, int cluster, int threads)
         return cgppd_fail("cgppd_engine_finalize: system too large for shared memory (reduce molecule size or N)");
     if (cgppd_check(set_mc_smem_limit(std::max(e->smem, s_init)), "engine shared-memory limit") != 0)
         return -1;
-    if (cgppd_check(cudaStreamCreateWithFlags(&e->own_stream, cudaStreamNonBlocking), "engine stream") != 0)
+    if (cgppd_check(cudaStreamCreateWithFlags(&e->own_stream, cudaStreamNonBlocking), "engine stream") != 0 ||
+        cgppd_check(cudaEventCreateWithFlags(&e->ordinary, cudaEventDisableTiming), "engine stream") != 0)
         return -1;
     EngineArgs a = e->args();
     if (cgppd_check(launch_init_energy(a, e->total_replicas, e->init_work, e->d_potential.ptr, e->own_stream),
@@ -1095,6 +1099,17 @@ static int ensure_reports(cgppd_engine *e, int rows)
     return 0;
 }
 
+// What is enqueued on `st` from here on follows what the legacy stream, and the streams that
+// synchronise with it, hold now: an upload or a block on another such stream, a clear of the
+// sample log.  (On the device: the host does not wait.)
+static int after_ordinary_streams(cgppd_engine *e, cudaStream_t st)
+{
+    return cgppd_check(cudaEventRecord(e->ordinary, cudaStreamLegacy), "order of streams") != 0 ||
+                   cgppd_check(cudaStreamWaitEvent(st, e->ordinary, 0), "order of streams") != 0
+               ? -1
+               : 0;
+}
+
 int cgppd_engine_run(cgppd_engine *e, int n_blocks, int steps_per_block, int exchange_after_last, void *stream)
 {
     if (!e->finalized)
@@ -1104,7 +1119,7 @@ int cgppd_engine_run(cgppd_engine *e, int n_blocks, int steps_per_block, int exc
     cudaStream_t st = stream ? (cudaStream_t)stream : e->own_stream;
     // report rows: one per exchange (+1 for a closing report)
     const int need = e->exchanges + n_blocks + 1;
-    if (ensure_reports(e, need) != 0)
+    if (ensure_reports(e, need) != 0 || after_ordinary_streams(e, st) != 0)
         return -1;
     EngineArgs a = e->args();
     const int nsims = (int)e->sims.size();

@@ -15,6 +15,9 @@ def busy():
     torch.cuda._sleep(200_000_000)  # about 0.1 s on the default stream
 
 
+LEGACY = 1  # cudaStreamLegacy
+
+
 def build(config="c4", nrep=4):
     wl = workloads.make(config)
     s = wl.sims[0]
@@ -32,4 +35,25 @@ def test_first_recompute():
     torch.cuda.synchronize()
     assert np.array_equal(got, want)
     assert np.array_equal(e.recompute(write_state=False), want)
+    e.close()
+
+
+def positions(e):
+    return np.concatenate([e.state(0, r)[0] for r in range(4)])
+
+
+def test_blocks_on_the_default_stream_and_then_on_the_engines():
+    """A block waits for the one before it on a stream that synchronises with the default one."""
+    e = build()
+    e.run(1, 60)
+    e.run(1, 60)
+    e.synchronize()
+    want, pot = positions(e), e.replicas(0)["potential"]
+    e.close()
+    e = build()
+    busy()
+    e.run(1, 60, stream=LEGACY)
+    e.run(1, 60)
+    e.synchronize()
+    assert np.array_equal(positions(e), want) and np.array_equal(e.replicas(0)["potential"], pot)
     e.close()
