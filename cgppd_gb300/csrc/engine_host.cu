@@ -1479,12 +1479,13 @@ extern "C" int cgppd_engine_restore(cgppd_engine *e, const char *path)
     });
     e->report_capacity = saved_cap;
     std::fclose(fp);
-    if (rc != 0 || !ok)
-        return cgppd_fail("cgppd_engine_restore: truncated or mismatched checkpoint");
+    // (also of a file cut off past it: the device's count is then the file's)
     int st[4] = {0, 0, 0, 0};
     if (cgppd_check(cudaMemcpy(st, e->d_sim_state.ptr, sizeof(st), cudaMemcpyDeviceToHost), "restore") != 0)
         return -1;
     e->exchanges = st[1];
+    if (rc != 0 || !ok)
+        return cgppd_fail("cgppd_engine_restore: truncated or mismatched checkpoint");
     // rows past the checkpoint's capacity held this engine's earlier run: clear them, as
     // in the engine that wrote the checkpoint (report rows start zeroed)
     if ((int)cap < e->report_capacity) {

@@ -80,3 +80,22 @@ def test_restore_clears_report_rows_past_the_checkpoint(tmp_path):
         assert np.all(rep == 0) and tuple(ex) == (0, 0), (row, rep, ex)
     a.close()
     b.close()
+
+
+def test_reports_after_a_truncated_checkpoint(tmp_path):
+    """A file cut off at its end is refused, but the exchange count before it is already in
+    place: the rows of later exchanges are kept at that count."""
+    a = make(workloads.make("c4"), 4, 1)
+    a.run(6, 20)
+    path = tmp_path / "state.ck"
+    a.checkpoint(path)
+    path.write_bytes(path.read_bytes()[:-8])
+    b = make(workloads.make("c4"), 4, 1)
+    with pytest.raises(CgppdError):
+        b.restore(path)
+    b.run(3, 20)
+    b.synchronize()
+    for row in (6, 7, 8):
+        assert b.report(0, row)[1][1] > 0  # exchanges tested
+    a.close()
+    b.close()
