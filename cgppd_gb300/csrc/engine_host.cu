@@ -1297,6 +1297,9 @@ int cgppd_engine_set_state(cgppd_engine *e, int sim, int replica, const float *x
         rc |= cgppd_check(cudaMemcpy(e->d_center.ptr + S.molst_off + (long long)replica * S.M, buf.data(),
                                      sizeof(float4) * S.M, cudaMemcpyHostToDevice), "copy");
     }
+    // (a copy from pageable memory may return before its end, and the engine's stream does
+    // not wait for the legacy one)
+    rc |= cgppd_check(cudaStreamSynchronize(cudaStreamLegacy), "copy");
     return rc ? -1 : 0;
 }
 
@@ -1496,7 +1499,7 @@ extern "C" int cgppd_engine_restore(cgppd_engine *e, const char *path)
                                    sizeof(int2) * rows * e->sims.size()), "restore clear") != 0)
             return -1;
     }
-    return 0;
+    return cgppd_check(cudaStreamSynchronize(cudaStreamLegacy), "restore");
 }
 
 extern "C" {

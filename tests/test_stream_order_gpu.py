@@ -57,3 +57,23 @@ def test_blocks_on_the_default_stream_and_then_on_the_engines():
     e.synchronize()
     assert np.array_equal(positions(e), want) and np.array_equal(e.replicas(0)["potential"], pot)
     e.close()
+
+
+def test_state_set_and_recomputed(tmp_path):
+    """The state that set_state or restore returns from is the one that is evaluated next."""
+    a = build()
+    a.run(1, 60)
+    a.synchronize()
+    want, states = a.recompute(write_state=False), [a.state(0, r) for r in range(4)]
+    a.checkpoint(tmp_path / "state.ck")
+    b = build()
+    busy()
+    for r in range(4):
+        b.set_state(0, r, *states[r])
+    assert np.array_equal(b.recompute(write_state=True), want)
+    c = build()
+    busy()
+    c.restore(tmp_path / "state.ck")
+    assert np.array_equal(c.recompute(write_state=False), want)
+    for e in (a, b, c):
+        e.close()
