@@ -807,18 +807,12 @@ static int autotune(cgppd_engine *e, int fixed_cluster, int fixed_threads)
     DevBuf<ReplicaStats> st;
     DevBuf<unsigned long long> sc, pc;
     DevBuf<unsigned> ef;
-    auto clone = [](auto &dst, const auto &src) {
-        if (dst.alloc(src.n) != 0)
-            return -1;
-        return cgppd_check(cudaMemcpy(dst.ptr, src.ptr, src.n * sizeof(*src.ptr), cudaMemcpyDeviceToDevice),
-                           "autotune copy");
-    };
-    if (clone(pos, e->d_pos) || clone(rel, e->d_rel) || clone(cen, e->d_center) || clone(em, e->d_emat) ||
-        clone(in, e->d_intra) || clone(pot, e->d_potential) || clone(st, e->d_stats) || clone(sc, e->d_stepc) ||
-        clone(pc, e->d_pairc) || clone(ef, e->d_errflags))
+    if (pos.alloc(e->d_pos.n) || rel.alloc(e->d_rel.n) || cen.alloc(e->d_center.n) || em.alloc(e->d_emat.n) ||
+        in.alloc(e->d_intra.n) || pot.alloc(e->d_potential.n) || st.alloc(e->d_stats.n) || sc.alloc(e->d_stepc.n) ||
+        pc.alloc(e->d_pairc.n) || ef.alloc(e->d_errflags.n))
         return -1;
     DevBuf<DAStats> das;
-    if (e->da && clone(das, e->d_dastats))
+    if (e->da && das.alloc(e->d_dastats.n))
         return -1;
     EngineArgs base = e->args();
     base.pos = pos.ptr, base.rel = rel.ptr, base.center = cen.ptr, base.emat = em.ptr, base.intra = in.ptr;
@@ -827,7 +821,7 @@ static int autotune(cgppd_engine *e, int fixed_cluster, int fixed_threads)
     base.sample_xyz = nullptr;
     if (e->da)
         base.dastats = das.ptr;
-    // the clones back to the engine's state (on the engine's stream, before a timed launch)
+    // the scratch copies to the engine's state (on the engine's stream, before a timed launch)
     auto restore = [&]() -> int {
         auto back = [&](auto &dst, const auto &src) {
             return cudaMemcpyAsync(dst.ptr, src.ptr, src.n * sizeof(*src.ptr), cudaMemcpyDeviceToDevice, e->own_stream);
@@ -865,6 +859,8 @@ static int autotune(cgppd_engine *e, int fixed_cluster, int fixed_threads)
             a.cluster = C;
             a.resident = e->resident;
             a.early = e->early;
+            if (restore() != 0)
+                return -1;
             if (launch_mc_block(a, e->total_replicas, 4, T, e->smem, e->own_stream) != cudaSuccess) {
                 cudaGetLastError();  // a shape the device cannot schedule: skip it
                 continue;

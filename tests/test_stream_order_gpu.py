@@ -18,12 +18,12 @@ def busy():
 LEGACY = 1  # cudaStreamLegacy
 
 
-def build(config="c4", nrep=4):
+def build(config="c4", nrep=4, cluster=2, threads=256):
     wl = workloads.make(config)
     s = wl.sims[0]
     wl.sims = [workloads.Simulation(s.molecules, s.box, s.temperatures[:nrep], s.translate_steps[:nrep],
                                     s.rotate_steps[:nrep], s.move_weights, s.rigid_rotate_prob)]
-    return eng.from_workload(wl, cluster=2, threads=256)
+    return eng.from_workload(wl, cluster=cluster, threads=threads)
 
 
 def test_first_recompute():
@@ -77,3 +77,15 @@ def test_state_set_and_recomputed(tmp_path):
     assert np.array_equal(c.recompute(write_state=False), want)
     for e in (a, b, c):
         e.close()
+
+
+def test_shape_tuned_behind_a_busy_default_stream():
+    """Every trial launch runs on a copy of the state that is complete."""
+    busy()
+    e = build(nrep=7, cluster=0, threads=0)
+    assert len(e.tuning()) > 0
+    e.run(1, 40)
+    e.synchronize()
+    assert e.error_bits() == 0
+    assert np.allclose(e.replicas(0)["potential"], e.recompute(write_state=False), rtol=1e-5, atol=1e-6)
+    e.close()
