@@ -28,13 +28,14 @@
 #include "surrogate_internal.h"
 
 namespace cgppd {
-size_t engine_smem_bytes(int max_mol, int max_n, int max_m, int cluster, int resident, int any_flexible, int da,
+int mover_records(int n, int n1, int N, int C, int W);
+size_t engine_smem_bytes(int max_mol, int records, int max_n, int max_m, int cluster, int resident, int any_flexible, int da,
                          const int *lmax);
 cudaError_t launch_pose_samples(const EngineArgs &a, const int4 *items, int n, uint32_t key0, uint32_t key1, float *X,
                                 float *Y, cudaStream_t stream);
 cudaError_t launch_mc_block(const EngineArgs &a, int total_replicas, int nsteps, int threads, size_t smem,
                             cudaStream_t stream);
-cudaError_t set_mc_smem_limit(size_t smem);
+cudaError_t set_mc_smem_limit(const EngineArgs &a, size_t smem);
 cudaError_t launch_init_energy(const EngineArgs &a, int total_replicas, int n_work, double *potential_out,
                                cudaStream_t stream);
 cudaError_t launch_exchange(const EngineArgs &a, int nsims, int total_replicas, int steps_per_block,
@@ -184,7 +185,7 @@ struct cgppd_engine {
     int total_replicas = 0;
     int max_n = 0, max_m = 0, max_mol = 0;
     int lmax[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};  // largest per-simulation static list sizes
-    int resident = 0, early = 0, any_flexible = 0;
+    int resident = 0, early = 0, records = 0, any_flexible = 0;
     int resident_pref = 1;
     // delayed acceptance
     cgppd_surrogate *sur = nullptr;
@@ -315,6 +316,7 @@ struct cgppd_engine {
         a.resident = resident;
         a.any_flexible = any_flexible;
         a.early = early;
+        a.records = records;
         // the charged-first mover order (Debye-Hueckel terms for charged residues only)
         // pays off for rigid systems with long per-thread i loops; elsewhere it lengthens
         // the kernel for nothing (measured: C2 +6 %, C3 +10 %; C4 -3 % and C1 -3 % when
@@ -699,13 +701,22 @@ static void configure_shape(cgppd_engine *e, int C, int T)
     e->cluster = C;
     e->threads = T;
     const int da = e->da;
-    const size_t s_res = engine_smem_bytes(e->max_mol, e->max_n, e->max_m, C, 1, e->any_flexible, da, e->lmax);
-    const size_t s_da = da ? s_res - engine_smem_bytes(e->max_mol, e->max_n, e->max_m, C, 1, e->any_flexible, 0, e->lmax) : 0;
+    const int qfirst = e->args().qfirst && !da;
+    e->records = 0;
+    for (const DevSim &S : e->h_sims)
+        for (int k = 0; k < S.M; ++k) {
+            const DevMol &m = e->h_mols[S.mol_off + k];
+            e->records = std::max(e->records, mover_records(m.count, qfirst ? m.nq : m.count, S.N, C, T / 32));
+        }
+    const auto bytes = [&](int resident, int screened) {
+        return engine_smem_bytes(e->max_mol, e->records, e->max_n, e->max_m, C, resident, e->any_flexible, screened,
+                                 e->lmax);
+    };
+    const size_t s_res = bytes(1, da), s_da = s_res - bytes(1, 0);
     e->resident = (e->resident_pref != 0) && s_res <= 212 * 1024 + s_da && s_res <= 226 * 1024;
     // room for the next proposal beside the current one, where that does not cost residency
-    e->early = e->resident && !da &&
-               engine_smem_bytes(e->max_mol, e->max_n, e->max_m, C, 2, e->any_flexible, 0, e->lmax) <= 212 * 1024;
-    e->smem = engine_smem_bytes(e->max_mol, e->max_n, e->max_m, C, e->resident + e->early, e->any_flexible, da, e->lmax);
+    e->early = e->resident && !da && bytes(2, 0) <= 212 * 1024;
+    e->smem = bytes(e->resident + e->early, da);
 }
 
 // Autotuner: time k_mc for each candidate launch shape on scratch copies of the mutable
@@ -853,12 +864,13 @@ static int autotune(cgppd_engine *e, int fixed_cluster, int fixed_threads)
             if (fixed_threads > 0 && T != fixed_threads)
                 continue;
             configure_shape(e, C, T);
-            if (e->smem > 227 * 1024 || set_mc_smem_limit(e->smem) != cudaSuccess)
-                continue;
             EngineArgs a = base;
             a.cluster = C;
             a.resident = e->resident;
             a.early = e->early;
+            a.records = e->records;
+            if (e->smem > 227 * 1024 || set_mc_smem_limit(a, e->smem) != cudaSuccess)
+                continue;
             if (restore() != 0)
                 return -1;
             if (launch_mc_block(a, e->total_replicas, 4, T, e->smem, e->own_stream) != cudaSuccess) {
@@ -1027,10 +1039,12 @@ int cgppd_engine_finalize(cgppd_engine *e, int cluster, int threads)
     const bool tune = cluster <= 0 || threads <= 0;
     configure_shape(e, std::min(16, std::max(1, cluster > 0 ? cluster : 1)),
                     threads == 128 ? 128 : threads == 512 ? 512 : 256);
-    const size_t s_init = engine_smem_bytes(e->max_mol, e->max_n, e->max_m, 1, 0, e->any_flexible, 0, nullptr);
-    if (std::max(e->smem, s_init) > 227 * 1024)
+    // (the size of a one-CTA replica outside shared memory bounds the systems that are taken)
+    const size_t s_one = engine_smem_bytes(e->max_mol, (e->max_mol + 1) / 2, e->max_n, e->max_m, 1, 0, e->any_flexible, 0,
+                                           nullptr);
+    if (std::max(e->smem, s_one) > 227 * 1024)
         return cgppd_fail("cgppd_engine_finalize: system too large for shared memory (reduce molecule size or N)");
-    if (cgppd_check(set_mc_smem_limit(std::max(e->smem, s_init)), "engine shared-memory limit") != 0)
+    if (cgppd_check(set_mc_smem_limit(e->args(), e->smem), "engine shared-memory limit") != 0)
         return -1;
     if (cgppd_check(cudaStreamCreateWithFlags(&e->own_stream, cudaStreamNonBlocking), "engine stream") != 0 ||
         cgppd_check(cudaEventCreateWithFlags(&e->ordinary, cudaEventDisableTiming), "engine stream") != 0)
@@ -1041,7 +1055,8 @@ int cgppd_engine_finalize(cgppd_engine *e, int cluster, int threads)
         return -1;
     if (cgppd_check(cudaStreamSynchronize(e->own_stream), "initial energy") != 0)
         return -1;
-    if (tune && autotune(e, cluster, threads) != 0)
+    if (tune && (autotune(e, cluster, threads) != 0 ||
+                 cgppd_check(set_mc_smem_limit(e->args(), e->smem), "engine shared-memory limit") != 0))
         return -1;
     if (e->d_sim_da.zero(e->sims.size()) != 0 || e->d_dastats.zero((size_t)e->total_replicas) != 0)
         return -1;
@@ -1770,7 +1785,7 @@ int cgppd_engine_set_surrogate(cgppd_engine *e, cgppd_surrogate *s, float rmse_t
     }
     if (e->smem > 227 * 1024)
         return cgppd_fail("cgppd_engine_set_surrogate: the screened kernel does not fit in shared memory");
-    if (cgppd_check(set_mc_smem_limit(e->smem), "engine shared-memory limit") != 0)
+    if (cgppd_check(set_mc_smem_limit(e->args(), e->smem), "engine shared-memory limit") != 0)
         return -1;
     return count;
 }

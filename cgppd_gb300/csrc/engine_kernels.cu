@@ -44,6 +44,7 @@
 // Replica::fraction_bound / acceptance_ratio (src/Replica.cpp:1095-1122) and the
 // surrogate's fallback check.
 #include <array>
+#include <mutex>
 #include <type_traits>
 #include <cooperative_groups.h>
 
@@ -116,10 +117,6 @@ struct SmemLayout {
 // so that the fragment loads of 8 consecutive rows hit distinct banks.
 constexpr int kDaWS = kSurH + 8;
 
-// Records of a MoverView for molecules of up to n residues: each of its two spans rounds
-// up to an even number of rows of g <= min(32, n) lanes.
-__host__ __device__ inline int mover_records(int n) { return (n + 1) / 2 + 2 * (n < 32 ? n : 32); }
-
 __host__ __device__ inline int da_rows(int max_m) { return (((max_m - 1 > 1 ? max_m - 1 : 1) + 15) / 16) * 16; }
 
 __host__ __device__ inline int align16(int v) { return (v + 15) & ~15; }
@@ -129,21 +126,41 @@ __host__ __device__ inline int align16(int v) { return (v + 15) & ~15; }
 // g-th residue i of the mover, a warp holds floor(32 / g) such groups.  Cost of the busiest
 // thread: passes over the CTA's slice x (ceil(n / g) pairs + a per-j overhead for the
 // loads, the periodic image and the log2(g)-step reduction); the cheapest g wins, ties
-// to the smaller g.  One warp, a lane per g.
+// to the smaller g.
+__host__ __device__ inline int pair_cost(int g, int n, int N, int C, int W)
+{
+    const int sl = (N - n + C - 1) / C, per = W * (32 / g), passes = (sl + per - 1) / per;
+    const int lg = (g > 1) + (g > 2) + (g > 4) + (g > 8) + (g > 16);  // ceil(log2 g)
+    return passes * ((n + g - 1) / g + 2 + lg);
+}
+
+// One warp, a lane per g.
 __device__ __forceinline__ int pair_lanes(int n, int N, int C, int W)
 {
     const int g = (threadIdx.x & 31) + 1;
-    const int sl = (N - n + C - 1) / C, per = W * (32 / g), passes = (sl + per - 1) / per;
-    const int lg = 32 - __clz(g - 1);  // ceil(log2 g), 0 for g = 1
-    const int cost = g <= n ? passes * ((n + g - 1) / g + 2 + lg) : 0x7fffffff;
+    const int cost = g <= n ? pair_cost(g, n, N, C, W) : 0x7fffffff;
     const int best = __reduce_min_sync(0xffffffffu, cost);
     return __ffs(__ballot_sync(0xffffffffu, cost == best));
+}
+
+// Records of a MoverView that a molecule's plan takes (n1 residues in the first span): each
+// span is a whole number of pairs of rows of g lanes.
+int mover_records(int n, int n1, int N, int C, int W)
+{
+    int g = 1;
+    for (int k = 2; k <= 32 && k <= n; ++k)
+        if (pair_cost(k, n, N, C, W) < pair_cost(g, n, N, C, W))
+            g = k;
+    const auto span = [g](int residues) { return ((residues + g - 1) / g + 1) / 2 * g; };
+    return span(n1) + span(n - n1);
 }
 
 enum ListId { kLBond = 0, kLAng, kLTor, kLInd, kLFlex, kLFopt, kLBranch, kLLocal, kLCrank, kLTile };
 constexpr int kNumLists = 10;
 
-__host__ __device__ inline SmemLayout smem_layout(int max_mol, int slice, int max_m, int max_n, int resident,
+// records: the most that a molecule's plan takes at the launch's shape (mover_records; at
+// least half of max_mol, so that the displacements fit before the records' types).
+__host__ __device__ inline SmemLayout smem_layout(int max_mol, int records, int slice, int max_m, int max_n, int resident,
                                                   int any_flexible, int da = 0, int C = 1,
                                                   const int *lmax = nullptr)
 {
@@ -158,7 +175,7 @@ __host__ __device__ inline SmemLayout smem_layout(int max_mol, int slice, int ma
     L.iq = off;     off = align16(off + 8 * max_mol);
     // the mover's records (MoverView); a flex move's displacements stand in their positions
     // until these are written
-    L.ipq = off;    off += 48 * mover_records(max_mol);
+    L.ipq = off;    off += 48 * records;
     L.idisp = L.ipq;
     L.ej = off;     off = align16(off + 8 * slice);
     L.rowp = off;   off = align16(off + 8 * (max_m + 1));
@@ -210,11 +227,11 @@ __host__ __device__ inline SmemLayout smem_layout(int max_mol, int slice, int ma
     return L;
 }
 
-size_t engine_smem_bytes(int max_mol, int max_n, int max_m, int cluster, int resident, int any_flexible, int da,
+size_t engine_smem_bytes(int max_mol, int records, int max_n, int max_m, int cluster, int resident, int any_flexible, int da,
                          const int *lmax)
 {
     const int slice = (max_n + cluster - 1) / cluster;
-    return (size_t)smem_layout(max_mol, slice, max_m, max_n, resident, any_flexible, da, cluster, lmax).total;
+    return (size_t)smem_layout(max_mol, records, slice, max_m, max_n, resident, any_flexible, da, cluster, lmax).total;
 }
 
 // Static per-molecule lists (DevMol offsets index the global arrays).  Resident launches
@@ -1180,7 +1197,7 @@ template <bool RES, bool DA, bool QF, bool FLEX>
 __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ MoveDesc s_mv[2];   // this step's move and (resident) the next one's
+    __shared__ MoveDesc s_mv[RES ? 2 : 1];  // this step's move and (resident) the next one's
     __shared__ FF s_red[kMaxWarps];
     __shared__ float s_fred[3 * kMaxWarps];
     // running total, old/new row of the moved molecule and its internal energy, all as
@@ -1212,7 +1229,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
     const int N = S.N, M = S.M;
     const int slice = (a.max_n + C - 1) / C;
     const SmemLayout Ly =
-        smem_layout(a.max_mol, slice, a.max_m, a.max_n, RES ? 1 + a.early : 0, any_flexible, DA ? 1 : 0, C, a.lmax);
+        smem_layout(a.max_mol, a.records, slice, a.max_m, a.max_n, RES ? 1 + a.early : 0, any_flexible, DA ? 1 : 0, C, a.lmax);
     // screening is on for this simulation (uniform over the cluster: one simulation)
     const bool da_on = DA && a.sim_da[s] != 0;
     float *s_table = reinterpret_cast<float *>(smem + Ly.table);
@@ -1220,8 +1237,11 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
     int4 *s_iexcl = reinterpret_cast<int4 *>(smem + Ly.iexcl);
     float4 *s_disp = reinterpret_cast<float4 *>(smem + Ly.idisp);
     float2 *s_iq = reinterpret_cast<float2 *>(smem + Ly.iq);
-    const int records = mover_records(a.max_mol);
     float4 *s_ipq = reinterpret_cast<float4 *>(smem + Ly.ipq);
+    // (in a register from here on: read from the launch's arguments wherever the records are
+    // addressed, it took identical copies 565 -> 581, uneven batch 5,980 -> 6,000 us a block)
+    int records = a.records;
+    asm("" : "+r"(records));
     const MoverView mover{s_ipq, s_ipq + records, s_ipq + 2 * records};
     unsigned short *s_qpos = reinterpret_cast<unsigned short *>(smem + Ly.QP);
     float *s_rad = reinterpret_cast<float *>(smem + Ly.rad);
@@ -2745,20 +2765,27 @@ cudaError_t launch_pose_samples(const EngineArgs &a, const int4 *items, int n, u
     return cudaGetLastError();
 }
 
-// Every instantiation of k_mc a launch can pick: resident or not x delayed acceptance or
-// not x any molecule or rigid only, and the charged-first mover order (rigid only, without
-// delayed acceptance).  An engine without flexible molecules takes a kernel without their
+// Every instantiation of k_mc: resident or not x delayed acceptance or not x any molecule
+// or rigid only, and the charged-first mover order (rigid only, without delayed
+// acceptance).  An engine without flexible molecules takes a kernel without their
 // code: with it, preparing proposals early left the crowded replicas slower (1,236 -> 1,386
 // us a block of 100 steps), without it they gain (1,218).
 static const std::array<const void *, 10> &mc_kernels()
 {
     static const std::array<const void *, 10> k = {
-        (const void *)k_mc<true, false, false, true>,  (const void *)k_mc<false, false, false, true>,
-        (const void *)k_mc<true, false, false, false>, (const void *)k_mc<false, false, false, false>,
-        (const void *)k_mc<true, true, false, true>,   (const void *)k_mc<false, true, false, true>,
-        (const void *)k_mc<true, true, false, false>,  (const void *)k_mc<false, true, false, false>,
-        (const void *)k_mc<true, false, true, false>,  (const void *)k_mc<false, false, true, false>};
+        (const void *)k_mc<false, false, false, true>,  (const void *)k_mc<true, false, false, true>,
+        (const void *)k_mc<false, false, false, false>, (const void *)k_mc<true, false, false, false>,
+        (const void *)k_mc<false, true, false, true>,   (const void *)k_mc<true, true, false, true>,
+        (const void *)k_mc<false, true, false, false>,  (const void *)k_mc<true, true, false, false>,
+        (const void *)k_mc<false, false, true, false>,  (const void *)k_mc<true, false, true, false>};
     return k;
+}
+
+// The one that a launch picks (its place among them).
+static int mc_kernel(const EngineArgs &a)
+{
+    const int form = a.da ? (a.any_flexible ? 2 : 3) : a.qfirst ? 4 : a.any_flexible ? 0 : 1;
+    return 2 * form + (a.resident ? 1 : 0);
 }
 
 cudaError_t launch_mc_block(const EngineArgs &a, int total_replicas, int nsteps, int threads, size_t smem,
@@ -2788,31 +2815,25 @@ cudaError_t launch_mc_block(const EngineArgs &a, int total_replicas, int nsteps,
             allowed = true;
         }
     }
-    const auto launch = [&](auto resident, auto general) {
-        return cudaLaunchKernelEx(&cfg, a.resident ? resident : general, a, nsteps);
-    };
-    if (a.da)
-        return a.any_flexible ? launch(k_mc<true, true, false, true>, k_mc<false, true, false, true>)
-                              : launch(k_mc<true, true, false, false>, k_mc<false, true, false, false>);
-    if (a.qfirst)
-        return launch(k_mc<true, false, true, false>, k_mc<false, false, true, false>);
-    if (!a.any_flexible)
-        return launch(k_mc<true, false, false, false>, k_mc<false, false, false, false>);
-    return launch(k_mc<true, false, false, true>, k_mc<false, false, false, true>);
+    EngineArgs args = a;
+    void *params[] = {&args, &nsteps};
+    return cudaLaunchKernelExC(&cfg, mc_kernels()[mc_kernel(a)], params);
 }
 
-cudaError_t set_mc_smem_limit(size_t smem)
+cudaError_t set_mc_smem_limit(const EngineArgs &a, size_t smem)
 {
     // The attribute belongs to the kernel, not to an engine: never lower it below what an
-    // engine created earlier (and its captured graphs) needs.
-    static size_t s_max = 0;
-    if (smem <= s_max)
+    // engine created earlier (and its captured graphs) needs.  Of the kernel that the engine
+    // launches alone: the others' own shared memory differs, and with it their limit.
+    static std::mutex mu;
+    static size_t s_max[10] = {};
+    std::lock_guard<std::mutex> lock(mu);
+    const int k = mc_kernel(a);
+    if (smem <= s_max[k])
         return cudaSuccess;
-    s_max = smem;
-    cudaError_t e = cudaSuccess;
-    for (const void *f : mc_kernels())
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = cudaFuncSetAttribute(mc_kernels()[k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess)
+        s_max[k] = smem;
     return e;
 }
 

@@ -165,6 +165,7 @@ struct EngineArgs {
     int ntypes;
     int cluster;                 // CTAs per replica
     int resident;                // 1: each CTA keeps its replica's state in shared memory
+    int records;                 // mover records of the largest plan (mover_records)
     int early;                   // 1: resident, with room to prepare the next step's proposal early
     int any_flexible;            // some molecule carries internal energy terms
     int qfirst;                  // 1: k_mc<.., .., true, ..> reads rigid movers charged first
