@@ -341,6 +341,10 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net_rows(NetRowsArgs a)
                         a.dO[row] = d;
                         a.r2[row] = res * res;
                     }
+                } else if (a.y && row < a.rows) {
+                    const float res = out - a.y[row];
+                    a.dO[row] = 2.0f * res / (float)a.rows;
+                    a.r2[row] = res * res;
                 }
             }
         }

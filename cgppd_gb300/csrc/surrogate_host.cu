@@ -141,7 +141,8 @@ struct cgppd_surrogate {
 
     // Enqueue the loss sum over n rows (n % 128 == 0, n <= batch) into *loss and, with
     // `grad`, their gradient: into G, or straight into an Adam step of rate `lr` (lr > 0).
-    // `rows_of`: the batch's rows of dX / dY (targets clipped), or null for rows 0 .. n - 1.
+    // `rows_of` (with `grad`): the batch's rows of dX / dY (targets clipped), or null for rows
+    // 0 .. n - 1.
     int enqueue_step(const float *dX, const float *dY, const int *rows_of, float clip, int n, bool grad, float lr,
                      float *loss)
     {
@@ -160,7 +161,7 @@ struct cgppd_surrogate {
         r.act = act.ptr;
         r.xb = xb.ptr, r.dO = dO.ptr, r.r2 = r2.ptr;
         r.err = err.ptr;
-        if (cgppd_check(launch_net_rows(r, true, max_ctas, stream), "surrogate forward and backward pass"))
+        if (cgppd_check(launch_net_rows(r, grad, max_ctas, stream), "surrogate forward and backward pass"))
             return -1;
         NetUpdateArgs u{};
         u.wpart = wpart.ptr;

@@ -21,7 +21,7 @@ enum NetAct { kActH1 = 0, kActZ1 = 4, kActKinds = 8 };
 
 struct NetRowsArgs {
     const float *X;                // [..][8] features
-    const float *y;                // targets (backward)
+    const float *y;                // targets (backward; forward: or null)
     const int *perm;               // row -> row of X and y (targets then clipped to +-clip), or null
     float clip;
     int rows;
@@ -29,7 +29,8 @@ struct NetRowsArgs {
     const __nv_bfloat16 *wtiles;   // [6][4][256 x 64]: W2 W3 W4, then their transposes W4 W3 W2
     float *o;                      // [rows] predictions, or null
     __nv_bfloat16 *act;            // [kActKinds][tiles][256 x 64] (backward)
-    float *xb, *dO, *r2;           // (backward) the batch's features, [8][rows]; 2 (o - y) / rows; (o - y)^2
+    float *xb;                     // (backward) the batch's features, [8][rows]
+    float *dO, *r2;                // (with targets) 2 (o - y) / rows; (o - y)^2
     unsigned *err;
 };
 
