@@ -139,6 +139,15 @@ struct cgppd_surrogate {
         return cgppd_check(launch_net_rows(r, false, max_ctas, stream), "surrogate forward pass");
     }
 
+    // The weight gradients of n rows are summed over whole splits of them.
+    int check_splits(int n) const
+    {
+        const int ks = std::min(n, k_split);
+        if (n % ks != 0 || ks % 64 != 0)
+            return cgppd_fail("surrogate: batch must be a multiple of 64 (and of the split size)");
+        return 0;
+    }
+
     // Enqueue the loss sum over n rows (n % 128 == 0, n <= batch) into *loss and, with
     // `grad`, their gradient: into G, or straight into an Adam step of rate `lr` (lr > 0).
     // `rows_of` (with `grad`): the batch's rows of dX / dY (targets clipped), or null for rows
@@ -147,8 +156,8 @@ struct cgppd_surrogate {
                      float *loss)
     {
         const int ks = std::min(n, k_split);
-        if (grad && (n % ks != 0 || ks % 64 != 0))
-            return cgppd_fail("surrogate: batch must be a multiple of 64 (and of the split size)");
+        if (grad && check_splits(n))
+            return -1;
         const int tiles = (n + kNetRows - 1) / kNetRows;
         NetRowsArgs r{};
         r.X = dX;
@@ -280,6 +289,8 @@ int cgppd_surrogate_loss_grad(cgppd_surrogate *s, const float *X, const float *y
         return cgppd_fail("cgppd_surrogate_loss_grad: null argument");
     if (n <= 0 || n > s->batch || n % 128 != 0)
         return cgppd_fail("cgppd_surrogate_loss_grad: n must be a multiple of 128 no larger than the batch");
+    if (grad && s->check_splits(n))  // (before copies from the caller's memory are under way)
+        return -1;
     if (cgppd_check(cudaMemcpyAsync(s->X.ptr, X, (size_t)n * kSurIn * sizeof(float), cudaMemcpyHostToDevice, s->stream),
                     "X") ||
         cgppd_check(cudaMemcpyAsync(s->y.ptr, y, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, s->stream), "y") ||

@@ -21,7 +21,7 @@ RUNTIME = r"""
 #include <set>
 #include <cuda_runtime.h>
 
-int allocations = 0, refuse = 0;
+int allocations = 0, refuse = 0, copies = 0;
 std::set<void *> freed;
 
 extern "C" {
@@ -40,6 +40,7 @@ cudaError_t cudaMemset(void *p, int v, size_t n) { memset(p, v, n); return cudaS
 cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) { memcpy(d, s, n); return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t)
 {
+    ++copies;
     memcpy(d, s, n);
     return cudaSuccess;
 }

@@ -12,6 +12,7 @@ HARNESS = r"""
 #include "surrogate_internal.h"
 
 
+extern int copies;
 static int rows_fwd = 0, rows_bwd = 0, wgrad = 0, update[3] = {0, 0, 0};
 
 namespace cgppd {
@@ -56,6 +57,10 @@ int main()
     show("loss of an uneven batch", rc);
     rc = cgppd_surrogate_loss_grad(s, X.data(), y.data(), 1024, &loss, g.data());
     show("gradient", rc);
+    copies = 0;
+    rc = cgppd_surrogate_loss_grad(s, X.data(), y.data(), 1152, &loss, g.data());
+    show("gradient of an uneven batch", rc);
+    printf("copies %d\n", copies);
     cgppd_surrogate_destroy(s);
 }
 """
@@ -67,4 +72,6 @@ def test_launches_of_loss_and_gradient(tmp_path):
         "loss: rc 0 loss 1 rows 1 0 wgrad 0 update 1 0 0",
         "loss of an uneven batch: rc 0 loss 1 rows 1 0 wgrad 0 update 1 0 0",
         "gradient: rc 0 loss 1 rows 0 1 wgrad 1 update 0 1 0",
+        "gradient of an uneven batch: rc -1 loss 0 rows 0 0 wgrad 0 update 0 0 0",
+        "copies 0",
     ]
