@@ -29,7 +29,8 @@
 
 namespace cgppd {
 int mover_records(int n, int n1, int N, int C, int W);
-size_t engine_smem_bytes(int max_mol, int records, int max_n, int max_m, int cluster, int resident, int any_flexible, int da,
+int mover_size(int records);
+size_t engine_smem_bytes(int max_mol, int rec_mol, int max_n, int max_m, int cluster, int resident, int any_flexible, int da,
                          const int *lmax);
 cudaError_t launch_pose_samples(const EngineArgs &a, const int4 *items, int n, uint32_t key0, uint32_t key1, float *X,
                                 float *Y, cudaStream_t stream);
@@ -185,7 +186,7 @@ struct cgppd_engine {
     int total_replicas = 0;
     int max_n = 0, max_m = 0, max_mol = 0;
     int lmax[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};  // largest per-simulation static list sizes
-    int resident = 0, early = 0, records = 0, any_flexible = 0;
+    int resident = 0, early = 0, rec_mol = 0, any_flexible = 0;
     int resident_pref = 1;
     // delayed acceptance
     cgppd_surrogate *sur = nullptr;
@@ -316,7 +317,7 @@ struct cgppd_engine {
         a.resident = resident;
         a.any_flexible = any_flexible;
         a.early = early;
-        a.records = records;
+        a.rec_mol = rec_mol;
         // the charged-first mover order (Debye-Hueckel terms for charged residues only)
         // pays off for rigid systems with long per-thread i loops; elsewhere it lengthens
         // the kernel for nothing (measured: C2 +6 %, C3 +10 %; C4 -3 % and C1 -3 % when
@@ -702,14 +703,15 @@ static void configure_shape(cgppd_engine *e, int C, int T)
     e->threads = T;
     const int da = e->da;
     const int qfirst = e->args().qfirst && !da;
-    e->records = 0;
+    int records = 0;
     for (const DevSim &S : e->h_sims)
         for (int k = 0; k < S.M; ++k) {
             const DevMol &m = e->h_mols[S.mol_off + k];
-            e->records = std::max(e->records, mover_records(m.count, qfirst ? m.nq : m.count, S.N, C, T / 32));
+            records = std::max(records, mover_records(m.count, qfirst ? m.nq : m.count, S.N, C, T / 32));
         }
+    e->rec_mol = mover_size(records);
     const auto bytes = [&](int resident, int screened) {
-        return engine_smem_bytes(e->max_mol, e->records, e->max_n, e->max_m, C, resident, e->any_flexible, screened,
+        return engine_smem_bytes(e->max_mol, e->rec_mol, e->max_n, e->max_m, C, resident, e->any_flexible, screened,
                                  e->lmax);
     };
     const size_t s_res = bytes(1, da), s_da = s_res - bytes(1, 0);
@@ -868,7 +870,7 @@ static int autotune(cgppd_engine *e, int fixed_cluster, int fixed_threads)
             a.cluster = C;
             a.resident = e->resident;
             a.early = e->early;
-            a.records = e->records;
+            a.rec_mol = e->rec_mol;
             if (e->smem > 227 * 1024 || set_mc_smem_limit(a, e->smem) != cudaSuccess)
                 continue;
             if (restore() != 0)
@@ -1040,7 +1042,7 @@ int cgppd_engine_finalize(cgppd_engine *e, int cluster, int threads)
     configure_shape(e, std::min(16, std::max(1, cluster > 0 ? cluster : 1)),
                     threads == 128 ? 128 : threads == 512 ? 512 : 256);
     // (the size of a one-CTA replica outside shared memory bounds the systems that are taken)
-    const size_t s_one = engine_smem_bytes(e->max_mol, (e->max_mol + 1) / 2, e->max_n, e->max_m, 1, 0, e->any_flexible, 0,
+    const size_t s_one = engine_smem_bytes(e->max_mol, mover_size((e->max_mol + 1) / 2), e->max_n, e->max_m, 1, 0, e->any_flexible, 0,
                                            nullptr);
     if (std::max(e->smem, s_one) > 227 * 1024)
         return cgppd_fail("cgppd_engine_finalize: system too large for shared memory (reduce molecule size or N)");

@@ -117,6 +117,10 @@ struct SmemLayout {
 // so that the fragment loads of 8 consecutive rows hit distinct banks.
 constexpr int kDaWS = kSurH + 8;
 
+// Records of a MoverView that hold any plan of a molecule of n residues: each of its two
+// spans rounds up to an even number of rows of g <= min(32, n) lanes.
+__host__ __device__ inline int mover_bound(int n) { return (n + 1) / 2 + 2 * (n < 32 ? n : 32); }
+
 __host__ __device__ inline int da_rows(int max_m) { return (((max_m - 1 > 1 ? max_m - 1 : 1) + 15) / 16) * 16; }
 
 __host__ __device__ inline int align16(int v) { return (v + 15) & ~15; }
@@ -143,8 +147,8 @@ __device__ __forceinline__ int pair_lanes(int n, int N, int C, int W)
     return __ffs(__ballot_sync(0xffffffffu, cost == best));
 }
 
-// Records of a MoverView that a molecule's plan takes (n1 residues in the first span): each
-// span is a whole number of pairs of rows of g lanes.
+// Records that a molecule's plan takes (n1 residues in the first span): each span is a whole
+// number of pairs of rows of g lanes.
 int mover_records(int n, int n1, int N, int C, int W)
 {
     int g = 1;
@@ -155,12 +159,22 @@ int mover_records(int n, int n1, int N, int C, int W)
     return span(n1) + span(n - n1);
 }
 
+// The smallest molecule whose bound holds `records`.
+int mover_size(int records)
+{
+    int n = 1;
+    while (mover_bound(n) < records)
+        ++n;
+    return n;
+}
+
 enum ListId { kLBond = 0, kLAng, kLTor, kLInd, kLFlex, kLFopt, kLBranch, kLLocal, kLCrank, kLTile };
 constexpr int kNumLists = 10;
 
-// records: the most that a molecule's plan takes at the launch's shape (mover_records; at
-// least half of max_mol, so that the displacements fit before the records' types).
-__host__ __device__ inline SmemLayout smem_layout(int max_mol, int records, int slice, int max_m, int max_n, int resident,
+// rec_mol: the molecule that the mover's records are laid out for, the smallest whose bound
+// holds every plan at the launch's shape (at least half of max_mol records, so that the
+// displacements fit before the records' types).
+__host__ __device__ inline SmemLayout smem_layout(int max_mol, int rec_mol, int slice, int max_m, int max_n, int resident,
                                                   int any_flexible, int da = 0, int C = 1,
                                                   const int *lmax = nullptr)
 {
@@ -175,7 +189,7 @@ __host__ __device__ inline SmemLayout smem_layout(int max_mol, int records, int 
     L.iq = off;     off = align16(off + 8 * max_mol);
     // the mover's records (MoverView); a flex move's displacements stand in their positions
     // until these are written
-    L.ipq = off;    off += 48 * records;
+    L.ipq = off;    off += 48 * mover_bound(rec_mol);
     L.idisp = L.ipq;
     L.ej = off;     off = align16(off + 8 * slice);
     L.rowp = off;   off = align16(off + 8 * (max_m + 1));
@@ -227,11 +241,11 @@ __host__ __device__ inline SmemLayout smem_layout(int max_mol, int records, int 
     return L;
 }
 
-size_t engine_smem_bytes(int max_mol, int records, int max_n, int max_m, int cluster, int resident, int any_flexible, int da,
+size_t engine_smem_bytes(int max_mol, int rec_mol, int max_n, int max_m, int cluster, int resident, int any_flexible, int da,
                          const int *lmax)
 {
     const int slice = (max_n + cluster - 1) / cluster;
-    return (size_t)smem_layout(max_mol, records, slice, max_m, max_n, resident, any_flexible, da, cluster, lmax).total;
+    return (size_t)smem_layout(max_mol, rec_mol, slice, max_m, max_n, resident, any_flexible, da, cluster, lmax).total;
 }
 
 // Static per-molecule lists (DevMol offsets index the global arrays).  Resident launches
@@ -1229,7 +1243,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
     const int N = S.N, M = S.M;
     const int slice = (a.max_n + C - 1) / C;
     const SmemLayout Ly =
-        smem_layout(a.max_mol, a.records, slice, a.max_m, a.max_n, RES ? 1 + a.early : 0, any_flexible, DA ? 1 : 0, C, a.lmax);
+        smem_layout(a.max_mol, a.rec_mol, slice, a.max_m, a.max_n, RES ? 1 + a.early : 0, any_flexible, DA ? 1 : 0, C, a.lmax);
     // screening is on for this simulation (uniform over the cluster: one simulation)
     const bool da_on = DA && a.sim_da[s] != 0;
     float *s_table = reinterpret_cast<float *>(smem + Ly.table);
@@ -1238,10 +1252,10 @@ __global__ void __launch_bounds__(kMaxThreads) k_mc(EngineArgs a, int nsteps)
     float4 *s_disp = reinterpret_cast<float4 *>(smem + Ly.idisp);
     float2 *s_iq = reinterpret_cast<float2 *>(smem + Ly.iq);
     float4 *s_ipq = reinterpret_cast<float4 *>(smem + Ly.ipq);
-    // (in a register from here on: read from the launch's arguments wherever the records are
-    // addressed, it took identical copies 565 -> 581, uneven batch 5,980 -> 6,000 us a block)
-    int records = a.records;
-    asm("" : "+r"(records));
+    // (the bound of a size, last among the arguments: with the number itself, or with one more
+    // argument between the others, the step kernels were allotted other registers and a
+    // crowded replica took 1 to 2 % longer)
+    const int records = mover_bound(a.rec_mol);
     const MoverView mover{s_ipq, s_ipq + records, s_ipq + 2 * records};
     unsigned short *s_qpos = reinterpret_cast<unsigned short *>(smem + Ly.QP);
     float *s_rad = reinterpret_cast<float *>(smem + Ly.rad);
@@ -2773,11 +2787,11 @@ cudaError_t launch_pose_samples(const EngineArgs &a, const int4 *items, int n, u
 static const std::array<const void *, 10> &mc_kernels()
 {
     static const std::array<const void *, 10> k = {
-        (const void *)k_mc<false, false, false, true>,  (const void *)k_mc<true, false, false, true>,
-        (const void *)k_mc<false, false, false, false>, (const void *)k_mc<true, false, false, false>,
-        (const void *)k_mc<false, true, false, true>,   (const void *)k_mc<true, true, false, true>,
-        (const void *)k_mc<false, true, false, false>,  (const void *)k_mc<true, true, false, false>,
-        (const void *)k_mc<false, false, true, false>,  (const void *)k_mc<true, false, true, false>};
+        (const void *)k_mc<true, false, false, true>,  (const void *)k_mc<false, false, false, true>,
+        (const void *)k_mc<true, false, false, false>, (const void *)k_mc<false, false, false, false>,
+        (const void *)k_mc<true, true, false, true>,   (const void *)k_mc<false, true, false, true>,
+        (const void *)k_mc<true, true, false, false>,  (const void *)k_mc<false, true, false, false>,
+        (const void *)k_mc<true, false, true, false>,  (const void *)k_mc<false, false, true, false>};
     return k;
 }
 
@@ -2785,7 +2799,7 @@ static const std::array<const void *, 10> &mc_kernels()
 static int mc_kernel(const EngineArgs &a)
 {
     const int form = a.da ? (a.any_flexible ? 2 : 3) : a.qfirst ? 4 : a.any_flexible ? 0 : 1;
-    return 2 * form + (a.resident ? 1 : 0);
+    return 2 * form + (a.resident ? 0 : 1);
 }
 
 cudaError_t launch_mc_block(const EngineArgs &a, int total_replicas, int nsteps, int threads, size_t smem,

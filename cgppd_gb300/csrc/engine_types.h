@@ -165,7 +165,6 @@ struct EngineArgs {
     int ntypes;
     int cluster;                 // CTAs per replica
     int resident;                // 1: each CTA keeps its replica's state in shared memory
-    int records;                 // mover records of the largest plan (mover_records)
     int early;                   // 1: resident, with room to prepare the next step's proposal early
     int any_flexible;            // some molecule carries internal energy terms
     int qfirst;                  // 1: k_mc<.., .., true, ..> reads rigid movers charged first
@@ -182,6 +181,7 @@ struct EngineArgs {
     float sur_thr2;              // fallback when mean squared error > sur_thr2
     float sur_window;            // errors counted for |exact change| <= sur_window
     int sur_min;                 // ... once a block has at least sur_min of them
+    int rec_mol;                 // molecule that the mover's records are laid out for (mover_bound)
 };
 
 }  // namespace cgppd
