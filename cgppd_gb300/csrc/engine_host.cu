@@ -649,46 +649,47 @@ int cgppd_engine::build()
     init_work = (int)work.size();
 
     int rc = 0;
-    rc |= d_init_tasks.upload(init_tasks);
-    rc |= d_init_work.upload(work);
-    rc |= d_sims.upload(h_sims);
-    rc |= d_rep_sim.upload(rep_sim);
-    rc |= d_rep_order.upload(rep_order);
-    rc |= d_mols.upload(h_mols);
-    rc |= d_rstat.upload(rstat);
-    rc |= d_rqpos.upload(rqpos);
-    rc |= d_rexcl.upload(rexcl);
-    rc |= d_bonds.upload(bonds);
-    rc |= d_indsub.upload(indsub);
-    rc |= d_angles.upload(angles);
-    rc |= d_tors.upload(tors);
-    rc |= d_torsV.upload(torsVv);
-    rc |= d_torsS.upload(torsSv);
-    rc |= d_flexres.upload(flexres);
-    rc |= d_flexopt.upload(flexopt);
-    rc |= d_branch.upload(branch);
-    rc |= d_localres.upload(localres);
-    rc |= d_crankres.upload(crankres);
-    rc |= d_tiles.upload(tiles);
-    rc |= d_table.upload(table);
-    rc |= d_pos.upload(pos);
-    rc |= d_rel.upload(rel);
-    rc |= d_center.upload(center);
-    rc |= d_emat.zero((size_t)emat_off);
-    rc |= d_intra.zero((size_t)molst_off);
-    rc |= d_potential.zero((size_t)total_replicas);
-    rc |= d_scratch_pot.zero((size_t)total_replicas);
-    rc |= d_temperature.upload(temperature);
-    rc |= d_tstep.upload(tstep);
-    rc |= d_rstep.upload(rstep);
-    rc |= d_stepc.zero((size_t)total_replicas);
-    rc |= d_pairc.zero((size_t)total_replicas);
-    rc |= d_stats.zero((size_t)total_replicas);
-    rc |= d_tindex.upload(tindex);
-    rc |= d_label.upload(label);
-    rc |= d_slot_of_t.upload(slot_of_t);
-    rc |= d_sim_state.upload(sim_state);
-    rc |= d_errflags.zero((size_t)total_replicas);
+    rc |= d_init_tasks.upload(init_tasks, false);
+    rc |= d_init_work.upload(work, false);
+    rc |= d_sims.upload(h_sims, false);
+    rc |= d_rep_sim.upload(rep_sim, false);
+    rc |= d_rep_order.upload(rep_order, false);
+    rc |= d_mols.upload(h_mols, false);
+    rc |= d_rstat.upload(rstat, false);
+    rc |= d_rqpos.upload(rqpos, false);
+    rc |= d_rexcl.upload(rexcl, false);
+    rc |= d_bonds.upload(bonds, false);
+    rc |= d_indsub.upload(indsub, false);
+    rc |= d_angles.upload(angles, false);
+    rc |= d_tors.upload(tors, false);
+    rc |= d_torsV.upload(torsVv, false);
+    rc |= d_torsS.upload(torsSv, false);
+    rc |= d_flexres.upload(flexres, false);
+    rc |= d_flexopt.upload(flexopt, false);
+    rc |= d_branch.upload(branch, false);
+    rc |= d_localres.upload(localres, false);
+    rc |= d_crankres.upload(crankres, false);
+    rc |= d_tiles.upload(tiles, false);
+    rc |= d_table.upload(table, false);
+    rc |= d_pos.upload(pos, false);
+    rc |= d_rel.upload(rel, false);
+    rc |= d_center.upload(center, false);
+    rc |= d_emat.zero((size_t)emat_off, false);
+    rc |= d_intra.zero((size_t)molst_off, false);
+    rc |= d_potential.zero((size_t)total_replicas, false);
+    rc |= d_scratch_pot.zero((size_t)total_replicas, false);
+    rc |= d_temperature.upload(temperature, false);
+    rc |= d_tstep.upload(tstep, false);
+    rc |= d_rstep.upload(rstep, false);
+    rc |= d_stepc.zero((size_t)total_replicas, false);
+    rc |= d_pairc.zero((size_t)total_replicas, false);
+    rc |= d_stats.zero((size_t)total_replicas, false);
+    rc |= d_tindex.upload(tindex, false);
+    rc |= d_label.upload(label, false);
+    rc |= d_slot_of_t.upload(slot_of_t, false);
+    rc |= d_sim_state.upload(sim_state, false);
+    rc |= d_errflags.zero((size_t)total_replicas, false);
+    rc |= buffers_settled();
     report_capacity = 0;
     return rc ? -1 : 0;
 }
