@@ -294,12 +294,24 @@ __device__ __forceinline__ void clean_block(const XBlock &X, const YLane &y, flo
 
 // ------------------------------------------------------------------ work of a call
 
-// x blocks of a CTA for nt tiles of 128 residues: the blocks of a CTA are a serial chain, so
-// one while that leaves SMs short of warps, more once the copies and keys of a CTA cost
-// more than the chain.  us a call on three streams with 1 / 2 / 4 blocks: 21 tiles 5.6 / 6.5 /
-// 8.7, 28 tiles 8.6 / 9.4, 32 tiles 11.1 / 10.7, 36 tiles 14.2 / 13.1, 39 tiles 16.1 / 14.6 /
-// 12.6, 55 tiles - / 26.5 / 22.3; of a synchronous call with 1 / 2: 28 tiles 28.8 / 31.2, 32
-// tiles 31.0 / 32.9, 36 tiles 34.5 / 35.3, and in bursts on one stream 28 tiles 17.7 / 19.7.
+// x blocks of a CTA for nt tiles: the blocks of a CTA are a serial chain, so one while that
+// leaves SMs short of warps, more once the copies and keys of a CTA cost more than the
+// chain.  us a call with 1 / 2 / 4 blocks:
+//   tiles                    28               34               39               44
+//   async, three streams      8.4/ 8.7/10.2   12.4/11.0/12.0   15.9/14.4/13.3   20.3/18.7/15.4
+//   async, one stream        16.9/19.0/24.5   20.8/21.4/27.5   25.0/25.1/29.7   29.6/29.5/31.9
+//   synchronous              28.3/30.9/35.0   32.9/32.9/37.9   37.0/36.8/40.0   40.7/41.1/42.5
+//   synchronous, NC          25.5/25.7/26.2   29.9/28.4/28.7   34.4/32.3/32.7   38.0/35.4/34.6
+//   tiles                    48               56               64              100
+//   async, three streams     23.9/21.9/18.0   32.0/29.4/24.3   41.3/37.8/31.4   99.1/90.7/75.5
+//   async, one stream        32.5/33.0/35.7   41.5/40.9/41.5   50.0/49.1/48.9  109.4/102.3/93.1
+//   synchronous              44.1/43.4/47.0   52.4/51.5/52.5   61.7/59.7/59.7  120.7/113.2/104.1
+//   synchronous, NC          40.7/38.7/37.3   49.3/46.1/43.2   57.7/54.0/50.2  114.0/104.4/93.0
+// The size is all that a call knows of what runs beside it, so the lines lie between the
+// two: two blocks from 34 tiles, where they take 11 % off calls on several streams and add 3 %
+// to others (at 30: 5 against 11); four from 40, where they take 12 to 18 % off calls on
+// several streams and add up to 15 % to others (at 38 and 39 they would take 4 to 8 and add
+// 18 to 19); from 60 tiles on they are the best, or level, for all.
 __host__ __device__ constexpr int x_blocks(int nt) { return nt >= kFourBlocks ? 4 : nt >= kTwoBlocks ? 2 : 1; }
 
 // CTAs of a call: for each tile ty the chunks of x blocks on or after it, rows of
