@@ -880,10 +880,6 @@ __device__ void predecide_move(const Lists &a, const DevSim &S, const DevMol *mo
     pre.w_stage1 = w[9];
 }
 
-// The move of a step from its draw-only part and the state: the centre, the translation
-// and its wrap, the flex pivot, the crankshaft rotation.  `last` (or null): an accepted
-// move that is being committed meanwhile, its positions in `lastpos`; the state of every
-// other molecule is at rest.
 // The molecule's centre after a translation along the decision's direction (rounded step
 // by step: two places evaluate it, with the same bits).
 __device__ __forceinline__ float3 translated(const MovePre &pre, float4 c, float tstep, float box)
@@ -892,6 +888,10 @@ __device__ __forceinline__ float3 translated(const MovePre &pre, float4 c, float
     return make_float3(axis(c.x, pre.R[0]), axis(c.y, pre.R[1]), axis(c.z, pre.R[2]));
 }
 
+// The move of a step from its draw-only part and the state: the centre, the translation
+// and its wrap, the flex pivot, the crankshaft rotation.  `last` (or null): an accepted
+// move that is being committed meanwhile, its positions in `lastpos`; the state of every
+// other molecule is at rest.
 template <bool RES, bool FLEX>
 __device__ void finish_move(const DevSim &S, const DevMol *mols, const float4 *CEN, const float4 *P, float tstep,
                             const float4 rsc, const MovePre &pre, MoveDesc &mv, const MoveDesc *last,

@@ -12,7 +12,8 @@
 // Network: 8 -> 256 -> 256 -> 256 -> 256 -> 1, SiLU after each hidden layer.  Layer 1
 // (K = 8) and the output dot product run in FP32; layers 2-4 are BF16 tensor-core
 // GEMMs with FP32 accumulation.  Master parameters are FP32 (Adam); the GEMM layers
-// also keep BF16 copies: Wf[out][in] (forward operand) and Wt[in][out] (backward).
+// also keep BF16 copies: Wf[out][in] (the engine's screening kernel) and the tile images of
+// the weights and their transposes that the training kernels read.
 #pragma once
 
 #include <cuda_bf16.h>
