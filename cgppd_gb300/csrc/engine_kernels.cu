@@ -2848,6 +2848,8 @@ cudaError_t set_mc_smem_limit(const EngineArgs &a, size_t smem)
     const cudaError_t e = cudaFuncSetAttribute(mc_kernels()[k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess)
         s_max[k] = smem;
+    else
+        cudaGetLastError();  // (reported here: a later launch must not find it)
     return e;
 }
 

@@ -36,6 +36,17 @@ def test_nearly_full(count, cluster):
     e.close()
 
 
+def test_shape_that_is_tried_and_does_not_fit():
+    """868 molecules over 8 CTAs pass the size check, but not with the kernel's own part: the
+    tuner goes on to another shape, and the failed try leaves no error to a later launch."""
+    e = many_small(868, 0)
+    assert 8 not in [c for c, _, _ in e.tuning()] and len(e.tuning()) > 0
+    e.run(2, 50)
+    e.synchronize()
+    assert e.error_bits() == 0
+    e.close()
+
+
 def test_past_the_end():
     with pytest.raises(CgppdError):
         many_small(900, 8)
